@@ -54,13 +54,16 @@ struct PbfK {
     int32_t n;                // particle count when n_dev is null
     const int32_t* n_dev;     // device-resident particle count (emitters append on the device)
     DomDev d0; // the scene when there is only one
-    // candidate masks (cell h only): per particle the candidates within h + skin, per cell a mark that a
+    // candidate lists (cell h only): per particle the candidates within h + skin, per cell a mark that a
     // particle of the 3 x 3 cells around it moved too far for them
     const uint32_t* keys;     // sort cell of each slot
-    uint4* nmask;
+    uint4* nhdr;
+    uint4* nlist;
     uint8_t* mflag;
+    int64_t nstride;          // particles a list chunk's array holds (the capacity)
+    int32_t wide;             // lists of 32-bit slots
     float skin2;              // (h + skin)^2
-    float move2;              // (skin / (2 iters))^2, shrunk by 1%
+    float move2;              // (skin / 2)^2, shrunk for rounding
     // set for the XSPH pass of a step that also computes the next step's predicted cell keys and their
     // histogram (from the positions and velocities it writes); null otherwise
     uint2* hist_kr;
@@ -86,6 +89,14 @@ __device__ __forceinline__ int32_t cell_coord(float pos, float org, float inv, i
     if (!(u >= 0.f)) { return 0; }
     if (u >= (float)nc) { return nc - 1; }
     return (int32_t)u;
+}
+
+// the sort cell key of position ps in scene d
+__device__ __forceinline__ uint32_t cell_key(const PbfK& k, const DomDev& d, float2 ps)
+{
+    const int32_t cx = cell_coord(ps.x, d.ox, k.inv_cell, d.ncx);
+    const int32_t cy = cell_coord(ps.y, d.oy, k.inv_cell, d.ncy);
+    return d.coff + (uint32_t)cy * (uint32_t)d.ncx + (uint32_t)cx;
 }
 
 template <bool MULTI>
@@ -133,6 +144,21 @@ struct Nbr {
     float a;
 };
 
+// loads a candidate's record, or its record and the value beside it
+template <bool CG>
+struct Records {
+    const float4* __restrict__ xd;
+    __device__ __forceinline__ float4 record(uint32_t j) const { return ldn<CG>(&xd[j]); }
+    __device__ __forceinline__ float4 operator()(uint32_t j) const { return record(j); }
+};
+template <bool CG>
+struct RecordsAnd {
+    const float4* __restrict__ xd;
+    const float* __restrict__ a;
+    __device__ __forceinline__ float4 record(uint32_t j) const { return ldn<CG>(&xd[j]); }
+    __device__ __forceinline__ Nbr operator()(uint32_t j) const { return Nbr{ldn<CG>(&xd[j]), ldn<CG>(&a[j])}; }
+};
+
 // Visits every particle index in the cells within R of the base cell of (px, py) (the reference scans the
 // 3x3 cells around clamp(floorf(x)/kCellDim), PBF.cu:252-263). Each row of cells is one contiguous range.
 template <class F>
@@ -149,14 +175,17 @@ __device__ __forceinline__ void for_neighbours(const DomDev& d, const PbfK& k, c
         const uint32_t row = d.coff + (uint32_t)y * (uint32_t)d.ncx;
         const uint32_t b   = __ldg(&start[row + x0]);
         const uint32_t e   = __ldg(&start[row + x1 + 1]);
+#pragma unroll 1
         for (uint32_t j = b; j < e; ++j) { f(j); }
     }
 }
 
-// for_neighbours from a given base cell
-template <class F>
+// The same candidates in the same order from base cell (bx, by), four at a time so that their records' loads are in
+// flight together: ap(j, ld(j), valid), the last candidate of a row standing in (valid false) for those that the
+// row's last four lack.
+template <class L, class A>
 __device__ __forceinline__ void for_neighbours_at(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start,
-                                                  int32_t bx, int32_t by, F&& f)
+                                                  int32_t bx, int32_t by, L&& ld, A&& ap)
 {
     const int32_t x0 = max(bx - k.R, 0);
     const int32_t x1 = min(bx + k.R, d.ncx - 1);
@@ -166,148 +195,220 @@ __device__ __forceinline__ void for_neighbours_at(const DomDev& d, const PbfK& k
         const uint32_t row = d.coff + (uint32_t)y * (uint32_t)d.ncx;
         const uint32_t b   = __ldg(&start[row + x0]);
         const uint32_t e   = __ldg(&start[row + x1 + 1]);
-        for (uint32_t j = b; j < e; ++j) { f(j); }
+#pragma unroll 1
+        for (uint32_t j = b; j < e; j += 4u) {
+            const uint32_t j1 = min(j + 1u, e - 1u), j2 = min(j + 2u, e - 1u), j3 = min(j + 3u, e - 1u);
+            const auto q0 = ld(j), q1 = ld(j1), q2 = ld(j2), q3 = ld(j3);
+            ap(j, q0, true);
+            ap(j1, q1, j + 1u < e);
+            ap(j2, q2, j + 2u < e);
+            ap(j3, q3, j + 3u < e);
+        }
     }
 }
 
-// ----- candidate masks -----------------------------------------------------------------------------------
+// ----- candidate lists -----------------------------------------------------------------------------------
 // With sort cells of edge h a particle scans three rows of three cells, each row one contiguous range of
-// slots. The first plain lambda pass of a step records which candidates of each row lie within h + skin
-// (word r, bit t: the candidate at slot start[row r, first cell] + t), and the later passes of the step
-// visit only those. Every pair within h is still visited, in the scan order, as long as
+// slots. The first plain lambda pass of a step records the candidates that lie within h + skin as a list, and
+// the later passes of the step visit only those. Every pair within h is still visited, in the scan order, as
+// long as
 //   - the particle's base cell is still its sort cell (so its rows are the recorded ones), and
-//   - no particle of the 3 x 3 cells around it has moved by skin / 2 or more since the masks were made:
-//     a delta p pass that moves a particle by skin / (2 iters) or more marks the 9 cells around that
-//     particle's sort cell for the rest of the step, and a particle whose own cell is marked scans in full.
+//   - no particle of the 3 x 3 cells around it is skin / 2 or more away from where it was when the lists were
+//     made: a delta p pass that leaves a particle that far from there marks the 9 cells around that particle's
+//     sort cell for the rest of the step, and a particle whose own cell is marked scans in full.
 // The terms of pairs beyond h are exact zeros in every sum (the sums start at +0, and adding a masked
-// +-0 leaves any value bit for bit), so masked and full scans give the same result.
-enum { MASK_OFF = 0, MASK_BUILD = 1, MASK_USE = 2 };
-constexpr uint32_t MASK_BAD = 0x80000000u; // in word 0: this particle's masks are not usable
+// +-0 leaves any value bit for bit), so listed and full scans give the same result.
+//
+// Per particle: a header {sort cell, candidates, d when the list was made} and the candidates' slots in groups
+// of four, relative to the particle's own slot in 16 bits, eight to a 16-byte chunk; chunk c of particle i is
+// nlist[c * nstride + i], so a warp reads a chunk with one coalesced 512-byte access. Scenes so wide that the
+// slots of the next cell row can be more than 2^15 away hold 32-bit slots instead, four to a chunk (k.wide).
+//
+// The passes are bound by instruction issue and by the gathers' latency. A list costs two instructions a candidate
+// to find its record, where one bit per slot of the three rows (what the lists replaced) cost about fourteen, and
+// it lets four records be in flight at once. The distance from the lists' making replaces a bound of
+// skin / (2 iterations) on every single pass's move, which a state fresh from outside broke nearly everywhere.
+// One step of 1,048,576 particles from such a state: listed lambda 50 -> 25 us, delta p 41 -> 26 us, XSPH
+// 41 -> 28 us, the step with its state's copies 0.468 -> 0.325 ms; from an evolved state lambda 27 -> 23 us and
+// delta p 27 -> 23 us. 256 batched scenes (5.1M particles) 2.20 -> 1.42 ms.
+enum { LIST_OFF = 0, LIST_BUILD = 1, LIST_USE = 2 };
+constexpr uint32_t LIST_BAD   = 0x80000000u; // in the header's count: this particle's list is not usable
+constexpr uint32_t LIST_MAX   = 48;          // candidates a list holds (a multiple of 8)
+constexpr uint32_t LIST_REACH = 32767;       // largest distance of a 16-bit slot
 
-// The full scan of particle i whose base cell is (bx, by) (cell h, R = 1), recording its masks. f(j)
-// returns whether candidate j lies within h + skin. The particle's own slot is not recorded: no pass takes
-// a term from the self pair inside its loop (the density's self term is added after it); its bit is cleared
-// after the scan, and self_in tells whether the scan met that slot.
-template <class F>
-__device__ __forceinline__ uint4 scan_build(const DomDev& d, const uint32_t* __restrict__ start, int32_t bx,
-                                            int32_t by, int32_t i, bool& self_in, F&& f)
+// rsqrt of a value that is never subnormal (here: above 1e-12): the hardware's approximation, which rsqrtf
+// returns for such values too, without rsqrtf's scaling of subnormal arguments
+__device__ __forceinline__ float rsqrt_normal(float v)
 {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Particle i's full scan around base cell (bx, by) (cell h, R = 1), recording its list. near(j): candidate j lies
+// within h + skin; ap(j, ld(j), valid) applies a recorded candidate (valid is false for the filler of the last
+// group of four), full(j, ld(j), valid) a candidate when the list cannot hold them. The particle's own slot is not
+// recorded: no pass takes a term from the self pair inside its loop (the density's self term is added after it).
+// Returns whether the recorded scan met that slot. A distance-only scan finds the candidates as one bit per slot
+// of each row, four slots a turn so that their loads are in flight together (the slots past a row's end that the
+// last turn reads are masked off; the record arrays are three records longer than the capacity); then the
+// candidates are taken out of the bits in scan order, stored, and applied: the same terms in the same order as the
+// full scan, whose other candidates add exact zeros.
+template <bool CG, class T, class L, class A, class F>
+__device__ __forceinline__ bool scan_record(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start,
+                                            float px, float py, float2 disp, int32_t i, T&& near, L&& ld, A&& ap,
+                                            F&& full)
+{
+    const int32_t bx = cell_coord(px, d.ox, k.inv_cell, d.ncx);
+    const int32_t by = cell_coord(py, d.oy, k.inv_cell, d.ncy);
     const int32_t x0 = max(bx - 1, 0);
     const int32_t x1 = min(bx + 1, d.ncx - 1);
     uint32_t w[3]    = {0u, 0u, 0u};
-    bool bad         = false;
-    self_in          = false;
+    uint32_t b[3]    = {0u, 0u, 0u};
+    bool fits        = true; // the rows fit their bits, the slots their 16 bits
+    bool self_in     = false;
 #pragma unroll
     for (int32_t r = 0; r < 3; ++r) {
         const int32_t y = by - 1 + r;
         if (y < 0 || y >= d.ncy) { continue; }
         const uint32_t row = d.coff + (uint32_t)y * (uint32_t)d.ncx;
-        const uint32_t b   = __ldg(&start[row + x0]);
+        b[r]               = __ldg(&start[row + x0]);
         const uint32_t e   = __ldg(&start[row + x1 + 1]);
-        bad                = bad || (e - b > 31u);
-        // one bit per slot, shifted along with the slot (a row of more than 31 slots is marked bad above,
-        // and its bits are never read)
-        uint32_t wr = 0u, bit = 1u;
-        for (uint32_t j = b; j < e; ++j, bit <<= 1) { wr |= f(j) ? bit : 0u; }
-        const uint32_t t = (uint32_t)i - b;
-        if (t < e - b) { // the particle's own slot is in this row
+        const uint32_t len = e - b[r];
+        if (len > 31u || (!k.wide && ((uint32_t)i - b[r] + LIST_REACH > 2u * LIST_REACH ||
+                                      e - (uint32_t)i + LIST_REACH > 2u * LIST_REACH))) {
+            fits = false;
+            continue;
+        }
+        uint32_t wr = 0u;
+        for (uint32_t t = 0u; t < len; t += 4u) {
+            const uint32_t j = b[r] + t;
+            const float4 q0 = ld.record(j), q1 = ld.record(j + 1u), q2 = ld.record(j + 2u), q3 = ld.record(j + 3u);
+            uint32_t n4 = near(q0) ? 1u : 0u;
+            n4 |= near(q1) ? 2u : 0u;
+            n4 |= near(q2) ? 4u : 0u;
+            n4 |= near(q3) ? 8u : 0u;
+            wr |= n4 << t;
+        }
+        wr &= (1u << len) - 1u;
+        const uint32_t t = (uint32_t)i - b[r];
+        if (t < len) { // the particle's own slot is in this row
             self_in = true;
-            wr &= t < 31u ? ~(1u << t) : 0xffffffffu;
+            wr &= ~(1u << t);
         }
         w[r] = wr;
     }
-    return make_uint4((w[0] & ~MASK_BAD) | (bad ? MASK_BAD : 0u), w[1], w[2], 0u);
-}
-
-// Visits the candidates of the masks m around base cell (bx, by), in scan order. The three rows run as one
-// loop (the next row with candidates takes over when a row's bits run out), so a warp iterates as often as
-// its lane with the most candidates, not the sum over rows of each row's maximum.
-template <class L, class A>
-__device__ __forceinline__ void scan_masked(const DomDev& d, const uint32_t* __restrict__ start, int32_t bx,
-                                            int32_t by, const uint4 m, L&& ld, A&& ap)
-{
-    // a row outside the scene has no bits, and its start is not read
-    const uint32_t row0 = d.coff + (uint32_t)max(bx - 1, 0);
-    const uint32_t ncx  = (uint32_t)d.ncx;
-    uint32_t w1 = m.y, w2 = m.z;
-    uint32_t bits = m.x & ~MASK_BAD;
-    uint32_t base = bits ? __ldg(&start[row0 + (uint32_t)(by - 1) * ncx]) : 0u;
-    uint32_t b1   = w1 ? __ldg(&start[row0 + (uint32_t)by * ncx]) : 0u;
-    const uint32_t b2 = w2 ? __ldg(&start[row0 + (uint32_t)(by + 1) * ncx]) : 0u;
-    if (bits == 0u) {
-        bits = w1 ? w1 : w2;
-        base = w1 ? b1 : b2;
-        w1   = w1 ? w2 : 0u;
-        b1   = b2;
-        w2   = 0u;
+    const uint32_t cnt = (uint32_t)(__popc(w[0]) + __popc(w[1]) + __popc(w[2]));
+    fits               = fits && cnt <= LIST_MAX;
+    const uint32_t key = ldn<CG>(&k.keys[i]);
+    // a list built around another cell than the sort cell (or none) is not used later
+    const bool usable  = fits && key == d.coff + (uint32_t)by * (uint32_t)d.ncx + (uint32_t)bx;
+    k.nhdr[i] = make_uint4(key, cnt | (usable ? 0u : LIST_BAD), __float_as_uint(disp.x), __float_as_uint(disp.y));
+    if (!fits) {
+        for_neighbours_at(d, k, start, bx, by, ld, full);
+        return false;
     }
-    while (bits) {
-        const uint32_t t = (uint32_t)__ffs(bits) - 1u;
-        bits &= bits - 1u;
-        ap(base + t, ld(base + t));
+    // the rows run as one sequence: the next row with candidates takes over when a row's bits run out
+    uint32_t bits = w[0], base = b[0], w1 = w[1], b1 = b[1], w2 = w[2];
+    auto turn = [&]() {
         if (bits == 0u) {
             bits = w1 ? w1 : w2;
-            base = w1 ? b1 : b2;
+            base = w1 ? b1 : b[2];
             w1   = w1 ? w2 : 0u;
-            b1   = b2;
+            b1   = b[2];
             w2   = 0u;
+        }
+    };
+    turn();
+    for (uint32_t c = 0u; c < cnt; c += 4u) {
+        uint32_t j[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool v = bits != 0u;
+            j[q]         = v ? base + (uint32_t)__ffs(bits) - 1u : (uint32_t)i;
+            bits &= bits - 1u;
+            turn();
+        }
+        if (!k.wide) {
+            const uint32_t s = (uint32_t)i;
+            reinterpret_cast<uint2*>(k.nlist + (size_t)(c >> 3) * k.nstride + i)[(c >> 2) & 1u] =
+                make_uint2(__byte_perm(j[0] - s, j[1] - s, 0x5410), __byte_perm(j[2] - s, j[3] - s, 0x5410));
+        } else {
+            k.nlist[(size_t)(c >> 2) * k.nstride + i] = make_uint4(j[0], j[1], j[2], j[3]);
+        }
+        const auto q0 = ld(j[0]), q1 = ld(j[1]), q2 = ld(j[2]), q3 = ld(j[3]);
+        ap(j[0], q0, true);
+        ap(j[1], q1, c + 1u < cnt);
+        ap(j[2], q2, c + 2u < cnt);
+        ap(j[3], q3, c + 3u < cnt);
+    }
+    return self_in;
+}
+
+// Applies the cnt candidates of particle i's list in scan order, four at a time: their records' loads are in
+// flight together. w0 is the first chunk, loaded beside the header.
+template <bool CG, class L, class A>
+__device__ __forceinline__ void scan_list(const PbfK& k, int32_t i, uint32_t cnt, const uint4 w0, L&& ld, A&& ap)
+{
+    auto four = [&](uint32_t c, uint32_t j0, uint32_t j1, uint32_t j2, uint32_t j3) {
+        const auto q0 = ld(j0), q1 = ld(j1), q2 = ld(j2), q3 = ld(j3);
+        ap(j0, q0, true);
+        ap(j1, q1, c + 1u < cnt);
+        ap(j2, q2, c + 2u < cnt);
+        ap(j3, q3, c + 3u < cnt);
+    };
+    uint4 w          = w0;
+    const uint4* src = k.nlist + i;
+    if (!k.wide) {
+        auto lo = [&](uint32_t v) { return (uint32_t)(i + (int32_t)(int16_t)(v & 0xffffu)); };
+        auto hi = [&](uint32_t v) { return (uint32_t)(i + ((int32_t)v >> 16)); };
+        for (uint32_t c = 0u; c < cnt; c += 8u) {
+            if (c) {
+                src += k.nstride;
+                w = ldn<CG>(src);
+            }
+            four(c, lo(w.x), hi(w.x), lo(w.y), hi(w.y));
+            if (c + 4u < cnt) { four(c + 4u, lo(w.z), hi(w.z), lo(w.w), hi(w.w)); }
+        }
+    } else {
+        for (uint32_t c = 0u; c < cnt; c += 4u) {
+            if (c) {
+                src += k.nstride;
+                w = ldn<CG>(src);
+            }
+            four(c, w.x, w.y, w.z, w.w);
         }
     }
 }
 
-// The neighbour scan of particle i at (px, py) in mask mode MASK: ap(j, ld(j)) for every candidate j in
-// scan order. ap returns whether j lies within h + skin (used by MASK_BUILD only). Returns true when the
-// candidates came from the masks, which skip the particle's own slot: masks are used only while the
-// particle is in its sort cell, so the full scan would have met that slot.
-template <int MASK, bool CG, class L, class A, class AM>
-__device__ __forceinline__ bool scan_ld2(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start,
-                                         float px, float py, int32_t i, L&& ld, A&& ap, AM&& apm)
+// The neighbour scan of particle i at (px, py) in list mode LIST (LIST_OFF or LIST_USE): ap(j, ld(j)) for every
+// candidate j in scan order, or apl(j, ld(j), valid) for those of the list, which skip the particle's own slot:
+// true is returned then (lists are used only while the particle is in its sort cell, so the full scan would have
+// met that slot). valid is false for the filler (the particle itself) of the last group of four.
+template <int LIST, bool CG, class L, class A, class AL>
+__device__ __forceinline__ bool scan_ld(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start, float px,
+                                        float py, int32_t i, L&& ld, A&& ap, AL&& apl)
 {
-    auto f = [&](uint32_t j) -> bool { return ap(j, ld(j)); };
-    if constexpr (MASK == MASK_OFF) {
-        for_neighbours(d, k, start, px, py, f);
+    if constexpr (LIST == LIST_OFF) {
+        for_neighbours(d, k, start, px, py, [&](uint32_t j) { ap(j, ld(j), true); });
     } else {
+        const uint4 hd = ldn<CG>(&k.nhdr[i]);
+        const uint4 w0 = ldn<CG>(&k.nlist[i]);
+        const bool far     = ldn<CG>(&k.mflag[hd.x]) != 0;
         const int32_t bx   = cell_coord(px, d.ox, k.inv_cell, d.ncx);
         const int32_t by   = cell_coord(py, d.oy, k.inv_cell, d.ncy);
         const uint32_t key = d.coff + (uint32_t)by * (uint32_t)d.ncx + (uint32_t)bx;
-        if constexpr (MASK == MASK_BUILD) {
-            bool self_in;
-            uint4 m = scan_build(d, start, bx, by, i, self_in, f);
-            if (key != __ldg(&k.keys[i])) { m.x |= MASK_BAD; } // built around another cell than the sort cell
-            k.nmask[i] = m;
-        } else {
-            const uint4 m = ldn<CG>(&k.nmask[i]);
-            if (!(m.x & MASK_BAD) && key == __ldg(&k.keys[i]) && ldn<CG>(&k.mflag[key]) == 0) {
-                scan_masked(d, start, bx, by, m, ld, apm);
-                return true;
-            } else {
-                for_neighbours_at(d, k, start, bx, by, f);
-            }
+        if (!(hd.y & LIST_BAD) && key == hd.x && !far) {
+            scan_list<CG>(k, i, hd.y, w0, ld, apl);
+            return true;
         }
+        for_neighbours_at(d, k, start, bx, by, ld, ap);
     }
     return false;
 }
 
-// scan_ld2 with apm = ap. apm applies the candidates of masked scans, which never include the particle
-// itself, so it may leave out the self-pair test.
-template <int MASK, bool CG, class L, class A>
-__device__ __forceinline__ bool scan_ld(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start,
-                                        float px, float py, int32_t i, L&& ld, A&& ap)
-{
-    return scan_ld2<MASK, CG>(d, k, start, px, py, i, ld, ap, ap);
-}
-
-// scan_ld with one functor f(j) that loads and applies
-template <int MASK, bool CG, class F>
-__device__ __forceinline__ bool scan(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start, float px,
-                                     float py, int32_t i, F&& f)
-{
-    return scan_ld<MASK, CG>(d, k, start, px, py, i, [](uint32_t j) { return j; },
-                             [&](uint32_t j, uint32_t) -> bool { return f(j); });
-}
-
-// A delta p pass moved particle i (sort cell key) by at least skin / (2 iters): the particles of the 3 x 3
-// cells around its sort cell scan in full for the rest of the step.
+// A delta p pass left a particle (sort cell key) skin / 2 or more from where it was when the lists were made: the
+// particles of the 3 x 3 cells around its sort cell scan in full for the rest of the step.
 // Arguments by value: the call keeps them in registers (a reference would put the scene's DomDev on the stack).
 __device__ __noinline__ void mark_mover(uint8_t* __restrict__ mflag, uint32_t coff, int32_t ncx, int32_t ncy,
                                         uint32_t key)
@@ -371,14 +472,6 @@ __device__ __forceinline__ void hist_rank(uint32_t key, bool valid, uint2* __res
         const uint32_t rank = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
         keyrank[i]          = make_uint2(key, rank);
     }
-}
-
-// the sort cell key of predicted position ps in scene d
-__device__ __forceinline__ uint32_t cell_key(const PbfK& k, const DomDev& d, float2 ps)
-{
-    const int32_t cx = cell_coord(ps.x, d.ox, k.inv_cell, d.ncx);
-    const int32_t cy = cell_coord(ps.y, d.oy, k.inv_cell, d.ncy);
-    return d.coff + (uint32_t)cy * (uint32_t)d.ncx + (uint32_t)cx;
 }
 
 template <bool MULTI>
@@ -472,7 +565,7 @@ __global__ void __launch_bounds__(T_PART)
 //           unclamped, and the pass moves the particles by the change of L; a sum that overshot is relaxed
 //           again and L never turns into a pull (accumulated-multiplier clamping).
 enum { ACC_NONE = 0, ACC_SUM = 1, ACC_PROJ = 2 };
-template <bool MULTI, bool SELFG, int ACC, bool CG = false, int MASK = MASK_OFF>
+template <bool MULTI, bool SELFG, int ACC, bool CG = false, int LIST = LIST_OFF>
 __device__ __forceinline__ void lambda_one(const PbfK& k, const DomDev* __restrict__ doms,
                                            const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
                                            const float4* __restrict__ xd, float* __restrict__ lam,
@@ -493,18 +586,18 @@ __device__ __forceinline__ void lambda_one(const PbfK& k, const DomDev* __restri
     // Branch-free body: every lane of a warp runs the same instructions for every candidate and the terms of
     // pairs beyond h (and of the self pair) are masked to zero; a data-dependent accept branch here would
     // make each warp execute both paths on almost every iteration.
-    // ME: the candidate may be the particle itself (full scans); masked scans never visit it
-    auto body = [&](uint32_t j, const float4 q, auto me) -> bool {
+    // me: the candidate may be the particle itself (full scans); lists hold it only as filler (valid false)
+    auto body = [&](uint32_t j, const float4 q, auto me, bool valid) {
         const float2 r  = offset(px, pd, q);
         const float r2  = fmaf(r.x, r.x, r.y * r.y);
         const bool self = decltype(me)::value && j == (uint32_t)i;
         self_seen       = self_seen || self;
-        const bool in   = (r2 <= k.h2) && !self;
+        const bool in   = (r2 <= k.h2) && !self && valid;
         const bool dir  = in && (r2 > 1e-12f);
         const float qq  = in ? k.h2 - r2 : 0.f;
         s6              = fmaf(qq * qq, qq, s6);
-        const float inv = rsqrtf(dir ? r2 : 1.f);
-        const float dif = dir ? k.h - r2 * inv : 0.f;
+        const float inv = rsqrt_normal(dir ? r2 : 1.f);
+        const float dif = dir ? fmaf(-r2, inv, k.h) : 0.f;
         const float d2  = dif * dif;
         const float w   = d2 * inv;
         sg              = fma2(make_float2(w, w), r, sg);
@@ -521,36 +614,20 @@ __device__ __forceinline__ void lambda_one(const PbfK& k, const DomDev* __restri
             sg.y = fmaf(k.h2, ny, sg.y);
             s4 = fmaf(k.h2, k.h2, s4);
         }
-        return r2 < k.skin2;
     };
-    auto ld   = [&](uint32_t j) { return ldn<CG>(&xd[j]); };
-    auto full = [&](uint32_t j, const float4 q) -> bool { return body(j, q, std::true_type{}); };
-    auto near = [&](uint32_t j, const float4 q) -> bool { return body(j, q, std::false_type{}); };
-    if constexpr (MASK == MASK_BUILD) {
-        // Record the masks with a distance-only scan of the 3 x 3 cells, then apply the lambda terms to the
-        // recorded candidates alone (their loads hit L1): the same terms in the same order as the full
-        // scan, whose other candidates (beyond h, or the particle itself) add exact zeros.
-        const int32_t bx   = cell_coord(p.x, d.ox, k.inv_cell, d.ncx);
-        const int32_t by   = cell_coord(p.y, d.oy, k.inv_cell, d.ncy);
-        const uint32_t key = d.coff + (uint32_t)by * (uint32_t)d.ncx + (uint32_t)bx;
-        bool seen          = false;
-        uint4 m            = scan_build(d, start, bx, by, i, seen, [&](uint32_t j) -> bool {
-            const float2 r = offset(px, pd, ld(j));
+    const Records<CG> ld{xd};
+    auto full = [&](uint32_t j, const float4 q, bool valid) { body(j, q, std::true_type{}, valid); };
+    auto list = [&](uint32_t j, const float4 q, bool valid) { body(j, q, std::false_type{}, valid); };
+    bool listed;
+    if constexpr (LIST == LIST_BUILD) {
+        listed = scan_record<CG>(d, k, start, p.x, p.y, pd, i, [&](const float4 q) {
+            const float2 r = offset(px, pd, q);
             return fmaf(r.x, r.x, r.y * r.y) < k.skin2;
-        });
-        const bool fits = !(m.x & MASK_BAD); // no row held more candidates than a mask word
-        if (key != __ldg(&k.keys[i])) { m.x |= MASK_BAD; } // built around another cell than the sort cell
-        k.nmask[i] = m;
-        if (fits) {
-            scan_masked(d, start, bx, by, m, ld, near);
-            self_seen = seen;
-        } else {
-            for_neighbours_at(d, k, start, bx, by, [&](uint32_t j) { full(j, ld(j)); });
-        }
+        }, ld, list, full);
     } else {
-        const bool self_masked = scan_ld2<MASK, CG>(d, k, start, p.x, p.y, i, ld, full, near);
-        self_seen              = self_seen || self_masked;
+        listed = scan_ld<LIST, CG>(d, k, start, p.x, p.y, i, ld, full, list);
     }
+    self_seen = self_seen || listed;
     if (self_seen) {
         s6 = fmaf(k.h2 * k.h2, k.h2, s6);
         if (SELFG) {
@@ -582,22 +659,24 @@ __device__ __forceinline__ void lambda_one(const PbfK& k, const DomDev* __restri
     }
 }
 
-// the mask-recording pass in 40 registers (3 blocks of 512 per SM), the masked passes in 32
-template <bool MULTI, bool SELFG, int ACC, int MASK>
-__global__ void __launch_bounds__(T_MAX, (MASK == MASK_BUILD && !SELFG) ? 3 : (MASK == MASK_USE ? 4 : 1))
+// 40 registers (48 warps per SM) for the recording and the listed passes, although a few values spill there: 1M
+// particles 0.325 ms a pass against 0.343 at 64 registers; with pair directions the spills cost more than the
+// warps give (16,384 atoms in 20 substeps 0.88 against 0.79 ms)
+template <bool MULTI, bool SELFG, int ACC, int LIST>
+__global__ void __launch_bounds__(T_MAX, LIST == LIST_OFF ? 1 : (SELFG ? 2 : 3))
     k_lambda(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
              const uint32_t* __restrict__ start, const float4* __restrict__ xd, float* __restrict__ lam,
              const uint32_t* __restrict__ pair_id, float* __restrict__ acc)
 {
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count_of(k)) {
-        lambda_one<MULTI, SELFG, ACC, false, MASK>(k, doms, dom, start, xd, lam, pair_id, acc, i);
+        lambda_one<MULTI, SELFG, ACC, false, LIST>(k, doms, dom, start, xd, lam, pair_id, acc, i);
     }
 }
 
 // ----- delta p with artificial pressure and over-relaxation, then walls (PBF.cu:398-447, 471-499) -------
 // ACCINIT: this pass applies the warm start; its multiplier starts the step's running sum.
-template <bool MULTI, bool SCORR, bool ACCINIT, bool CG = false, int MASK = MASK_OFF>
+template <bool MULTI, bool SCORR, bool ACCINIT, bool CG = false, int LIST = LIST_OFF>
 __device__ __forceinline__ void delta_p_one(const PbfK& k, const DomDev* __restrict__ doms,
                                             const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
                                             const float4* __restrict__ xd, const float* __restrict__ lam,
@@ -614,14 +693,13 @@ __device__ __forceinline__ void delta_p_one(const PbfK& k, const DomDev* __restr
     // closer than 1e-6 (the self pair included) have a zero direction there and are skipped here.
     const float c6w = k.c6 * k.inv_w_dq;
     float2 sg = make_float2(0.f, 0.f); // (sx, sy)
-    scan_ld<MASK, CG>(d, k, start, p.x, p.y, i,
-                      [&](uint32_t j) { return Nbr{ldn<CG>(&xd[j]), ldn<CG>(&lam[j])}; },
-                      [&](uint32_t, const Nbr ql) -> bool {
+    // (a list's filler is the particle itself, which the direction test leaves out)
+    auto body = [&](const Nbr ql, bool valid) {
         const float lj  = ql.a;
         const float2 r  = offset(px, pd, ql.q);
         const float r2  = fmaf(r.x, r.x, r.y * r.y);
-        const bool ok   = (r2 <= k.h2) && (r2 > 1e-12f); // masked, branch-free (see k_lambda)
-        const float inv = rsqrtf(ok ? r2 : 1.f);
+        const bool ok   = (r2 <= k.h2) && (r2 > 1e-12f) && valid; // masked, branch-free (see k_lambda)
+        const float inv = rsqrt_normal(ok ? r2 : 1.f);
         float l         = fmaf(lj, k.mass, mli);
         if (SCORR) {
             const float qq    = k.h2 - r2;
@@ -629,11 +707,13 @@ __device__ __forceinline__ void delta_p_one(const PbfK& k, const DomDev* __restr
             const float r2q   = ratio * ratio;
             l                 = fmaf(-k.scorr_k, r2q * r2q, l);
         }
-        const float diff = k.h - r2 * inv;
+        const float diff = fmaf(-r2, inv, k.h);
         const float w    = ok ? diff * diff * inv * l : 0.f;
         sg               = fma2(make_float2(w, w), r, sg);
-        return false;
-    });
+    };
+    scan_ld<LIST, CG>(d, k, start, p.x, p.y, i, RecordsAnd<CG>{xd, lam},
+                      [&](uint32_t, const Nbr q, bool valid) { body(q, valid); },
+                      [&](uint32_t, const Nbr q, bool) { body(q, true); });
     const float s = -k.cs * k.dp_scale;
     // the correction moves the displacement; the position x + d is clamped to the walls (clamp<float>(v, lb,
     // ub), PBF.cu:496-497) by setting d = wall - x, exact next to the wall, so that x + d lands on it
@@ -642,21 +722,23 @@ __device__ __forceinline__ void delta_p_one(const PbfK& k, const DomDev* __restr
     dy = (oy > d.hiy) ? __fsub_rn(d.hiy, px.y) : ((oy < d.loy) ? __fsub_rn(d.loy, px.y) : dy);
     dx = (ox > d.hix) ? __fsub_rn(d.hix, px.x) : ((ox < d.lox) ? __fsub_rn(d.lox, px.x) : dx);
     xd_out[i] = make_float4(px.x, px.y, dx, dy);
-    if constexpr (MASK == MASK_USE) {
-        const float mx = dx - pd.x, my = dy - pd.y;
-        if (!(fmaf(mx, mx, my * my) < k.move2)) { mark_mover(k.mflag, d.coff, d.ncx, d.ncy, __ldg(&k.keys[i])); }
+    if constexpr (LIST == LIST_USE) {
+        // how far the particle is from where it was when the lists were made
+        const uint4 hd = ldn<CG>(&k.nhdr[i]);
+        const float mx = dx - __uint_as_float(hd.z), my = dy - __uint_as_float(hd.w);
+        if (!(fmaf(mx, mx, my * my) < k.move2)) { mark_mover(k.mflag, d.coff, d.ncx, d.ncy, hd.x); }
     }
 }
 
-template <bool MULTI, bool SCORR, bool ACCINIT, int MASK>
-__global__ void __launch_bounds__(T_MAX)
+template <bool MULTI, bool SCORR, bool ACCINIT, int LIST>
+__global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : 1)
     k_delta_p(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
               const uint32_t* __restrict__ start, const float4* __restrict__ xd, const float* __restrict__ lam,
               float4* __restrict__ xd_out, float* __restrict__ acc)
 {
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count_of(k)) {
-        delta_p_one<MULTI, SCORR, ACCINIT, false, MASK>(k, doms, dom, start, xd, lam, xd_out, acc, i);
+        delta_p_one<MULTI, SCORR, ACCINIT, false, LIST>(k, doms, dom, start, xd, lam, xd_out, acc, i);
     }
 }
 
@@ -664,7 +746,7 @@ __global__ void __launch_bounds__(T_MAX)
 // The lambda sums of k_lambda plus the neighbour count and the poly6-weighted sum of the neighbours'
 // lambda_prev; returns the cold first-iteration lambda and fills the network's 12 features (the order is
 // the one documented with gpe_pbf_set_warm_start).
-template <bool MULTI, bool SELFG, int MASK = MASK_OFF>
+template <bool MULTI, bool SELFG, int LIST = LIST_OFF>
 __device__ __forceinline__ float warm_features(const PbfK& k, const DomDev& d, const uint32_t* __restrict__ start,
                                                const float4* __restrict__ xd, const float* __restrict__ prev,
                                                const uint32_t* __restrict__ pair_id, int32_t i, uint32_t pbase,
@@ -677,22 +759,22 @@ __device__ __forceinline__ float warm_features(const PbfK& k, const DomDev& d, c
     float s4 = 0.f, s6 = 0.f, swl = 0.f;
     int32_t nn     = 0;
     bool self_seen = false;
-    // ME: the candidate may be the particle itself (full scans); masked scans never visit it
-    auto body = [&](uint32_t j, const Nbr ql, auto me) -> bool {
+    // me: the candidate may be the particle itself (full scans); lists hold it only as filler (valid false)
+    auto body = [&](uint32_t j, const Nbr ql, auto me, bool valid) {
         const float4 q  = ql.q;
         const float lp  = ql.a;
         const float2 r  = offset(px, pd, q);
         const float r2  = fmaf(r.x, r.x, r.y * r.y);
         const bool self = decltype(me)::value && j == (uint32_t)i;
         self_seen       = self_seen || self;
-        const bool in   = (r2 <= k.h2) && !self;
+        const bool in   = (r2 <= k.h2) && !self && valid;
         const bool dir  = in && (r2 > 1e-12f);
         const float qq  = in ? k.h2 - r2 : 0.f;
         s6              = fmaf(qq * qq, qq, s6); // as in k_lambda, so the cold lambda is bit-identical
         swl             = fmaf(qq * qq * qq, lp, swl);
         nn += in ? 1 : 0;
-        const float inv = rsqrtf(dir ? r2 : 1.f);
-        const float dif = dir ? k.h - r2 * inv : 0.f;
+        const float inv = rsqrt_normal(dir ? r2 : 1.f);
+        const float dif = dir ? fmaf(-r2, inv, k.h) : 0.f;
         const float d2  = dif * dif;
         const float w   = d2 * inv;
         sg              = fma2(make_float2(w, w), r, sg);
@@ -708,33 +790,17 @@ __device__ __forceinline__ float warm_features(const PbfK& k, const DomDev& d, c
             sg.y = fmaf(k.h2, ny, sg.y);
             s4 = fmaf(k.h2, k.h2, s4);
         }
-        return r2 < k.skin2;
     };
-    auto ld   = [&](uint32_t j) { return Nbr{__ldg(&xd[j]), __ldg(&prev[j])}; };
-    auto full = [&](uint32_t j, const Nbr q) -> bool { return body(j, q, std::true_type{}); };
-    auto near = [&](uint32_t j, const Nbr q) -> bool { return body(j, q, std::false_type{}); };
-    if constexpr (MASK == MASK_BUILD) {
-        // as in k_lambda: a distance-only scan records the masks, then the feature terms run over the
-        // recorded candidates alone (the full scan's other candidates add exact zeros)
-        const int32_t bx   = cell_coord(p.x, d.ox, k.inv_cell, d.ncx);
-        const int32_t by   = cell_coord(p.y, d.oy, k.inv_cell, d.ncy);
-        const uint32_t key = d.coff + (uint32_t)by * (uint32_t)d.ncx + (uint32_t)bx;
-        bool seen          = false;
-        uint4 m            = scan_build(d, start, bx, by, i, seen, [&](uint32_t j) -> bool {
-            const float2 r = offset(px, pd, __ldg(&xd[j]));
+    const RecordsAnd<false> ld{xd, prev};
+    auto full = [&](uint32_t j, const Nbr q, bool valid) { body(j, q, std::true_type{}, valid); };
+    if constexpr (LIST == LIST_BUILD) {
+        const bool listed = scan_record<false>(d, k, start, p.x, p.y, pd, i, [&](const float4 q) {
+            const float2 r = offset(px, pd, q);
             return fmaf(r.x, r.x, r.y * r.y) < k.skin2;
-        });
-        const bool fits = !(m.x & MASK_BAD);
-        if (key != __ldg(&k.keys[i])) { m.x |= MASK_BAD; } // built around another cell than the sort cell
-        k.nmask[i] = m;
-        if (fits) {
-            scan_masked(d, start, bx, by, m, ld, near);
-            self_seen = seen;
-        } else {
-            for_neighbours_at(d, k, start, bx, by, [&](uint32_t j) { full(j, ld(j)); });
-        }
+        }, ld, [&](uint32_t j, const Nbr q, bool valid) { body(j, q, std::false_type{}, valid); }, full);
+        self_seen = self_seen || listed;
     } else {
-        scan_ld<MASK, false>(d, k, start, p.x, p.y, i, ld, full);
+        for_neighbours(d, k, start, p.x, p.y, [&](uint32_t j) { full(j, ld(j), true); });
     }
     const float lpi = prev[i];
     if (self_seen) {
@@ -780,9 +846,9 @@ __device__ __forceinline__ float warm_features(const PbfK& k, const DomDev& d, c
 // particles is 4 KB at feat + t * 2048 in the tensor cores' K-major layout, so part 2 moves it to shared
 // memory with one bulk copy. (Computing the features inside the tensor-core kernel caps the neighbour loop
 // at the 7 CTAs of 4 warps that fit an SM beside their TMEM and operand tiles: 126 us against about 50 us
-// here at 1M particles.) With MASK_BUILD the pass records the step's candidate masks with a distance-only
-// scan and computes the features over the recorded candidates alone, as k_lambda does.
-template <bool MULTI, bool SELFG, int MASK>
+// here at 1M particles.) With LIST_BUILD the pass records the step's candidate lists and computes the features
+// over the recorded candidates alone, as k_lambda does.
+template <bool MULTI, bool SELFG, int LIST>
 __global__ void __launch_bounds__(T_PART)
     k_lambda_feat(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
                   const uint32_t* __restrict__ start, const float4* __restrict__ xd, const float* __restrict__ prev,
@@ -793,7 +859,7 @@ __global__ void __launch_bounds__(T_PART)
     const DomDev d       = load_dom<MULTI>(k, doms, dom, i);
     const uint32_t pbase = MULTI ? __ldg(&start[d.coff]) : 0u;
     float f[MLP_F];
-    (void)warm_features<MULTI, SELFG, MASK>(k, d, start, xd, prev, pair_id, i, pbase, f);
+    (void)warm_features<MULTI, SELFG, LIST>(k, d, start, xd, prev, pair_id, i, pbase, f);
     float mu[MLP_FP], isd[MLP_FP];
 #pragma unroll
     for (int q = 0; q < MLP_FP; ++q) {
@@ -909,7 +975,7 @@ __device__ __forceinline__ void velocity_clamp(const PbfK& k, float& vx, float& 
 }
 
 // ----- velocity + XSPH (+ vorticity omega) (PBF.cu:538, 585-627) ---------------------------------------
-template <bool MULTI, bool VORT, bool CG = false, int MASK = MASK_OFF>
+template <bool MULTI, bool VORT, bool CG = false, int LIST = LIST_OFF>
 __device__ __forceinline__ void xsph_one(const PbfK& k, const DomDev* __restrict__ doms,
                                          const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
                                          const float4* __restrict__ xd, float2* __restrict__ x_out,
@@ -926,16 +992,16 @@ __device__ __forceinline__ void xsph_one(const PbfK& k, const DomDev* __restrict
     // omega = sum (v_j - v_i) x grad_j W with grad_j W = +cs (h-r)^2 r/|r| (cs hoisted as well).
     float2 dvs = make_float2(0.f, 0.f); // (dvx, dvy)
     float w    = 0.f;
-    // ME: the candidate may be the particle itself (full scans); masked scans never visit it
-    auto xbody = [&](uint32_t j, const float4 q, auto me) -> bool {
+    // me: the candidate may be the particle itself (full scans); lists hold it only as filler (valid false)
+    auto xbody = [&](uint32_t j, const float4 q, auto me, bool valid) {
         const float2 r  = offset(px, pd, q);
         const float rx = r.x, ry = r.y;
         // explicit fused forms: the result must not depend on how the compiler contracts this body in the
         // kernel it is inlined into (separate launches and the persistent solve are compared bit for bit)
         const float r2  = fmaf(rx, rx, ry * ry);
         // masked, branch-free (see k_lambda); the self pair adds nothing in exact arithmetic (v_i - v_i) and is
-        // left out (masked scans skip the particle's own slot)
-        const bool in   = (r2 <= k.h2) && !(decltype(me)::value && j == (uint32_t)i);
+        // left out
+        const bool in   = (r2 <= k.h2) && valid && !(decltype(me)::value && j == (uint32_t)i);
         const float2 dv = fma2(d_of(q), make_float2(k.inv_dt, k.inv_dt), make_float2(-vax, -vay));
         const float dx = dv.x, dy = dv.y;
         const float qq  = in ? k.h2 - r2 : 0.f;
@@ -943,16 +1009,15 @@ __device__ __forceinline__ void xsph_one(const PbfK& k, const DomDev* __restrict
         dvs             = fma2(dv, make_float2(p6, p6), dvs);
         if (VORT) {
             const bool dir   = in && (r2 > 1e-12f);
-            const float inv  = rsqrtf(dir ? r2 : 1.f);
-            const float diff = k.h - r2 * inv;
+            const float inv  = rsqrt_normal(dir ? r2 : 1.f);
+            const float diff = fmaf(-r2, inv, k.h);
             const float gm   = dir ? diff * diff * inv : 0.f;
             w                = fmaf(gm, fmaf(dx, ry, -(dy * rx)), w);
         }
-        return false;
     };
-    scan_ld2<MASK, CG>(d, k, start, p.x, p.y, i, [&](uint32_t j) { return ldn<CG>(&xd[j]); },
-                       [&](uint32_t j, const float4 q) -> bool { return xbody(j, q, std::true_type{}); },
-                       [&](uint32_t j, const float4 q) -> bool { return xbody(j, q, std::false_type{}); });
+    scan_ld<LIST, CG>(d, k, start, p.x, p.y, i, Records<CG>{xd},
+                      [&](uint32_t j, const float4 q, bool valid) { xbody(j, q, std::true_type{}, valid); },
+                      [&](uint32_t j, const float4 q, bool valid) { xbody(j, q, std::false_type{}, valid); });
     w *= k.cs;
     const float cx = k.xsph_c * k.c6;
     float vx       = fmaf(dvs.x, cx, vax);
@@ -968,8 +1033,8 @@ __device__ __forceinline__ void xsph_one(const PbfK& k, const DomDev* __restrict
     if (next_key) { *next_key = cell_key(k, d, predict(k, p, make_float2(vx, vy))); }
 }
 
-template <bool MULTI, bool VORT, int MASK>
-__global__ void __launch_bounds__(T_MAX)
+template <bool MULTI, bool VORT, int LIST>
+__global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : 1)
     k_xsph(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
            const uint32_t* __restrict__ start, const float4* __restrict__ xd, float2* __restrict__ x_out,
            float2* __restrict__ v_out, float* __restrict__ omega, uint32_t* __restrict__ status)
@@ -977,7 +1042,7 @@ __global__ void __launch_bounds__(T_MAX)
     const int32_t i  = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < count_of(k);
     if (!k.hist_cnt) { // uniform
-        if (valid) { xsph_one<MULTI, VORT, false, MASK>(k, doms, dom, start, xd, x_out, v_out, omega, status, i); }
+        if (valid) { xsph_one<MULTI, VORT, false, LIST>(k, doms, dom, start, xd, x_out, v_out, omega, status, i); }
         return;
     }
     // XSPH of a step followed by another step without anything in between: the next step's cell keys and
@@ -985,12 +1050,12 @@ __global__ void __launch_bounds__(T_MAX)
     // from the same positions and velocities; only the order of the atomic ranks within a cell differs, which
     // the stable placement does not depend on)
     uint32_t key = 0xffffffffu;
-    if (valid) { xsph_one<MULTI, VORT, false, MASK>(k, doms, dom, start, xd, x_out, v_out, omega, status, i, &key); }
+    if (valid) { xsph_one<MULTI, VORT, false, LIST>(k, doms, dom, start, xd, x_out, v_out, omega, status, i, &key); }
     hist_rank(key, valid, k.hist_kr, k.hist_cnt, i);
 }
 
 // ----- vorticity confinement (Macklin & Mueller 2013 eq. 16) --------------------------------------------
-template <bool MULTI, bool CG = false, int MASK = MASK_OFF>
+template <bool MULTI, bool CG = false, int LIST = LIST_OFF>
 __device__ __forceinline__ void vorticity_one(const PbfK& k, const DomDev* __restrict__ doms,
                                               const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
                                               const float4* __restrict__ xd, const float* __restrict__ omega,
@@ -1003,20 +1068,20 @@ __device__ __forceinline__ void vorticity_one(const PbfK& k, const DomDev* __res
     const float wi = omega[i];
     const float aw = fabsf(wi);
     float2 eg = make_float2(0.f, 0.f); // (ex, ey)
-    scan_ld<MASK, CG>(d, k, start, p.x, p.y, i,
-                      [&](uint32_t j) { return Nbr{ldn<CG>(&xd[j]), ldn<CG>(&omega[j])}; },
-                      [&](uint32_t, const Nbr qw) -> bool {
+    auto body = [&](const Nbr qw, bool valid) { // (the direction test leaves out the particle itself)
         const float wj   = qw.a;
         const float2 r   = offset(px, pd, qw.q);
         const float rx = r.x, ry = r.y;
         const float r2   = fmaf(rx, rx, ry * ry); // explicit fused forms, as in xsph_one
-        const bool ok    = (r2 <= k.h2) && (r2 > 1e-12f); // masked, branch-free (see k_lambda)
-        const float inv  = rsqrtf(ok ? r2 : 1.f);
-        const float diff = k.h - r2 * inv;
+        const bool ok    = (r2 <= k.h2) && (r2 > 1e-12f) && valid; // masked, branch-free (see k_lambda)
+        const float inv  = rsqrt_normal(ok ? r2 : 1.f);
+        const float diff = fmaf(-r2, inv, k.h);
         const float dwg  = ok ? (fabsf(wj) - aw) * (diff * diff * inv) : 0.f; // grad_i W = -cs (...)
         eg               = fma2(make_float2(dwg, dwg), r, eg);
-        return false;
-    });
+    };
+    scan_ld<LIST, CG>(d, k, start, p.x, p.y, i, RecordsAnd<CG>{xd, omega},
+                      [&](uint32_t, const Nbr q, bool valid) { body(q, valid); },
+                      [&](uint32_t, const Nbr q, bool) { body(q, true); });
     // only the direction of eta = grad|omega| is used, so the positive factor cs drops out; the sign stays
     const float ex = -eg.x;
     const float ey = -eg.y;
@@ -1031,14 +1096,14 @@ __device__ __forceinline__ void vorticity_one(const PbfK& k, const DomDev* __res
     v[i] = vv;
 }
 
-template <bool MULTI, int MASK>
+template <bool MULTI, int LIST>
 __global__ void __launch_bounds__(T_MAX)
     k_vorticity(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
                 const uint32_t* __restrict__ start, const float4* __restrict__ xd,
                 const float* __restrict__ omega, float2* __restrict__ v)
 {
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count_of(k)) { vorticity_one<MULTI, false, MASK>(k, doms, dom, start, xd, omega, v, i); }
+    if (i < count_of(k)) { vorticity_one<MULTI, false, LIST>(k, doms, dom, start, xd, omega, v, i); }
 }
 
 // ----- the persistent solve: every Jacobi pass (and XSPH) of a step in one launch -----------------------
@@ -1153,7 +1218,7 @@ __global__ void k_barrier_selftest(GridSync* g, uint32_t* status)
     grid_barrier(g, gen, status, GRID_SELFTEST_NS);
 }
 
-template <bool MULTI, bool SELFG, bool SCORR, bool XSPH, bool MASKS>
+template <bool MULTI, bool SELFG, bool SCORR, bool XSPH, bool LISTS>
 __device__ __forceinline__ bool solve_phases(const PbfK& k, const DomDev* __restrict__ doms,
                                              const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
                                              float4* __restrict__ xd_a, float4* __restrict__ xd_b,
@@ -1166,11 +1231,11 @@ __device__ __forceinline__ bool solve_phases(const PbfK& k, const DomDev* __rest
     uint32_t tbase       = 0u;
     float4* cur          = xd_a;
     float4* nxt          = xd_b;
-    constexpr int MU = MASKS ? MASK_USE : MASK_OFF;
+    constexpr int MU = LISTS ? LIST_USE : LIST_OFF;
     for (int32_t it = 0; it < iters; ++it) {
-        if (MASKS && it == 0) {
+        if (LISTS && it == 0) {
             for_blocks(gs, tbase, n, [&](int32_t i) {
-                lambda_one<MULTI, SELFG, ACC_NONE, true, MASK_BUILD>(k, doms, dom, start, cur, lam, pair_id, nullptr, i);
+                lambda_one<MULTI, SELFG, ACC_NONE, true, LIST_BUILD>(k, doms, dom, start, cur, lam, pair_id, nullptr, i);
             });
         } else {
             for_blocks(gs, tbase, n, [&](int32_t i) {
@@ -1194,7 +1259,7 @@ __device__ __forceinline__ bool solve_phases(const PbfK& k, const DomDev* __rest
     return true;
 }
 
-template <bool MULTI, bool SELFG, bool SCORR, bool XSPH, bool MASKS>
+template <bool MULTI, bool SELFG, bool SCORR, bool XSPH, bool LISTS>
 __global__ void __launch_bounds__(T_MAX, 3)
     k_solve_persistent(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
                        const uint32_t* __restrict__ start, float4* __restrict__ xd_a, float4* __restrict__ xd_b,
@@ -1203,7 +1268,7 @@ __global__ void __launch_bounds__(T_MAX, 3)
                        uint32_t* __restrict__ status)
 {
     unsigned int gen = 0u; // the barrier word is zeroed before every launch
-    solve_phases<MULTI, SELFG, SCORR, XSPH, MASKS>(k, doms, dom, start, xd_a, xd_b, x_out, lam, pair_id, v, omega,
+    solve_phases<MULTI, SELFG, SCORR, XSPH, LISTS>(k, doms, dom, start, xd_a, xd_b, x_out, lam, pair_id, v, omega,
                                                    iters, gs, gen, status);
 }
 
@@ -1258,11 +1323,11 @@ struct SortBufs {
     uint32_t* keys;
     const uint32_t* id_in;   // ids to carry (or null)
     uint32_t* id_out;
-    uint8_t* mflag;          // candidate-mask cell marks to clear (or null)
+    uint8_t* mflag;          // candidate-list cell marks to clear (or null)
     uint32_t ncells;
 };
 
-template <bool MULTI, bool SELFG, bool SCORR, bool XSPH, bool MASKS>
+template <bool MULTI, bool SELFG, bool SCORR, bool XSPH, bool LISTS>
 __global__ void __launch_bounds__(T_MAX, 3)
     k_step_persistent(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
                       const SortBufs sb, float4* __restrict__ xd_b, float* __restrict__ lam,
@@ -1281,7 +1346,7 @@ __global__ void __launch_bounds__(T_MAX, 3)
         const int32_t i = base + (int32_t)threadIdx.x;
         predict_hist_one<MULTI>(k, doms, dom, sb.x, sb.v, sb.keyrank, sb.count, i, i < n);
     }
-    if (MASKS) {
+    if (LISTS) {
         for (uint32_t c = (uint32_t)i0; c < M; c += (uint32_t)stride) { sb.mflag[c] = 0u; }
     }
     if (!grid_barrier(gs, gen, status)) { return; }
@@ -1344,7 +1409,7 @@ __global__ void __launch_bounds__(T_MAX, 3)
     }
     // (every block has read its unsorted positions before this barrier; XSPH overwrites them later)
     if (!grid_barrier(gs, gen, status)) { return; }
-    solve_phases<MULTI, SELFG, SCORR, XSPH, MASKS>(k, doms, dom, sb.start, sb.xd_sorted, xd_b, sb.x, lam, pair_id,
+    solve_phases<MULTI, SELFG, SCORR, XSPH, LISTS>(k, doms, dom, sb.start, sb.xd_sorted, xd_b, sb.x, lam, pair_id,
                                                    v_out, omega, iters, gs, gen, status);
 }
 
@@ -1708,14 +1773,14 @@ struct gpe_pbf {
     const void* coop_fn = nullptr; // the kernel coop_grid was sized for
     GridSync* gsync   = nullptr;  // its barrier word
     uint16_t* feat    = nullptr;  // network operand tiles (GPE_WARM_MLP), allocated on demand
-    float skin        = 0.075f;   // candidate-mask skin in units of h (tuning; 0: full scans only)
-    uint4* nmask      = nullptr;  // candidate masks of the current step
-    uint8_t* mflag    = nullptr;  // per cell: a particle of its 3 x 3 cells moved too far for the masks
-    bool masks_valid  = false;    // the masks were made in this step
+    float skin        = 0.075f;   // candidate-list skin in units of h (tuning; 0: full scans only)
+    uint4* nhdr       = nullptr;  // candidate lists of the current step: headers
+    uint4* nlist      = nullptr;  // ... and chunks, an allocation of their own (null: none, full scans only)
+    bool wide         = false;    // ... of 32-bit slots
+    uint8_t* mflag    = nullptr;  // per cell: a particle of its 3 x 3 cells moved too far for the lists
+    bool lists_valid  = false;    // the lists were made in this step
     bool hist_ready   = false;    // the last step's XSPH left the next step's cell keys and histogram
     bool count_dirty  = false;    // ... and was dropped: the histogram array must be cleared before a sort
-    int32_t dp_since_build = 0;   // delta p passes since they were made
-    int32_t mask_passes = 1;      // delta p passes the move threshold k.move2 allows for
 
     // within a step (after PREDICT_SORT): XS = the current (x, d) records, XO = the other buffer; -1 between steps
     int XS = -1, XO = -1;
@@ -1794,25 +1859,26 @@ PbfK make_k(const gpe_pbf_params& p)
     return k;
 }
 
-// the engine's buffers and mask thresholds in the kernel constants
+// the engine's buffers and list thresholds in the kernel constants
 void bind_k(gpe_pbf* s)
 {
     s->k.n_dev       = s->d_count;
     s->k.ncells      = s->ncells;
     s->k.keys        = s->keys;
-    s->k.nmask       = s->nmask;
+    s->k.nhdr        = s->nhdr;
+    s->k.nlist       = s->nlist;
+    s->k.nstride     = s->cap;
+    s->k.wide        = s->wide ? 1 : 0;
     s->k.mflag       = s->mflag;
     const float skin = s->skin * s->prm.h;
     s->k.skin2       = (s->prm.h + skin) * (s->prm.h + skin);
-    // each of the step's delta p passes may move a particle by less than this, so all of them together
-    // by less than skin / 2 (with 5% to spare for rounding)
-    s->mask_passes   = std::max(s->prm.iters, 1);
-    const float mv   = 0.95f * skin / (2.f * (float)s->mask_passes);
+    // a particle may be less than skin / 2 from where it was when the lists were made (5% to spare for rounding)
+    const float mv   = 0.95f * 0.5f * skin;
     s->k.move2       = mv * mv;
 }
 
-// masks in this engine's configuration: cell h (3 x 3 scan), a skin, at least one iteration
-bool masks_on(const gpe_pbf* s) { return s->skin > 0.f && s->k.R == 1 && s->prm.iters > 0; }
+// lists in this engine's configuration: cell h (3 x 3 scan), a skin, at least one iteration
+bool lists_on(const gpe_pbf* s) { return s->nlist && s->skin > 0.f && s->k.R == 1 && s->prm.iters > 0; }
 
 // Cells along one edge of a scene; -1 when extent / cell is not finite or reaches 2^30 (the cast to int32
 // would be undefined there). Scene extents are checked to be > 0 before this is called.
@@ -1907,7 +1973,7 @@ int32_t clear_hist(gpe_pbf* s, cudaStream_t st)
 
 int32_t stage_predict_sort(gpe_pbf* s, cudaStream_t st)
 {
-    s->masks_valid  = false;
+    s->lists_valid  = false;
     const int32_t n = (int32_t)lsize(s);
     s->XS           = 0;
     s->XO           = 1;
@@ -1927,8 +1993,8 @@ int32_t stage_predict_sort(gpe_pbf* s, cudaStream_t st)
         }
         GPE_CHECK_LAUNCH("k_predict_hist");
     }
-    // the scan also clears the candidate masks' cell marks for this step
-    int32_t rc = launch_exclusive_scan(s->count, s->ncells, s->bsum, s->start, st, masks_on(s) ? s->mflag : nullptr);
+    // the scan also clears the candidate lists' cell marks for this step
+    int32_t rc = launch_exclusive_scan(s->count, s->ncells, s->bsum, s->start, st, lists_on(s) ? s->mflag : nullptr);
     if (rc) { return rc; }
     rc = launch_scatter(s->keyrank, n, s->start, s->bucket, (uint32_t)s->ncells, st, s->d_count);
     if (rc) { return rc; }
@@ -1953,19 +2019,19 @@ using LamFn = cudaError_t (*)(unsigned, unsigned, cudaStream_t, const PbfK&, con
                        const float4*, float*, const uint32_t*, float*, int);
 template <bool M, bool S, int A>
 cudaError_t lam_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
-                const uint32_t* start, const float4* xs, float* lam, const uint32_t* pid, float* acc, int mask)
+                const uint32_t* start, const float4* xs, float* lam, const uint32_t* pid, float* acc, int list)
 {
     if constexpr (A == ACC_PROJ) { // the projected-increment ablation keeps full scans
-        k_lambda<M, S, A, MASK_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
+        k_lambda<M, S, A, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
         return cudaGetLastError();
-    } else if (mask == MASK_BUILD) {
-        k_lambda<M, S, A, MASK_BUILD><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
+    } else if (list == LIST_BUILD) {
+        k_lambda<M, S, A, LIST_BUILD><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
         return cudaGetLastError();
-    } else if (mask == MASK_USE) {
-        k_lambda<M, S, A, MASK_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
+    } else if (list == LIST_USE) {
+        k_lambda<M, S, A, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
         return cudaGetLastError();
     } else {
-        k_lambda<M, S, A, MASK_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
+        k_lambda<M, S, A, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
         return cudaGetLastError();
     }
 }
@@ -1978,13 +2044,13 @@ using DpFn = cudaError_t (*)(unsigned, unsigned, cudaStream_t, const PbfK&, cons
                       const float4*, const float*, float4*, float*, int);
 template <bool M, bool S, bool A>
 cudaError_t dp_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
-               const uint32_t* start, const float4* xs, const float* lam, float4* out, float* acc, int mask)
+               const uint32_t* start, const float4* xs, const float* lam, float4* out, float* acc, int list)
 {
-    if (mask == MASK_USE) {
-        k_delta_p<M, S, A, MASK_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
+    if (list == LIST_USE) {
+        k_delta_p<M, S, A, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
         return cudaGetLastError();
     } else {
-        k_delta_p<M, S, A, MASK_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
+        k_delta_p<M, S, A, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
         return cudaGetLastError();
     }
 }
@@ -1998,12 +2064,12 @@ using FeatFn = void (*)(unsigned, unsigned, cudaStream_t, const PbfK&, const Dom
 template <bool M, bool S>
 void feat_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
                  const uint32_t* start, const float4* xd, const float* prev, const uint32_t* pid, const MlpDev* mlp,
-                 uint16_t* feat, int mask)
+                 uint16_t* feat, int list)
 {
-    if (mask == MASK_BUILD) {
-        k_lambda_feat<M, S, MASK_BUILD><<<g, blk, 0, st>>>(k, doms, dom, start, xd, prev, pid, mlp, feat);
+    if (list == LIST_BUILD) {
+        k_lambda_feat<M, S, LIST_BUILD><<<g, blk, 0, st>>>(k, doms, dom, start, xd, prev, pid, mlp, feat);
     } else {
-        k_lambda_feat<M, S, MASK_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xd, prev, pid, mlp, feat);
+        k_lambda_feat<M, S, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xd, prev, pid, mlp, feat);
     }
 }
 const FeatFn kFeat[2][2] = {{feat_launch<false, false>, feat_launch<false, true>},
@@ -2026,13 +2092,13 @@ using XsFn = cudaError_t (*)(unsigned, unsigned, cudaStream_t, const PbfK&, cons
 template <bool M, bool V>
 cudaError_t xs_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
                const uint32_t* start, const float4* xd, float2* x_out, float2* v, float* om, uint32_t* status,
-               int mask)
+               int list)
 {
-    if (mask == MASK_USE) {
-        k_xsph<M, V, MASK_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
+    if (list == LIST_USE) {
+        k_xsph<M, V, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
         return cudaGetLastError();
     } else {
-        k_xsph<M, V, MASK_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
+        k_xsph<M, V, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
         return cudaGetLastError();
     }
 }
@@ -2053,17 +2119,16 @@ int32_t stage_lambda(gpe_pbf* s, cudaStream_t st, int acc)
     if (lsize(s) == 0) { return GPE_OK; }
     const int sg        = (s->prm.flags & GPE_PBF_SELF_GRAD) ? 1 : 0;
     const uint32_t* pid = (s->prm.flags & GPE_PBF_PAIR_IDS) ? s->ids[s->id_cur] : nullptr;
-    int mask = MASK_OFF;
-    if (masks_on(s) && acc != ACC_PROJ) {
+    int list = LIST_OFF;
+    if (lists_on(s) && acc != ACC_PROJ) {
         // the cell marks were cleared by this step's sort (marks left by a stage sequence without one only
         // make scans full, never skip a candidate)
-        mask = s->masks_valid ? MASK_USE : MASK_BUILD;
+        list = s->lists_valid ? LIST_USE : LIST_BUILD;
     }
     GPE_TRY_CUDA(kLam[multi(s) ? 1 : 0][sg][acc](nblk(s), (unsigned)s->block, st, s->k, s->d_doms, s->dom, s->start,
-                                                 s->xd[s->XS], s->lam, pid, s->acc, mask));
-    if (mask == MASK_BUILD) {
-        s->masks_valid    = true;
-        s->dp_since_build = 0;
+                                                 s->xd[s->XS], s->lam, pid, s->acc, list));
+    if (list == LIST_BUILD) {
+        s->lists_valid = true;
     }
     s->launches += 1;
     return GPE_OK;
@@ -2081,14 +2146,13 @@ int32_t stage_lambda_warm(gpe_pbf* s, cudaStream_t st)
     const uint32_t* pid = (s->prm.flags & GPE_PBF_PAIR_IDS) ? s->ids[s->id_cur] : nullptr;
     if (s->warm == GPE_WARM_MLP && s->mem_valid && !s->collecting) {
         const gpe::MlpDev* md = gpe::mlp_device(s->mlp);
-        // the feature pass scans every neighbour on the sorted positions: it makes the step's masks
-        const int mask = masks_on(s) ? MASK_BUILD : MASK_OFF;
+        // the feature pass scans every neighbour on the sorted positions: it makes the step's lists
+        const int list = lists_on(s) ? LIST_BUILD : LIST_OFF;
         kFeat[mi][sg](nblk(s), (unsigned)s->block, st, s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev, pid,
-                      md, s->feat, mask);
+                      md, s->feat, list);
         GPE_CHECK_LAUNCH("k_lambda_feat");
-        if (mask == MASK_BUILD) {
-            s->masks_valid    = true;
-            s->dp_since_build = 0;
+        if (list == LIST_BUILD) {
+            s->lists_valid = true;
         }
         const int64_t tiles = (lsize(s) + MLP_TILE - 1) / MLP_TILE;
         const unsigned g    = (unsigned)std::min<int64_t>(tiles, s->lam_grid);
@@ -2108,14 +2172,10 @@ int32_t stage_delta_p(gpe_pbf* s, cudaStream_t st, bool accinit)
 {
     if (lsize(s) > 0) {
         const int sc = s->prm.scorr_k != 0.f ? 1 : 0;
-        // the move threshold covers mask_passes passes after the masks were made (a step with more
-        // iterations, such as the one that starts the network's memory, scans in full after those)
-        if (s->masks_valid && s->dp_since_build >= s->mask_passes) { s->masks_valid = false; }
-        const int mask = s->masks_valid ? MASK_USE : MASK_OFF;
-        s->dp_since_build += 1;
+        const int list = s->lists_valid ? LIST_USE : LIST_OFF;
         GPE_TRY_CUDA(kDp[multi(s) ? 1 : 0][sc][accinit ? 1 : 0](nblk(s), (unsigned)s->block, st, s->k, s->d_doms,
                                                                 s->dom, s->start, s->xd[s->XS], s->lam,
-                                                                s->xd[s->XO], s->acc, mask));
+                                                                s->xd[s->XO], s->acc, list));
         s->launches += 1;
     }
     std::swap(s->XS, s->XO);
@@ -2136,7 +2196,7 @@ int32_t stage_xsph(gpe_pbf* s, cudaStream_t st, bool next_hist = false)
     }
     GPE_TRY_CUDA(kXs[multi(s) ? 1 : 0][vort](nblk(s), (unsigned)s->block, st, kk, s->d_doms, s->dom, s->start,
                                              s->xd[s->XS], s->pos, s->vel, s->omega, s->status,
-                                             s->masks_valid ? MASK_USE : MASK_OFF));
+                                             s->lists_valid ? LIST_USE : LIST_OFF));
     s->launches += 1;
     s->hist_ready = next_hist;
     return GPE_OK;
@@ -2147,21 +2207,21 @@ int32_t stage_vorticity(gpe_pbf* s, cudaStream_t st)
 {
     if (lsize(s) == 0 || s->prm.vort_eps == 0.f) { return GPE_OK; }
     const unsigned g = nblk(s);
-    const bool mu = s->masks_valid;
+    const bool mu = s->lists_valid;
     if (multi(s)) {
         if (mu) {
-            k_vorticity<true, MASK_USE><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
+            k_vorticity<true, LIST_USE><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
                                                                          s->xd[s->XS], s->omega, s->vel);
         } else {
-            k_vorticity<true, MASK_OFF><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
+            k_vorticity<true, LIST_OFF><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
                                                                          s->xd[s->XS], s->omega, s->vel);
         }
     } else {
         if (mu) {
-            k_vorticity<false, MASK_USE><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
+            k_vorticity<false, LIST_USE><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
                                                                           s->xd[s->XS], s->omega, s->vel);
         } else {
-            k_vorticity<false, MASK_OFF><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
+            k_vorticity<false, LIST_OFF><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
                                                                           s->xd[s->XS], s->omega, s->vel);
         }
     }
@@ -2173,7 +2233,7 @@ int32_t stage_vorticity(gpe_pbf* s, cudaStream_t st)
 int32_t stage_finish(gpe_pbf* s)
 {
     // XSPH wrote the step's end positions (sorted) into pos
-    s->masks_valid = false;
+    s->lists_valid = false;
     s->XS = s->XO = -1;
     return GPE_OK;
 }
@@ -2202,7 +2262,7 @@ const void* solve_kernel(const gpe_pbf* s)
 {
     const bool m = multi(s), sg = (s->prm.flags & GPE_PBF_SELF_GRAD) != 0, sc = s->prm.scorr_k != 0.f,
                v = s->prm.vort_eps == 0.f; // XSPH inside the kernel
-    return masks_on(s) ? solve_kernel_k<true>(m, sg, sc, v) : solve_kernel_k<false>(m, sg, sc, v);
+    return lists_on(s) ? solve_kernel_k<true>(m, sg, sc, v) : solve_kernel_k<false>(m, sg, sc, v);
 }
 
 // Blocks of a persistent launch: one per block of particles, at most as many as are resident at once (a
@@ -2232,7 +2292,7 @@ int32_t stage_solve_persistent(gpe_pbf* s, cudaStream_t st)
         void* args[]        = {&k,  &s->d_doms, &s->dom, &s->start, &xa,   &xb,        &xo,
                                &s->lam, &pid, &s->vel, &s->omega, &iters, &s->gsync, &s->status};
         GPE_TRY_CUDA(cudaMemsetAsync(s->gsync, 0, sizeof(GridSync), st));
-        if (masks_on(s)) { GPE_TRY_CUDA(cudaMemsetAsync(s->mflag, 0, (size_t)s->ncells, st)); }
+        if (lists_on(s)) { GPE_TRY_CUDA(cudaMemsetAsync(s->mflag, 0, (size_t)s->ncells, st)); }
         GPE_TRY_CUDA(cudaLaunchCooperativeKernel(fn, dim3(coop_blocks(s)), dim3((unsigned)s->block), args, 0, st));
         s->launches += 1;
     }
@@ -2267,7 +2327,7 @@ int32_t stage_step_persistent(gpe_pbf* s, cudaStream_t st)
     drop_hist(s); // its sort phases build their own histogram
     const int32_t rch = clear_hist(s, st);
     if (rch) { return rch; }
-    s->masks_valid = false;
+    s->lists_valid = false;
     s->XS  = 0;
     s->XO  = 1;
     s->k.n = (int32_t)s->n;
@@ -2275,7 +2335,7 @@ int32_t stage_step_persistent(gpe_pbf* s, cudaStream_t st)
     if (lsize(s) > 0) {
         const bool m = multi(s), sg = (s->prm.flags & GPE_PBF_SELF_GRAD) != 0, sc = s->prm.scorr_k != 0.f,
                    v = s->prm.vort_eps == 0.f; // XSPH inside the kernel
-        const void* fn = masks_on(s) ? step_kernel_k<true>(m, sg, sc, v) : step_kernel_k<false>(m, sg, sc, v);
+        const void* fn = lists_on(s) ? step_kernel_k<true>(m, sg, sc, v) : step_kernel_k<false>(m, sg, sc, v);
         if (s->coop_grid <= 0 || s->coop_fn != fn) {
             s->coop_fn = fn;
             int per_sm = 0;
@@ -2295,7 +2355,7 @@ int32_t stage_step_persistent(gpe_pbf* s, cudaStream_t st)
         sb.keys      = s->keys;
         sb.id_in     = ids ? s->ids[s->id_cur] : nullptr;
         sb.id_out    = ids ? s->ids[s->id_cur ^ 1] : nullptr;
-        sb.mflag     = masks_on(s) ? s->mflag : nullptr;
+        sb.mflag     = lists_on(s) ? s->mflag : nullptr;
         sb.ncells    = (uint32_t)s->ncells;
         const uint32_t* pid = (s->prm.flags & GPE_PBF_PAIR_IDS) ? sb.id_out : nullptr;
         PbfK k              = s->k;
@@ -2371,8 +2431,8 @@ int32_t alloc_buffers(gpe_pbf* s)
     Carver c;
     const size_t o_doms = c.take<DomDev>((size_t)s->nd);
     const size_t o_pos   = c.take<float2>(N);
-    const size_t o_xd0   = c.take<float4>(N);
-    const size_t o_xd1   = c.take<float4>(N);
+    const size_t o_xd0   = c.take<float4>(N + 3); // (scan_record reads up to three records past a row)
+    const size_t o_xd1   = c.take<float4>(N + 3);
     const size_t o_vel   = c.take<float2>(N);
     const size_t o_lam   = c.take<float>(N);
     const size_t o_om    = c.take<float>(N);
@@ -2422,8 +2482,18 @@ int32_t alloc_buffers(gpe_pbf* s)
     s->acc     = reinterpret_cast<float*>(b + o_acc);
     s->prev    = reinterpret_cast<float*>(b + o_prev);
     s->gsync   = reinterpret_cast<GridSync*>(b + o_gs);
-    s->nmask   = reinterpret_cast<uint4*>(b + o_nm);
+    s->nhdr   = reinterpret_cast<uint4*>(b + o_nm);
     s->mflag   = b + o_mf;
+    // Candidate lists: 96 bytes a particle, 192 with 32-bit slots, of which a step touches what its lists fill (32 on
+    // a lattice of spacing h / 2). Slots of 16 bits reach 2^15 away: the next cell row of a scene 4096 cells wide
+    // at up to 8 particles a cell; wider scenes take 32-bit slots. Without room for them the passes scan in full.
+    float widest = 0.f;
+    for (const gpe_domain& d : s->doms) { widest = std::max(widest, d.extent[0]); }
+    s->wide = widest > 4096.f * s->prm.h;
+    if (cudaMalloc(&s->nlist, sizeof(uint4) * (LIST_MAX / (s->wide ? 4 : 8)) * std::max<size_t>(N, 1)) != cudaSuccess) {
+        cudaGetLastError();
+        s->nlist = nullptr;
+    }
     bind_k(s);
     GPE_TRY_CUDA(cudaMemcpy(s->d_doms, s->domdev.data(), sizeof(DomDev) * (size_t)s->nd, cudaMemcpyHostToDevice));
     return GPE_OK;
@@ -2488,6 +2558,7 @@ int32_t gpe_pbf_create(const gpe_pbf_params* params, const gpe_domain* domains, 
     rc = alloc_buffers(s);
     if (rc) {
         if (s->base) { cudaFree(s->base); }
+        if (s->nlist) { cudaFree(s->nlist); }
         delete s;
         return rc;
     }
@@ -2500,6 +2571,7 @@ int32_t gpe_pbf_destroy(gpe_pbf* s)
     if (!s) { return GPE_ERR_BAD_ARG; }
     s->drop_graphs();
     if (s->base) { cudaFree(s->base); }
+    if (s->nlist) { cudaFree(s->nlist); }
     if (s->feat) { cudaFree(s->feat); }
     delete s;
     return GPE_OK;
@@ -2920,7 +2992,7 @@ int32_t gpe_pbf_set_field(gpe_pbf* s, int32_t field, const void* src, int64_t n_
         gpe::set_error(GPE_ERR_BAD_ARG, "gpe_pbf_set_field: field %d is derived and read-only", field);
         return GPE_ERR_BAD_ARG;
     }
-    s->masks_valid = false; // a written position (or anything else) may move a particle past its masks
+    s->lists_valid = false; // a written position (or anything else) may move a particle past its lists
     drop_hist(s);
     FieldLoc f{};
     int32_t rc = field_ptr(s, field, &f);
@@ -3294,7 +3366,7 @@ extern "C" int32_t gpe_pbf_autotune(gpe_pbf* s, int32_t trial_steps, gpe_pbf_tun
         gpe_pbf_status(s, &stt, stream);
         return stt != 0 ? -1.f : ms / (float)trial_steps;
     };
-    // cell h with candidate masks (skin 0.1, 0.075 or 0.05 h) and without, and h/2 (no masks: its scan has
+    // cell h with candidate lists (skin 0.1, 0.075 or 0.05 h) and without, and h/2 (no lists: its scan has
     // five rows)
     const float cells[5] = {s->prm.h, s->prm.h, s->prm.h, s->prm.h, 0.5f * s->prm.h};
     const float skins[5] = {0.1f, 0.075f, 0.05f, 0.f, 0.f};

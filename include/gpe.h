@@ -364,19 +364,19 @@ typedef struct gpe_pbf_tuning {
                            five launches), so a plain step is one launch; 0: one launch per pass
                            (on a GB300, 0 measured fastest for 16k and 1M particles and 256 scenes, by
                            15-30%; the autotuner times all three)                                       */
-    float skin;         /* candidate masks, in units of h, in [0, 1] (cell h only; default 0.075): the
+    float skin;         /* candidate lists, in units of h, in [0, 1] (cell h only; default 0.075): the
                            first lambda pass of a step records per particle which candidates of its
                            3 x 3 cells lie within h + skin * h, and the later passes of the step visit
-                           only those while no particle nearby has moved by skin * h / 2 (else that
-                           particle's neighbourhood scans in full). Same result bit for bit; 0 turns
-                           the masks off                                                                */
+                           only those while no particle nearby is skin * h / 2 or more from where it was
+                           then (else that particle's neighbourhood scans in full). Same result bit for
+                           bit; 0 turns the lists off                                                   */
 } gpe_pbf_tuning;
 
 int32_t gpe_pbf_get_tuning(const gpe_pbf* pbf, gpe_pbf_tuning* tuning);
 /* A new cell size rebuilds the scenes' sort grids (the engine holds cell arrays for h/2 and for the cell
  * size it was created with). */
 int32_t gpe_pbf_set_tuning(gpe_pbf* pbf, const gpe_pbf_tuning* tuning);
-/* Times trial_steps steps of every candidate (cell h with mask skin 0.1, 0.075 or 0.05 or without masks,
+/* Times trial_steps steps of every candidate (cell h with list skin 0.1, 0.075 or 0.05 or without lists,
  * or h/2; block 128, 256 or 512; persistent 0, 1 or 2) on the current state, which is restored after every
  * trial and at the end; the three fastest run three more trials each, taking turns, and the one with the
  * smallest median time is applied;
