@@ -159,6 +159,24 @@ struct RecordsAnd {
     __device__ __forceinline__ Nbr operator()(uint32_t j) const { return Nbr{ldn<CG>(&xd[j]), ldn<CG>(&a[j])}; }
 };
 
+// What a pass's pair terms need of the particle itself: its record and one more value (a).
+struct Self {
+    int32_t i;
+    float2 px, pd;
+    float a;
+};
+
+// A pass over neighbours is a type P: P::Acc, the particle's sums; term(self, record, valid), the pair's term, all
+// zero beyond h or when !valid, with term.hit telling whether it is not; add(acc, term, i, j), which adds it. Every
+// lane of a warp runs the same instructions for every candidate; a data-dependent accept branch would make each
+// warp execute both paths on almost every iteration. The sums are taken in slot order in every scan below, with
+// explicit fused forms, so that they round alike wherever a pass is inlined.
+
+__device__ __forceinline__ float2 shfl2(uint32_t mask, float2 v, int src)
+{
+    return make_float2(__shfl_sync(mask, v.x, src), __shfl_sync(mask, v.y, src));
+}
+
 // Visits every particle index in the cells within R of the base cell of (px, py) (the reference scans the
 // 3x3 cells around clamp(floorf(x)/kCellDim), PBF.cu:252-263). Each row of cells is one contiguous range.
 template <class F>
@@ -180,32 +198,107 @@ __device__ __forceinline__ void for_neighbours(const DomDev& d, const PbfK& k, c
     }
 }
 
-// The same candidates in the same order from base cell (bx, by), four at a time so that their records' loads are in
-// flight together: ap(j, ld(j), valid), the last candidate of a row standing in (valid false) for those that the
-// row's last four lack.
-template <class L, class A>
-__device__ __forceinline__ void for_neighbours_at(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start,
-                                                  int32_t bx, int32_t by, L&& ld, A&& ap)
+// the slots of the three cell rows around base cell (bx, by), R = 1: row r holds n[r] slots from b[r]
+struct Rows {
+    uint32_t b[3], n[3];
+    __device__ __forceinline__ Rows(const DomDev& d, const uint32_t* __restrict__ start, int32_t bx, int32_t by)
+    {
+        const int32_t x0 = max(bx - 1, 0);
+        const int32_t x1 = min(bx + 1, d.ncx - 1);
+#pragma unroll
+        for (int32_t r = 0; r < 3; ++r) {
+            const int32_t y    = by - 1 + r;
+            const bool in      = y >= 0 && y < d.ncy;
+            const uint32_t row = d.coff + (uint32_t)(in ? y : by) * (uint32_t)d.ncx;
+            b[r]               = __ldg(&start[row + x0]);
+            n[r]               = in ? __ldg(&start[row + x1 + 1]) - b[r] : 0u;
+        }
+    }
+};
+
+// Every candidate of particle me.i around base cell (bx, by), R = 1, four at a time so that their records' loads are
+// in flight together (the last candidate of a row stands in for those that the row's last four lack). Returns
+// whether the rows hold the particle's own slot.
+template <class P, class L>
+__device__ __forceinline__ bool scan_full(const DomDev& d, const uint32_t* __restrict__ start, int32_t bx, int32_t by,
+                                          const Self& me, const L& ld, const P& pass, typename P::Acc& acc)
 {
-    const int32_t x0 = max(bx - k.R, 0);
-    const int32_t x1 = min(bx + k.R, d.ncx - 1);
-    const int32_t y0 = max(by - k.R, 0);
-    const int32_t y1 = min(by + k.R, d.ncy - 1);
-    for (int32_t y = y0; y <= y1; ++y) {
-        const uint32_t row = d.coff + (uint32_t)y * (uint32_t)d.ncx;
-        const uint32_t b   = __ldg(&start[row + x0]);
-        const uint32_t e   = __ldg(&start[row + x1 + 1]);
+    const Rows rows(d, start, bx, by);
+    const uint32_t i = (uint32_t)me.i;
+    bool self_in     = false;
+#pragma unroll 1
+    for (int r = 0; r < 3; ++r) {
+        const uint32_t b = r == 0 ? rows.b[0] : (r == 1 ? rows.b[1] : rows.b[2]);
+        const uint32_t n = r == 0 ? rows.n[0] : (r == 1 ? rows.n[1] : rows.n[2]);
+        const uint32_t e = b + n;
+        self_in          = self_in || i - b < n;
 #pragma unroll 1
         for (uint32_t j = b; j < e; j += 4u) {
             const uint32_t j1 = min(j + 1u, e - 1u), j2 = min(j + 2u, e - 1u), j3 = min(j + 3u, e - 1u);
             const auto q0 = ld(j), q1 = ld(j1), q2 = ld(j2), q3 = ld(j3);
-            ap(j, q0, true);
-            ap(j1, q1, j + 1u < e);
-            ap(j2, q2, j + 2u < e);
-            ap(j3, q3, j + 3u < e);
+            pass.add(acc, pass.term(me, q0, j != i), me.i, j);
+            pass.add(acc, pass.term(me, q1, j + 1u < e && j1 != i), me.i, j1);
+            pass.add(acc, pass.term(me, q2, j + 2u < e && j2 != i), me.i, j2);
+            pass.add(acc, pass.term(me, q3, j + 3u < e && j3 != i), me.i, j3);
         }
     }
+    return self_in;
 }
+
+// The same for the few lanes of a warp that cannot use their lists (mask fb of the lanes act that are here), one
+// after the other, every lane computing the terms of one candidate: two rounds of loads where scan_full's chain of
+// ten holds up the whole warp. The terms that are not zero are added in slot order, as in the other scans.
+template <class P, class L>
+__device__ __forceinline__ bool scan_together(uint32_t act, uint32_t fb, const DomDev& d,
+                                              const uint32_t* __restrict__ start, int32_t bx, int32_t by,
+                                              const Self& me, const L& ld, const P& pass, typename P::Acc& acc)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t rank = (uint32_t)__popc(act & ((1u << lane) - 1u)), width = (uint32_t)__popc(act);
+    bool self_in        = false;
+    while (fb != 0u) {
+        const int src = __ffs(fb) - 1;
+        fb &= fb - 1u;
+        Self s;
+        s.i  = __shfl_sync(act, me.i, src);
+        s.px = shfl2(act, me.px, src);
+        s.pd = shfl2(act, me.pd, src);
+        s.a  = P::USES_A ? __shfl_sync(act, me.a, src) : 0.f;
+        uint32_t b0 = 0u, b1 = 0u, b2 = 0u, n0 = 0u, n1 = 0u, n2 = 0u;
+        if ((int)lane == src) {
+            const Rows rows(d, start, bx, by);
+            b0 = rows.b[0], b1 = rows.b[1], b2 = rows.b[2];
+            n0 = rows.n[0], n1 = rows.n[1], n2 = rows.n[2];
+        }
+        b0 = __shfl_sync(act, b0, src);
+        b1 = __shfl_sync(act, b1, src);
+        b2 = __shfl_sync(act, b2, src);
+        n0 = __shfl_sync(act, n0, src);
+        n1 = __shfl_sync(act, n1, src);
+        n2 = __shfl_sync(act, n2, src);
+        const uint32_t i0    = (uint32_t)s.i;
+        const uint32_t total = n0 + n1 + n2;
+        typename P::Acc sum{};
+        for (uint32_t base = 0u; base < total; base += width) {
+            const uint32_t t = base + rank;
+            const bool valid = t < total;
+            const uint32_t j = !valid ? i0 : (t < n0 ? b0 + t : (t < n0 + n1 ? b1 + (t - n0) : b2 + (t - n0 - n1)));
+            const auto term  = pass.term(s, ld(j), valid && j != i0);
+            uint32_t hits    = __ballot_sync(act, term.hit != 0);
+            while (hits != 0u) {
+                const int l = __ffs(hits) - 1;
+                hits &= hits - 1u;
+                pass.add(sum, term.of(act, l), s.i, P::USES_J ? __shfl_sync(act, j, l) : 0u);
+            }
+        }
+        if ((int)lane == src) {
+            acc     = sum;
+            self_in = i0 - b0 < n0 || i0 - b1 < n1 || i0 - b2 < n2;
+        }
+    }
+    return self_in;
+}
+constexpr int TOGETHER_MAX = 4; // lanes for which that is cheaper: about 250 instructions each, 1,000 for scan_full
 
 // ----- candidate lists -----------------------------------------------------------------------------------
 // With sort cells of edge h a particle scans three rows of three cells, each row one contiguous range of
@@ -231,7 +324,11 @@ __device__ __forceinline__ void for_neighbours_at(const DomDev& d, const PbfK& k
 // One step of 1,048,576 particles from such a state: listed lambda 50 -> 25 us, delta p 41 -> 26 us, XSPH
 // 41 -> 28 us, the step with its state's copies 0.468 -> 0.325 ms; from an evolved state lambda 27 -> 23 us and
 // delta p 27 -> 23 us. 256 batched scenes (5.1M particles) 2.20 -> 1.42 ms.
-enum { LIST_OFF = 0, LIST_BUILD = 1, LIST_USE = 2 };
+// LIST_FEW is LIST_USE for launches whose warps are all resident at once at 64 registers a thread (stage launchers,
+// list_mode): there a pass lasts as long as its slowest warp, so its kernels take 64 registers instead of 40 and
+// spare the warp scan_full's chain of loads (scan_together). 16,384 atoms in 20 substeps 0.79 -> 0.70 ms; at 1M
+// particles the same form costs 0.339 against 0.318 ms.
+enum { LIST_OFF = 0, LIST_BUILD = 1, LIST_USE = 2, LIST_FEW = 3 };
 constexpr uint32_t LIST_BAD   = 0x80000000u; // in the header's count: this particle's list is not usable
 constexpr uint32_t LIST_MAX   = 48;          // candidates a list holds (a multiple of 8)
 constexpr uint32_t LIST_REACH = 32767;       // largest distance of a 16-bit slot
@@ -245,28 +342,45 @@ __device__ __forceinline__ float rsqrt_normal(float v)
     return r;
 }
 
-// Particle i's full scan around base cell (bx, by) (cell h, R = 1), recording its list. near(j): candidate j lies
-// within h + skin; ap(j, ld(j), valid) applies a recorded candidate (valid is false for the filler of the last
-// group of four), full(j, ld(j), valid) a candidate when the list cannot hold them. The particle's own slot is not
-// recorded: no pass takes a term from the self pair inside its loop (the density's self term is added after it).
-// Returns whether the recorded scan met that slot. A distance-only scan finds the candidates as one bit per slot
-// of each row, four slots a turn so that their loads are in flight together (the slots past a row's end that the
-// last turn reads are masked off; the record arrays are three records longer than the capacity); then the
-// candidates are taken out of the bits in scan order, stored, and applied: the same terms in the same order as the
-// full scan, whose other candidates add exact zeros.
-template <bool CG, class T, class L, class A, class F>
-__device__ __forceinline__ bool scan_record(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start,
-                                            float px, float py, float2 disp, int32_t i, T&& near, L&& ld, A&& ap,
-                                            F&& full)
+// Four candidates from place c of a list of cnt (the particle itself fills the last four): their records' loads are in
+// flight together.
+template <class P, class L>
+__device__ __forceinline__ void apply_four(int32_t i, uint32_t c, uint32_t cnt, uint32_t j0, uint32_t j1, uint32_t j2,
+                                           uint32_t j3, const Self& me, const L& ld, const P& pass,
+                                           typename P::Acc& acc)
 {
-    const int32_t bx = cell_coord(px, d.ox, k.inv_cell, d.ncx);
-    const int32_t by = cell_coord(py, d.oy, k.inv_cell, d.ncy);
+    const auto q0 = ld(j0), q1 = ld(j1), q2 = ld(j2), q3 = ld(j3);
+    pass.add(acc, pass.term(me, q0, true), i, j0);
+    pass.add(acc, pass.term(me, q1, c + 1u < cnt), i, j1);
+    pass.add(acc, pass.term(me, q2, c + 2u < cnt), i, j2);
+    pass.add(acc, pass.term(me, q3, c + 3u < cnt), i, j3);
+}
+
+// The full scan of a particle (cell h, R = 1) that records its list. The particle's own slot is not recorded: no
+// pass takes a term from the self pair inside its loop (the density's self term is added after it). Returns whether
+// the scan met that slot. A distance-only scan finds the candidates within h + skin as one bit per slot of each
+// row, four slots a turn so that their loads are in flight together (the slots past a row's end that the last turn
+// reads are dropped; the record arrays are three records longer than the capacity); then the candidates are taken
+// out of the bits in scan order, stored, and applied: the same terms in the same order as the full scan, whose other
+// candidates add exact zeros.
+template <bool CG, class P, class L>
+__device__ __forceinline__ bool scan_record(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start,
+                                            float2 p, const Self& me, const L& ld, const P& pass,
+                                            typename P::Acc& acc)
+{
+    const int32_t i  = me.i;
+    const int32_t bx = cell_coord(p.x, d.ox, k.inv_cell, d.ncx);
+    const int32_t by = cell_coord(p.y, d.oy, k.inv_cell, d.ncy);
     const int32_t x0 = max(bx - 1, 0);
     const int32_t x1 = min(bx + 1, d.ncx - 1);
     uint32_t w[3]    = {0u, 0u, 0u};
     uint32_t b[3]    = {0u, 0u, 0u};
     bool fits        = true; // the rows fit their bits, the slots their 16 bits
     bool self_in     = false;
+    auto near        = [&](const float4 q) {
+        const float2 r = offset(me.px, me.pd, q);
+        return fmaf(r.x, r.x, r.y * r.y) < k.skin2;
+    };
 #pragma unroll
     for (int32_t r = 0; r < 3; ++r) {
         const int32_t y = by - 1 + r;
@@ -303,11 +417,8 @@ __device__ __forceinline__ bool scan_record(const DomDev& d, const PbfK& k, cons
     const uint32_t key = ldn<CG>(&k.keys[i]);
     // a list built around another cell than the sort cell (or none) is not used later
     const bool usable  = fits && key == d.coff + (uint32_t)by * (uint32_t)d.ncx + (uint32_t)bx;
-    k.nhdr[i] = make_uint4(key, cnt | (usable ? 0u : LIST_BAD), __float_as_uint(disp.x), __float_as_uint(disp.y));
-    if (!fits) {
-        for_neighbours_at(d, k, start, bx, by, ld, full);
-        return false;
-    }
+    k.nhdr[i] = make_uint4(key, cnt | (usable ? 0u : LIST_BAD), __float_as_uint(me.pd.x), __float_as_uint(me.pd.y));
+    if (!fits) { return scan_full(d, start, bx, by, me, ld, pass, acc); }
     // the rows run as one sequence: the next row with candidates takes over when a row's bits run out
     uint32_t bits = w[0], base = b[0], w1 = w[1], b1 = b[1], w2 = w[2];
     auto turn = [&]() {
@@ -336,28 +447,18 @@ __device__ __forceinline__ bool scan_record(const DomDev& d, const PbfK& k, cons
         } else {
             k.nlist[(size_t)(c >> 2) * k.nstride + i] = make_uint4(j[0], j[1], j[2], j[3]);
         }
-        const auto q0 = ld(j[0]), q1 = ld(j[1]), q2 = ld(j[2]), q3 = ld(j[3]);
-        ap(j[0], q0, true);
-        ap(j[1], q1, c + 1u < cnt);
-        ap(j[2], q2, c + 2u < cnt);
-        ap(j[3], q3, c + 3u < cnt);
+        apply_four(i, c, cnt, j[0], j[1], j[2], j[3], me, ld, pass, acc);
     }
     return self_in;
 }
 
-// Applies the cnt candidates of particle i's list in scan order, four at a time: their records' loads are in
-// flight together. w0 is the first chunk, loaded beside the header.
-template <bool CG, class L, class A>
-__device__ __forceinline__ void scan_list(const PbfK& k, int32_t i, uint32_t cnt, const uint4 w0, L&& ld, A&& ap)
+// Applies the cnt candidates of the particle's list in scan order, four at a time. w is the first chunk, loaded
+// beside the header.
+template <bool CG, class P, class L>
+__device__ __forceinline__ void scan_list(const PbfK& k, uint32_t cnt, uint4 w, const Self& me, const L& ld,
+                                          const P& pass, typename P::Acc& acc)
 {
-    auto four = [&](uint32_t c, uint32_t j0, uint32_t j1, uint32_t j2, uint32_t j3) {
-        const auto q0 = ld(j0), q1 = ld(j1), q2 = ld(j2), q3 = ld(j3);
-        ap(j0, q0, true);
-        ap(j1, q1, c + 1u < cnt);
-        ap(j2, q2, c + 2u < cnt);
-        ap(j3, q3, c + 3u < cnt);
-    };
-    uint4 w          = w0;
+    const int32_t i  = me.i;
     const uint4* src = k.nlist + i;
     if (!k.wide) {
         auto lo = [&](uint32_t v) { return (uint32_t)(i + (int32_t)(int16_t)(v & 0xffffu)); };
@@ -367,8 +468,8 @@ __device__ __forceinline__ void scan_list(const PbfK& k, int32_t i, uint32_t cnt
                 src += k.nstride;
                 w = ldn<CG>(src);
             }
-            four(c, lo(w.x), hi(w.x), lo(w.y), hi(w.y));
-            if (c + 4u < cnt) { four(c + 4u, lo(w.z), hi(w.z), lo(w.w), hi(w.w)); }
+            apply_four(i, c, cnt, lo(w.x), hi(w.x), lo(w.y), hi(w.y), me, ld, pass, acc);
+            if (c + 4u < cnt) { apply_four(i, c + 4u, cnt, lo(w.z), hi(w.z), lo(w.w), hi(w.w), me, ld, pass, acc); }
         }
     } else {
         for (uint32_t c = 0u; c < cnt; c += 4u) {
@@ -376,35 +477,55 @@ __device__ __forceinline__ void scan_list(const PbfK& k, int32_t i, uint32_t cnt
                 src += k.nstride;
                 w = ldn<CG>(src);
             }
-            four(c, w.x, w.y, w.z, w.w);
+            apply_four(i, c, cnt, w.x, w.y, w.z, w.w, me, ld, pass, acc);
         }
     }
 }
 
-// The neighbour scan of particle i at (px, py) in list mode LIST (LIST_OFF or LIST_USE): ap(j, ld(j)) for every
-// candidate j in scan order, or apl(j, ld(j), valid) for those of the list, which skip the particle's own slot:
-// true is returned then (lists are used only while the particle is in its sort cell, so the full scan would have
-// met that slot). valid is false for the filler (the particle itself) of the last group of four.
-template <int LIST, bool CG, class L, class A, class AL>
-__device__ __forceinline__ bool scan_ld(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start, float px,
-                                        float py, int32_t i, L&& ld, A&& ap, AL&& apl)
+// The neighbour scan of a particle at p in list mode LIST (LIST_OFF, LIST_USE or LIST_FEW). Returns whether its own slot is
+// among the scanned cells' (lists are used only while the particle is in its sort cell, so then it is).
+template <int LIST, bool CG, class P, class L>
+__device__ __forceinline__ bool scan_ld(const DomDev& d, const PbfK& k, const uint32_t* __restrict__ start, float2 p,
+                                        const Self& me, const L& ld, const P& pass, typename P::Acc& acc)
 {
     if constexpr (LIST == LIST_OFF) {
-        for_neighbours(d, k, start, px, py, [&](uint32_t j) { ap(j, ld(j), true); });
+        bool self_in = false;
+        for_neighbours(d, k, start, p.x, p.y, [&](uint32_t j) {
+            self_in = self_in || j == (uint32_t)me.i;
+            pass.add(acc, pass.term(me, ld(j), j != (uint32_t)me.i), me.i, j);
+        });
+        return self_in;
     } else {
-        const uint4 hd = ldn<CG>(&k.nhdr[i]);
-        const uint4 w0 = ldn<CG>(&k.nlist[i]);
+        const uint4 hd     = ldn<CG>(&k.nhdr[me.i]);
+        const uint4 w0     = ldn<CG>(&k.nlist[me.i]);
         const bool far     = ldn<CG>(&k.mflag[hd.x]) != 0;
-        const int32_t bx   = cell_coord(px, d.ox, k.inv_cell, d.ncx);
-        const int32_t by   = cell_coord(py, d.oy, k.inv_cell, d.ncy);
+        const int32_t bx   = cell_coord(p.x, d.ox, k.inv_cell, d.ncx);
+        const int32_t by   = cell_coord(p.y, d.oy, k.inv_cell, d.ncy);
         const uint32_t key = d.coff + (uint32_t)by * (uint32_t)d.ncx + (uint32_t)bx;
-        if (!(hd.y & LIST_BAD) && key == hd.x && !far) {
-            scan_list<CG>(k, i, hd.y, w0, ld, apl);
-            return true;
+        const bool listed  = !(hd.y & LIST_BAD) && key == hd.x && !far;
+        bool self_in       = true;
+        if constexpr (LIST == LIST_USE) {
+            if (listed) {
+                scan_list<CG>(k, hd.y, w0, me, ld, pass, acc);
+            } else {
+                self_in = scan_full(d, start, bx, by, me, ld, pass, acc);
+            }
+        } else {
+            const uint32_t act = __activemask();
+            const uint32_t fb  = __ballot_sync(act, !listed);
+            if (listed) { scan_list<CG>(k, hd.y, w0, me, ld, pass, acc); }
+            if (fb != 0u) {
+                bool in;
+                if (__popc(fb) <= TOGETHER_MAX) {
+                    in = scan_together(act, fb, d, start, bx, by, me, ld, pass, acc);
+                } else {
+                    in = listed || scan_full(d, start, bx, by, me, ld, pass, acc);
+                }
+                self_in = listed || in;
+            }
         }
-        for_neighbours_at(d, k, start, bx, by, ld, ap);
+        return self_in;
     }
-    return false;
 }
 
 // A delta p pass left a particle (sort cell key) skin / 2 or more from where it was when the lists were made: the
@@ -565,80 +686,94 @@ __global__ void __launch_bounds__(T_PART)
 //           unclamped, and the pass moves the particles by the change of L; a sum that overshot is relaxed
 //           again and L never turns into a pull (accumulated-multiplier clamping).
 enum { ACC_NONE = 0, ACC_SUM = 1, ACC_PROJ = 2 };
+// The reference accumulates per pair sv = -cs m (h-r)^2 r/|r|, |sv|^2 / m and m W6 (PBF.cu:264-286). Constants are
+// hoisted: sg = sum (h-r)^2 r/|r|, s4 = sum (h-r)^4 (= |sv|^2 / (cs m)^2 since r/|r| is a unit vector), s6 = sum
+// (h^2 - r^2)^3. A distinct atom at the same position contributes the reference's pseudo-random pair direction. The
+// self pair (r = 0) is added after the scan (add_self): it contributes h^6 to the density and, in the reference, a
+// gradient of length cs m h^2 along pairDirection(i, i). Self's a holds the scene's first slot.
+template <bool SELFG>
+struct LambdaPass {
+    static constexpr bool USES_A = SELFG, USES_J = SELFG;
+    const PbfK& k;
+    const uint32_t* __restrict__ pair_id;
+    struct Acc {
+        float2 sg;
+        float s4, s6;
+    };
+    struct Term {
+        float2 r;
+        float qq, d2, w;
+        uint32_t hit; // 2: at the same position
+        float a;      // Self's a
+        __device__ __forceinline__ Term of(uint32_t m, int l) const
+        {
+            return Term{shfl2(m, r, l), __shfl_sync(m, qq, l), __shfl_sync(m, d2, l), __shfl_sync(m, w, l),
+                        SELFG ? __shfl_sync(m, hit, l) : 1u, a};
+        }
+    };
+    __device__ __forceinline__ Term term(const Self& me, const float4 q, bool valid) const
+    {
+        Term t;
+        t.r             = offset(me.px, me.pd, q);
+        const float r2  = fmaf(t.r.x, t.r.x, t.r.y * t.r.y);
+        const bool in   = (r2 <= k.h2) && valid;
+        const bool dir  = in && (r2 > 1e-12f);
+        t.qq            = in ? k.h2 - r2 : 0.f;
+        const float inv = rsqrt_normal(dir ? r2 : 1.f);
+        const float dif = dir ? fmaf(-r2, inv, k.h) : 0.f;
+        t.d2            = dif * dif;
+        t.w             = t.d2 * inv;
+        t.hit           = in ? (SELFG && !dir && t.r.x == 0.f && t.r.y == 0.f ? 2u : 1u) : 0u;
+        t.a             = me.a;
+        return t;
+    }
+    __device__ __forceinline__ void add_twin(Acc& s, uint32_t ia, uint32_t ja) const
+    {
+        float nx, ny;
+        pair_direction(ia, ja, nx, ny);
+        s.sg.x = fmaf(k.h2, nx, s.sg.x);
+        s.sg.y = fmaf(k.h2, ny, s.sg.y);
+        s.s4   = fmaf(k.h2, k.h2, s.s4);
+    }
+    __device__ __forceinline__ uint32_t name(uint32_t i, float a) const
+    {
+        return pair_id ? __ldg(&pair_id[i]) : i - __float_as_uint(a);
+    }
+    __device__ __forceinline__ void add(Acc& s, const Term& t, int32_t i, uint32_t j) const
+    {
+        s.s6 = fmaf(t.qq * t.qq, t.qq, s.s6);
+        s.sg = fma2(make_float2(t.w, t.w), t.r, s.sg);
+        s.s4 = fmaf(t.d2, t.d2, s.s4);
+        if (SELFG && t.hit == 2u) { add_twin(s, name((uint32_t)i, t.a), name(j, t.a)); }
+    }
+    __device__ __forceinline__ void add_self(Acc& s, const Self& me) const
+    {
+        s.s6 = fmaf(k.h2 * k.h2, k.h2, s.s6);
+        if (SELFG) { add_twin(s, name((uint32_t)me.i, me.a), name((uint32_t)me.i, me.a)); }
+    }
+};
+
 template <bool MULTI, bool SELFG, int ACC, bool CG = false, int LIST = LIST_OFF>
 __device__ __forceinline__ void lambda_one(const PbfK& k, const DomDev* __restrict__ doms,
                                            const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
                                            const float4* __restrict__ xd, float* __restrict__ lam,
                                            const uint32_t* __restrict__ pair_id, float* __restrict__ acc, int32_t i)
 {
-    const DomDev d       = load_dom<MULTI>(k, doms, dom, i);
-    const uint32_t pbase = MULTI ? __ldg(&start[d.coff]) : 0u;
-    const float4 p4      = ldn<CG>(&xd[i]);
-    const float2 px = xy_of(p4), pd = d_of(p4);
-    const float2 p       = add2(px, pd); // x*, for the cell lookup
-    // The reference accumulates per pair sv = -cs m (h-r)^2 r/|r|, |sv|^2 / m and m W6 (PBF.cu:264-286).
-    // Constants are hoisted: sx, sy = sum (h-r)^2 r/|r|, s4 = sum (h-r)^4 (= |sv|^2 / (cs m)^2 since r/|r| is a
-    // unit vector), s6 = sum (h^2 - r^2)^3. The self pair (r = 0) is added after the loop: it contributes
-    // h^6 to the density and, in the reference, a gradient of length cs m h^2 along pairDirection(i, i).
-    float2 sg = make_float2(0.f, 0.f); // (sx, sy)
-    float s4 = 0.f, s6 = 0.f;
-    bool self_seen = false; // the atom's own slot can fall outside the scanned cells after large moves
-    // Branch-free body: every lane of a warp runs the same instructions for every candidate and the terms of
-    // pairs beyond h (and of the self pair) are masked to zero; a data-dependent accept branch here would
-    // make each warp execute both paths on almost every iteration.
-    // me: the candidate may be the particle itself (full scans); lists hold it only as filler (valid false)
-    auto body = [&](uint32_t j, const float4 q, auto me, bool valid) {
-        const float2 r  = offset(px, pd, q);
-        const float r2  = fmaf(r.x, r.x, r.y * r.y);
-        const bool self = decltype(me)::value && j == (uint32_t)i;
-        self_seen       = self_seen || self;
-        const bool in   = (r2 <= k.h2) && !self && valid;
-        const bool dir  = in && (r2 > 1e-12f);
-        const float qq  = in ? k.h2 - r2 : 0.f;
-        s6              = fmaf(qq * qq, qq, s6);
-        const float inv = rsqrt_normal(dir ? r2 : 1.f);
-        const float dif = dir ? fmaf(-r2, inv, k.h) : 0.f;
-        const float d2  = dif * dif;
-        const float w   = d2 * inv;
-        sg              = fma2(make_float2(w, w), r, sg);
-        s4              = fmaf(d2, d2, s4);
-        if (SELFG && in && !dir && r.x == 0.f && r.y == 0.f) {
-            // a distinct atom at the same position: the reference's pseudo-random pair direction
-            float nx, ny;
-            if (pair_id) {
-                pair_direction(__ldg(&pair_id[i]), __ldg(&pair_id[j]), nx, ny);
-            } else {
-                pair_direction((uint32_t)i - pbase, j - pbase, nx, ny);
-            }
-            sg.x = fmaf(k.h2, nx, sg.x);
-            sg.y = fmaf(k.h2, ny, sg.y);
-            s4 = fmaf(k.h2, k.h2, s4);
-        }
-    };
-    const Records<CG> ld{xd};
-    auto full = [&](uint32_t j, const float4 q, bool valid) { body(j, q, std::true_type{}, valid); };
-    auto list = [&](uint32_t j, const float4 q, bool valid) { body(j, q, std::false_type{}, valid); };
-    bool listed;
+    const DomDev d  = load_dom<MULTI>(k, doms, dom, i);
+    const float4 p4 = ldn<CG>(&xd[i]);
+    const Self me{i, xy_of(p4), d_of(p4), __uint_as_float(SELFG && MULTI ? __ldg(&start[d.coff]) : 0u)};
+    const float2 p = add2(me.px, me.pd); // x*, for the cell lookup
+    const LambdaPass<SELFG> pass{k, pair_id};
+    typename LambdaPass<SELFG>::Acc sum{};
+    bool self_in; // the atom's own slot can fall outside the scanned cells after large moves
     if constexpr (LIST == LIST_BUILD) {
-        listed = scan_record<CG>(d, k, start, p.x, p.y, pd, i, [&](const float4 q) {
-            const float2 r = offset(px, pd, q);
-            return fmaf(r.x, r.x, r.y * r.y) < k.skin2;
-        }, ld, list, full);
+        self_in = scan_record<CG>(d, k, start, p, me, Records<CG>{xd}, pass, sum);
     } else {
-        listed = scan_ld<LIST, CG>(d, k, start, p.x, p.y, i, ld, full, list);
+        self_in = scan_ld<LIST, CG>(d, k, start, p, me, Records<CG>{xd}, pass, sum);
     }
-    self_seen = self_seen || listed;
-    if (self_seen) {
-        s6 = fmaf(k.h2 * k.h2, k.h2, s6);
-        if (SELFG) {
-            float nx, ny;
-            const uint32_t a = pair_id ? __ldg(&pair_id[i]) : (uint32_t)i - pbase;
-            pair_direction(a, a, nx, ny);
-            sg.x = fmaf(k.h2, nx, sg.x);
-            sg.y = fmaf(k.h2, ny, sg.y);
-            s4 = fmaf(k.h2, k.h2, s4);
-        }
-    }
+    if (self_in) { pass.add_self(sum, me); }
+    const float2 sg = sum.sg;
+    const float s4 = sum.s4, s6 = sum.s6;
     const float csm  = k.cs * k.mass;
     const float rho  = k.mass * k.c6 * s6;
     const float gx = csm * sg.x, gy = csm * sg.y;
@@ -660,10 +795,10 @@ __device__ __forceinline__ void lambda_one(const PbfK& k, const DomDev* __restri
 }
 
 // 40 registers (48 warps per SM) for the recording and the listed passes, although a few values spill there: 1M
-// particles 0.325 ms a pass against 0.343 at 64 registers; with pair directions the spills cost more than the
+// particles 0.325 ms a step against 0.343 at 64 registers; with pair directions the spills cost more than the
 // warps give (16,384 atoms in 20 substeps 0.88 against 0.79 ms)
 template <bool MULTI, bool SELFG, int ACC, int LIST>
-__global__ void __launch_bounds__(T_MAX, LIST == LIST_OFF ? 1 : (SELFG ? 2 : 3))
+__global__ void __launch_bounds__(T_MAX, LIST == LIST_OFF ? 1 : (SELFG || LIST == LIST_FEW ? 2 : 3))
     k_lambda(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
              const uint32_t* __restrict__ start, const float4* __restrict__ xd, float* __restrict__ lam,
              const uint32_t* __restrict__ pair_id, float* __restrict__ acc)
@@ -676,6 +811,46 @@ __global__ void __launch_bounds__(T_MAX, LIST == LIST_OFF ? 1 : (SELFG ? 2 : 3))
 
 // ----- delta p with artificial pressure and over-relaxation, then walls (PBF.cu:398-447, 471-499) -------
 // ACCINIT: this pass applies the warm start; its multiplier starts the step's running sum.
+// dp = omega/(m rho0) sum (m lambda_i + m lambda_j - s_corr) * (-cs (h-r)^2 r/|r|) (PBF.cu:415-437); pairs closer than
+// 1e-6 (the self pair included) have a zero direction there and are skipped here. Self's a holds m lambda_i.
+template <bool SCORR>
+struct DeltaPass {
+    static constexpr bool USES_A = true, USES_J = false;
+    const PbfK& k;
+    using Acc = float2; // sum of w r
+    struct Term {
+        float2 r;
+        float w;
+        bool hit;
+        __device__ __forceinline__ Term of(uint32_t m, int l) const
+        {
+            return Term{shfl2(m, r, l), __shfl_sync(m, w, l), true};
+        }
+    };
+    __device__ __forceinline__ Term term(const Self& me, const Nbr ql, bool valid) const
+    {
+        Term t;
+        t.r             = offset(me.px, me.pd, ql.q);
+        const float r2  = fmaf(t.r.x, t.r.x, t.r.y * t.r.y);
+        t.hit           = (r2 <= k.h2) && (r2 > 1e-12f) && valid;
+        const float inv = rsqrt_normal(t.hit ? r2 : 1.f);
+        float l         = fmaf(ql.a, k.mass, me.a);
+        if (SCORR) {
+            const float qq    = k.h2 - r2;
+            const float ratio = (k.c6 * k.inv_w_dq) * (qq * qq * qq);
+            const float r2q   = ratio * ratio;
+            l                 = fmaf(-k.scorr_k, r2q * r2q, l);
+        }
+        const float diff = fmaf(-r2, inv, k.h);
+        t.w              = t.hit ? diff * diff * inv * l : 0.f;
+        return t;
+    }
+    __device__ __forceinline__ void add(Acc& s, const Term& t, int32_t, uint32_t) const
+    {
+        s = fma2(make_float2(t.w, t.w), t.r, s);
+    }
+};
+
 template <bool MULTI, bool SCORR, bool ACCINIT, bool CG = false, int LIST = LIST_OFF>
 __device__ __forceinline__ void delta_p_one(const PbfK& k, const DomDev* __restrict__ doms,
                                             const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
@@ -685,35 +860,11 @@ __device__ __forceinline__ void delta_p_one(const PbfK& k, const DomDev* __restr
     const DomDev d  = load_dom<MULTI>(k, doms, dom, i);
     const float4 p4 = ldn<CG>(&xd[i]);
     const float2 px = xy_of(p4), pd = d_of(p4);
-    const float2 p  = add2(px, pd); // x*, for the cell lookup
     const float li  = ldn<CG>(&lam[i]);
     if (ACCINIT) { acc[i] = li; }
-    const float mli = li * k.mass;
-    // dp = omega/(m rho0) sum (m lambda_i + m lambda_j - s_corr) * (-cs (h-r)^2 r/|r|) (PBF.cu:415-437); pairs
-    // closer than 1e-6 (the self pair included) have a zero direction there and are skipped here.
-    const float c6w = k.c6 * k.inv_w_dq;
-    float2 sg = make_float2(0.f, 0.f); // (sx, sy)
-    // (a list's filler is the particle itself, which the direction test leaves out)
-    auto body = [&](const Nbr ql, bool valid) {
-        const float lj  = ql.a;
-        const float2 r  = offset(px, pd, ql.q);
-        const float r2  = fmaf(r.x, r.x, r.y * r.y);
-        const bool ok   = (r2 <= k.h2) && (r2 > 1e-12f) && valid; // masked, branch-free (see k_lambda)
-        const float inv = rsqrt_normal(ok ? r2 : 1.f);
-        float l         = fmaf(lj, k.mass, mli);
-        if (SCORR) {
-            const float qq    = k.h2 - r2;
-            const float ratio = c6w * (qq * qq * qq);
-            const float r2q   = ratio * ratio;
-            l                 = fmaf(-k.scorr_k, r2q * r2q, l);
-        }
-        const float diff = fmaf(-r2, inv, k.h);
-        const float w    = ok ? diff * diff * inv * l : 0.f;
-        sg               = fma2(make_float2(w, w), r, sg);
-    };
-    scan_ld<LIST, CG>(d, k, start, p.x, p.y, i, RecordsAnd<CG>{xd, lam},
-                      [&](uint32_t, const Nbr q, bool valid) { body(q, valid); },
-                      [&](uint32_t, const Nbr q, bool) { body(q, true); });
+    float2 sg = make_float2(0.f, 0.f);
+    scan_ld<LIST, CG>(d, k, start, add2(px, pd), Self{i, px, pd, li * k.mass}, RecordsAnd<CG>{xd, lam},
+                      DeltaPass<SCORR>{k}, sg);
     const float s = -k.cs * k.dp_scale;
     // the correction moves the displacement; the position x + d is clamped to the walls (clamp<float>(v, lb,
     // ub), PBF.cu:496-497) by setting d = wall - x, exact next to the wall, so that x + d lands on it
@@ -722,7 +873,7 @@ __device__ __forceinline__ void delta_p_one(const PbfK& k, const DomDev* __restr
     dy = (oy > d.hiy) ? __fsub_rn(d.hiy, px.y) : ((oy < d.loy) ? __fsub_rn(d.loy, px.y) : dy);
     dx = (ox > d.hix) ? __fsub_rn(d.hix, px.x) : ((ox < d.lox) ? __fsub_rn(d.lox, px.x) : dx);
     xd_out[i] = make_float4(px.x, px.y, dx, dy);
-    if constexpr (LIST == LIST_USE) {
+    if constexpr (LIST == LIST_USE || LIST == LIST_FEW) {
         // how far the particle is from where it was when the lists were made
         const uint4 hd = ldn<CG>(&k.nhdr[i]);
         const float mx = dx - __uint_as_float(hd.z), my = dy - __uint_as_float(hd.w);
@@ -731,7 +882,7 @@ __device__ __forceinline__ void delta_p_one(const PbfK& k, const DomDev* __restr
 }
 
 template <bool MULTI, bool SCORR, bool ACCINIT, int LIST>
-__global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : 1)
+__global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : (LIST == LIST_FEW ? 2 : 1))
     k_delta_p(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
               const uint32_t* __restrict__ start, const float4* __restrict__ xd, const float* __restrict__ lam,
               float4* __restrict__ xd_out, float* __restrict__ acc)
@@ -746,6 +897,31 @@ __global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : 1)
 // The lambda sums of k_lambda plus the neighbour count and the poly6-weighted sum of the neighbours'
 // lambda_prev; returns the cold first-iteration lambda and fills the network's 12 features (the order is
 // the one documented with gpe_pbf_set_warm_start).
+template <bool SELFG>
+struct FeaturePass {
+    using Base = LambdaPass<SELFG>; // as in k_lambda, so the cold lambda is bit-identical
+    Base base;
+    struct Acc {
+        typename Base::Acc lam;
+        float swl;
+        int32_t nn;
+    };
+    struct Term {
+        typename Base::Term lam;
+        float lp;
+    };
+    __device__ __forceinline__ Term term(const Self& me, const Nbr ql, bool valid) const
+    {
+        return Term{base.term(me, ql.q, valid), ql.a};
+    }
+    __device__ __forceinline__ void add(Acc& s, const Term& t, int32_t i, uint32_t j) const
+    {
+        s.swl = fmaf(t.lam.qq * t.lam.qq * t.lam.qq, t.lp, s.swl);
+        s.nn += t.lam.hit ? 1 : 0;
+        base.add(s.lam, t.lam, i, j);
+    }
+};
+
 template <bool MULTI, bool SELFG, int LIST = LIST_OFF>
 __device__ __forceinline__ float warm_features(const PbfK& k, const DomDev& d, const uint32_t* __restrict__ start,
                                                const float4* __restrict__ xd, const float* __restrict__ prev,
@@ -755,66 +931,24 @@ __device__ __forceinline__ float warm_features(const PbfK& k, const DomDev& d, c
     const float4 p4 = xd[i];
     const float2 px = xy_of(p4), pd = d_of(p4);
     const float2 p  = add2(px, pd); // x*
-    float2 sg = make_float2(0.f, 0.f); // (sx, sy)
-    float s4 = 0.f, s6 = 0.f, swl = 0.f;
-    int32_t nn     = 0;
-    bool self_seen = false;
-    // me: the candidate may be the particle itself (full scans); lists hold it only as filler (valid false)
-    auto body = [&](uint32_t j, const Nbr ql, auto me, bool valid) {
-        const float4 q  = ql.q;
-        const float lp  = ql.a;
-        const float2 r  = offset(px, pd, q);
-        const float r2  = fmaf(r.x, r.x, r.y * r.y);
-        const bool self = decltype(me)::value && j == (uint32_t)i;
-        self_seen       = self_seen || self;
-        const bool in   = (r2 <= k.h2) && !self && valid;
-        const bool dir  = in && (r2 > 1e-12f);
-        const float qq  = in ? k.h2 - r2 : 0.f;
-        s6              = fmaf(qq * qq, qq, s6); // as in k_lambda, so the cold lambda is bit-identical
-        swl             = fmaf(qq * qq * qq, lp, swl);
-        nn += in ? 1 : 0;
-        const float inv = rsqrt_normal(dir ? r2 : 1.f);
-        const float dif = dir ? fmaf(-r2, inv, k.h) : 0.f;
-        const float d2  = dif * dif;
-        const float w   = d2 * inv;
-        sg              = fma2(make_float2(w, w), r, sg);
-        s4              = fmaf(d2, d2, s4);
-        if (SELFG && in && !dir && r.x == 0.f && r.y == 0.f) {
-            float nx, ny;
-            if (pair_id) {
-                pair_direction(__ldg(&pair_id[i]), __ldg(&pair_id[j]), nx, ny);
-            } else {
-                pair_direction((uint32_t)i - pbase, j - pbase, nx, ny);
-            }
-            sg.x = fmaf(k.h2, nx, sg.x);
-            sg.y = fmaf(k.h2, ny, sg.y);
-            s4 = fmaf(k.h2, k.h2, s4);
-        }
-    };
+    const Self me{i, px, pd, __uint_as_float(pbase)};
+    const FeaturePass<SELFG> pass{LambdaPass<SELFG>{k, pair_id}};
+    typename FeaturePass<SELFG>::Acc sum{};
     const RecordsAnd<false> ld{xd, prev};
-    auto full = [&](uint32_t j, const Nbr q, bool valid) { body(j, q, std::true_type{}, valid); };
+    bool self_in;
     if constexpr (LIST == LIST_BUILD) {
-        const bool listed = scan_record<false>(d, k, start, p.x, p.y, pd, i, [&](const float4 q) {
-            const float2 r = offset(px, pd, q);
-            return fmaf(r.x, r.x, r.y * r.y) < k.skin2;
-        }, ld, [&](uint32_t j, const Nbr q, bool valid) { body(j, q, std::false_type{}, valid); }, full);
-        self_seen = self_seen || listed;
+        self_in = scan_record<false>(d, k, start, p, me, ld, pass, sum);
     } else {
-        for_neighbours(d, k, start, p.x, p.y, [&](uint32_t j) { full(j, ld(j), true); });
+        self_in = scan_ld<LIST_OFF, false>(d, k, start, p, me, ld, pass, sum);
     }
     const float lpi = prev[i];
-    if (self_seen) {
-        s6  = fmaf(k.h2 * k.h2, k.h2, s6);
-        swl = fmaf(k.h2 * k.h2 * k.h2, lpi, swl);
-        if (SELFG) {
-            float nx, ny;
-            const uint32_t a = pair_id ? __ldg(&pair_id[i]) : (uint32_t)i - pbase;
-            pair_direction(a, a, nx, ny);
-            sg.x = fmaf(k.h2, nx, sg.x);
-            sg.y = fmaf(k.h2, ny, sg.y);
-            s4 = fmaf(k.h2, k.h2, s4);
-        }
+    if (self_in) {
+        pass.base.add_self(sum.lam, me);
+        sum.swl = fmaf(k.h2 * k.h2 * k.h2, lpi, sum.swl);
     }
+    const float2 sg = sum.lam.sg;
+    const float s4 = sum.lam.s4, s6 = sum.lam.s6, swl = sum.swl;
+    const int32_t nn = sum.nn;
     const float csm  = k.cs * k.mass;
     const float rho  = k.mass * k.c6 * s6;
     const float gx = csm * sg.x, gy = csm * sg.y;
@@ -975,6 +1109,54 @@ __device__ __forceinline__ void velocity_clamp(const PbfK& k, float& vx, float& 
 }
 
 // ----- velocity + XSPH (+ vorticity omega) (PBF.cu:538, 585-627) ---------------------------------------
+// dv = c sum (v_j - v_i) W6 (PBF.cu:602-615) with the poly6 coefficient hoisted; the self pair adds 0. omega = sum
+// (v_j - v_i) x grad_j W with grad_j W = +cs (h-r)^2 r/|r| (cs hoisted as well).
+template <bool VORT>
+struct XsphPass {
+    static constexpr bool USES_A = false, USES_J = false;
+    const PbfK& k;
+    struct Acc {
+        float2 dv;
+        float w;
+    };
+    struct Term {
+        float2 dv;
+        float p6, gm, cross;
+        bool hit;
+        __device__ __forceinline__ Term of(uint32_t m, int l) const
+        {
+            return Term{shfl2(m, dv, l), __shfl_sync(m, p6, l), VORT ? __shfl_sync(m, gm, l) : 0.f,
+                        VORT ? __shfl_sync(m, cross, l) : 0.f, true};
+        }
+    };
+    __device__ __forceinline__ Term term(const Self& me, const float4 q, bool valid) const
+    {
+        Term t;
+        const float2 r = offset(me.px, me.pd, q);
+        const float r2 = fmaf(r.x, r.x, r.y * r.y);
+        t.hit          = (r2 <= k.h2) && valid;
+        // v = (x* - x) / dt = d / dt (PBF.cu:538)
+        t.dv           = fma2(d_of(q), make_float2(k.inv_dt, k.inv_dt),
+                              make_float2(-(me.pd.x * k.inv_dt), -(me.pd.y * k.inv_dt)));
+        const float qq = t.hit ? k.h2 - r2 : 0.f;
+        t.p6           = qq * qq * qq;
+        t.gm = t.cross = 0.f;
+        if (VORT) {
+            const bool dir   = t.hit && (r2 > 1e-12f);
+            const float inv  = rsqrt_normal(dir ? r2 : 1.f);
+            const float diff = fmaf(-r2, inv, k.h);
+            t.gm             = dir ? diff * diff * inv : 0.f;
+            t.cross          = fmaf(t.dv.x, r.y, -(t.dv.y * r.x));
+        }
+        return t;
+    }
+    __device__ __forceinline__ void add(Acc& s, const Term& t, int32_t, uint32_t) const
+    {
+        s.dv = fma2(t.dv, make_float2(t.p6, t.p6), s.dv);
+        if (VORT) { s.w = fmaf(t.gm, t.cross, s.w); }
+    }
+};
+
 template <bool MULTI, bool VORT, bool CG = false, int LIST = LIST_OFF>
 __device__ __forceinline__ void xsph_one(const PbfK& k, const DomDev* __restrict__ doms,
                                          const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
@@ -988,36 +1170,10 @@ __device__ __forceinline__ void xsph_one(const PbfK& k, const DomDev* __restrict
     const float2 p  = add2(px, pd); // x*: the step's end position
     // v = (x* - x) / dt = d / dt (PBF.cu:538): no cancellation of two large coordinates
     const float vax = pd.x * k.inv_dt, vay = pd.y * k.inv_dt;
-    // dv = c sum (v_j - v_i) W6 (PBF.cu:602-615) with the poly6 coefficient hoisted; the self pair adds 0.
-    // omega = sum (v_j - v_i) x grad_j W with grad_j W = +cs (h-r)^2 r/|r| (cs hoisted as well).
-    float2 dvs = make_float2(0.f, 0.f); // (dvx, dvy)
-    float w    = 0.f;
-    // me: the candidate may be the particle itself (full scans); lists hold it only as filler (valid false)
-    auto xbody = [&](uint32_t j, const float4 q, auto me, bool valid) {
-        const float2 r  = offset(px, pd, q);
-        const float rx = r.x, ry = r.y;
-        // explicit fused forms: the result must not depend on how the compiler contracts this body in the
-        // kernel it is inlined into (separate launches and the persistent solve are compared bit for bit)
-        const float r2  = fmaf(rx, rx, ry * ry);
-        // masked, branch-free (see k_lambda); the self pair adds nothing in exact arithmetic (v_i - v_i) and is
-        // left out
-        const bool in   = (r2 <= k.h2) && valid && !(decltype(me)::value && j == (uint32_t)i);
-        const float2 dv = fma2(d_of(q), make_float2(k.inv_dt, k.inv_dt), make_float2(-vax, -vay));
-        const float dx = dv.x, dy = dv.y;
-        const float qq  = in ? k.h2 - r2 : 0.f;
-        const float p6  = qq * qq * qq;
-        dvs             = fma2(dv, make_float2(p6, p6), dvs);
-        if (VORT) {
-            const bool dir   = in && (r2 > 1e-12f);
-            const float inv  = rsqrt_normal(dir ? r2 : 1.f);
-            const float diff = fmaf(-r2, inv, k.h);
-            const float gm   = dir ? diff * diff * inv : 0.f;
-            w                = fmaf(gm, fmaf(dx, ry, -(dy * rx)), w);
-        }
-    };
-    scan_ld<LIST, CG>(d, k, start, p.x, p.y, i, Records<CG>{xd},
-                      [&](uint32_t j, const float4 q, bool valid) { xbody(j, q, std::true_type{}, valid); },
-                      [&](uint32_t j, const float4 q, bool valid) { xbody(j, q, std::false_type{}, valid); });
+    typename XsphPass<VORT>::Acc sum{};
+    scan_ld<LIST, CG>(d, k, start, p, Self{i, px, pd, 0.f}, Records<CG>{xd}, XsphPass<VORT>{k}, sum);
+    const float2 dvs = sum.dv;
+    float w          = sum.w;
     w *= k.cs;
     const float cx = k.xsph_c * k.c6;
     float vx       = fmaf(dvs.x, cx, vax);
@@ -1034,7 +1190,7 @@ __device__ __forceinline__ void xsph_one(const PbfK& k, const DomDev* __restrict
 }
 
 template <bool MULTI, bool VORT, int LIST>
-__global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : 1)
+__global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : (LIST == LIST_FEW ? 2 : 1))
     k_xsph(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
            const uint32_t* __restrict__ start, const float4* __restrict__ xd, float2* __restrict__ x_out,
            float2* __restrict__ v_out, float* __restrict__ omega, uint32_t* __restrict__ status)
@@ -1055,6 +1211,37 @@ __global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : 1)
 }
 
 // ----- vorticity confinement (Macklin & Mueller 2013 eq. 16) --------------------------------------------
+// eta = grad |omega| up to a factor; Self's a holds |omega_i|
+struct VorticityPass {
+    static constexpr bool USES_A = true, USES_J = false;
+    const PbfK& k;
+    using Acc = float2;
+    struct Term {
+        float2 r;
+        float w;
+        bool hit;
+        __device__ __forceinline__ Term of(uint32_t m, int l) const
+        {
+            return Term{shfl2(m, r, l), __shfl_sync(m, w, l), true};
+        }
+    };
+    __device__ __forceinline__ Term term(const Self& me, const Nbr qw, bool valid) const
+    {
+        Term t;
+        t.r              = offset(me.px, me.pd, qw.q);
+        const float r2   = fmaf(t.r.x, t.r.x, t.r.y * t.r.y);
+        t.hit            = (r2 <= k.h2) && (r2 > 1e-12f) && valid;
+        const float inv  = rsqrt_normal(t.hit ? r2 : 1.f);
+        const float diff = fmaf(-r2, inv, k.h);
+        t.w              = t.hit ? (fabsf(qw.a) - me.a) * (diff * diff * inv) : 0.f; // grad_i W = -cs (...)
+        return t;
+    }
+    __device__ __forceinline__ void add(Acc& s, const Term& t, int32_t, uint32_t) const
+    {
+        s = fma2(make_float2(t.w, t.w), t.r, s);
+    }
+};
+
 template <bool MULTI, bool CG = false, int LIST = LIST_OFF>
 __device__ __forceinline__ void vorticity_one(const PbfK& k, const DomDev* __restrict__ doms,
                                               const int32_t* __restrict__ dom, const uint32_t* __restrict__ start,
@@ -1066,22 +1253,8 @@ __device__ __forceinline__ void vorticity_one(const PbfK& k, const DomDev* __res
     const float2 px = xy_of(p4), pd = d_of(p4);
     const float2 p  = add2(px, pd); // x*, for the cell lookup
     const float wi = omega[i];
-    const float aw = fabsf(wi);
-    float2 eg = make_float2(0.f, 0.f); // (ex, ey)
-    auto body = [&](const Nbr qw, bool valid) { // (the direction test leaves out the particle itself)
-        const float wj   = qw.a;
-        const float2 r   = offset(px, pd, qw.q);
-        const float rx = r.x, ry = r.y;
-        const float r2   = fmaf(rx, rx, ry * ry); // explicit fused forms, as in xsph_one
-        const bool ok    = (r2 <= k.h2) && (r2 > 1e-12f) && valid; // masked, branch-free (see k_lambda)
-        const float inv  = rsqrt_normal(ok ? r2 : 1.f);
-        const float diff = fmaf(-r2, inv, k.h);
-        const float dwg  = ok ? (fabsf(wj) - aw) * (diff * diff * inv) : 0.f; // grad_i W = -cs (...)
-        eg               = fma2(make_float2(dwg, dwg), r, eg);
-    };
-    scan_ld<LIST, CG>(d, k, start, p.x, p.y, i, RecordsAnd<CG>{xd, omega},
-                      [&](uint32_t, const Nbr q, bool valid) { body(q, valid); },
-                      [&](uint32_t, const Nbr q, bool) { body(q, true); });
+    float2 eg      = make_float2(0.f, 0.f);
+    scan_ld<LIST, CG>(d, k, start, p, Self{i, px, pd, fabsf(wi)}, RecordsAnd<CG>{xd, omega}, VorticityPass{k}, eg);
     // only the direction of eta = grad|omega| is used, so the positive factor cs drops out; the sign stays
     const float ex = -eg.x;
     const float ey = -eg.y;
@@ -1097,7 +1270,7 @@ __device__ __forceinline__ void vorticity_one(const PbfK& k, const DomDev* __res
 }
 
 template <bool MULTI, int LIST>
-__global__ void __launch_bounds__(T_MAX)
+__global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : (LIST == LIST_FEW ? 2 : 1))
     k_vorticity(const PbfK k, const DomDev* __restrict__ doms, const int32_t* __restrict__ dom,
                 const uint32_t* __restrict__ start, const float4* __restrict__ xd,
                 const float* __restrict__ omega, float2* __restrict__ v)
@@ -1949,6 +2122,10 @@ unsigned blocks_for(int64_t n) { return (unsigned)((n + T_PART - 1) / T_PART); }
 // blocks of a neighbour-kernel launch at the tuned block size
 unsigned nblk(const gpe_pbf* s) { return (unsigned)((lsize(s) + s->block - 1) / s->block); }
 
+// The form of a listed pass: few particles are those whose warps fit the GPU at once at 64 registers a thread
+// (1024 threads an SM; see LIST_FEW)
+int list_mode(const gpe_pbf* s) { return lsize(s) <= (int64_t)1024 * gpe::sm_count() ? LIST_FEW : LIST_USE; }
+
 // ----- stage launchers ----------------------------------------------------------------------------------
 
 // A call other than a step may change what the next step sorts (positions, velocities, count, parameters,
@@ -2030,6 +2207,9 @@ cudaError_t lam_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k,
     } else if (list == LIST_USE) {
         k_lambda<M, S, A, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
         return cudaGetLastError();
+    } else if (list == LIST_FEW) {
+        k_lambda<M, S, A, LIST_FEW><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
+        return cudaGetLastError();
     } else {
         k_lambda<M, S, A, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
         return cudaGetLastError();
@@ -2048,6 +2228,9 @@ cudaError_t dp_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, 
 {
     if (list == LIST_USE) {
         k_delta_p<M, S, A, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
+        return cudaGetLastError();
+    } else if (list == LIST_FEW) {
+        k_delta_p<M, S, A, LIST_FEW><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
         return cudaGetLastError();
     } else {
         k_delta_p<M, S, A, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
@@ -2097,6 +2280,9 @@ cudaError_t xs_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, 
     if (list == LIST_USE) {
         k_xsph<M, V, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
         return cudaGetLastError();
+    } else if (list == LIST_FEW) {
+        k_xsph<M, V, LIST_FEW><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
+        return cudaGetLastError();
     } else {
         k_xsph<M, V, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
         return cudaGetLastError();
@@ -2123,7 +2309,7 @@ int32_t stage_lambda(gpe_pbf* s, cudaStream_t st, int acc)
     if (lists_on(s) && acc != ACC_PROJ) {
         // the cell marks were cleared by this step's sort (marks left by a stage sequence without one only
         // make scans full, never skip a candidate)
-        list = s->lists_valid ? LIST_USE : LIST_BUILD;
+        list = s->lists_valid ? list_mode(s) : LIST_BUILD;
     }
     GPE_TRY_CUDA(kLam[multi(s) ? 1 : 0][sg][acc](nblk(s), (unsigned)s->block, st, s->k, s->d_doms, s->dom, s->start,
                                                  s->xd[s->XS], s->lam, pid, s->acc, list));
@@ -2172,7 +2358,7 @@ int32_t stage_delta_p(gpe_pbf* s, cudaStream_t st, bool accinit)
 {
     if (lsize(s) > 0) {
         const int sc = s->prm.scorr_k != 0.f ? 1 : 0;
-        const int list = s->lists_valid ? LIST_USE : LIST_OFF;
+        const int list = s->lists_valid ? list_mode(s) : LIST_OFF;
         GPE_TRY_CUDA(kDp[multi(s) ? 1 : 0][sc][accinit ? 1 : 0](nblk(s), (unsigned)s->block, st, s->k, s->d_doms,
                                                                 s->dom, s->start, s->xd[s->XS], s->lam,
                                                                 s->xd[s->XO], s->acc, list));
@@ -2196,7 +2382,7 @@ int32_t stage_xsph(gpe_pbf* s, cudaStream_t st, bool next_hist = false)
     }
     GPE_TRY_CUDA(kXs[multi(s) ? 1 : 0][vort](nblk(s), (unsigned)s->block, st, kk, s->d_doms, s->dom, s->start,
                                              s->xd[s->XS], s->pos, s->vel, s->omega, s->status,
-                                             s->lists_valid ? LIST_USE : LIST_OFF));
+                                             s->lists_valid ? list_mode(s) : LIST_OFF));
     s->launches += 1;
     s->hist_ready = next_hist;
     return GPE_OK;
@@ -2206,25 +2392,12 @@ int32_t stage_xsph(gpe_pbf* s, cudaStream_t st, bool next_hist = false)
 int32_t stage_vorticity(gpe_pbf* s, cudaStream_t st)
 {
     if (lsize(s) == 0 || s->prm.vort_eps == 0.f) { return GPE_OK; }
-    const unsigned g = nblk(s);
-    const bool mu = s->lists_valid;
-    if (multi(s)) {
-        if (mu) {
-            k_vorticity<true, LIST_USE><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
-                                                                         s->xd[s->XS], s->omega, s->vel);
-        } else {
-            k_vorticity<true, LIST_OFF><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
-                                                                         s->xd[s->XS], s->omega, s->vel);
-        }
-    } else {
-        if (mu) {
-            k_vorticity<false, LIST_USE><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
-                                                                          s->xd[s->XS], s->omega, s->vel);
-        } else {
-            k_vorticity<false, LIST_OFF><<<g, (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start,
-                                                                          s->xd[s->XS], s->omega, s->vel);
-        }
-    }
+    const int list = s->lists_valid ? list_mode(s) : LIST_OFF;
+    auto fn        = multi(s) ? (list == LIST_OFF ? k_vorticity<true, LIST_OFF>
+                                                  : (list == LIST_USE ? k_vorticity<true, LIST_USE> : k_vorticity<true, LIST_FEW>))
+                              : (list == LIST_OFF ? k_vorticity<false, LIST_OFF>
+                                                  : (list == LIST_USE ? k_vorticity<false, LIST_USE> : k_vorticity<false, LIST_FEW>));
+    fn<<<nblk(s), (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->omega, s->vel);
     GPE_CHECK_LAUNCH("k_vorticity");
     s->launches += 1;
     return GPE_OK;
