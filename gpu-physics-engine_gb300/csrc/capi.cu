@@ -46,6 +46,19 @@ int32_t current_device(int* dev)
     return GPE_OK;
 }
 
+bool kernel_can_use(const void* p, size_t align)
+{
+    if (!p) { return true; }
+    if (reinterpret_cast<uintptr_t>(p) % align != 0) { return false; }
+    int dev = 0;
+    cudaPointerAttributes a{};
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.device == dev && (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged);
+}
+
 int32_t sm_count()
 {
     int dev = 0, n = 0;

@@ -53,6 +53,10 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 
 int32_t current_device(int* dev);
 int32_t sm_count();
+// Whether a kernel on the current device may read or write the caller's array at p: device (or managed) memory of this
+// device, aligned to `align` bytes. What fails this (another device's memory, an odd offset into an array) goes through
+// cudaMemcpyAsync, which takes any. Null arrays pass.
+bool kernel_can_use(const void* p, size_t align);
 
 // ----- counting sort of 32-bit keys (shared by PBF and the MPM spatial sort) -----
 // Workspace sizes for a sort of up to n_max items into n_keys buckets.

@@ -620,7 +620,7 @@ __global__ void k_mpm_scene_ids(int32_t n, int32_t n_scenes, const uint32_t* __r
     sid[j] = q;
 }
 
-// get_state helper: put particle i back at its original index id[i]
+// get_state: particle i at its original index id[i] (null outputs are left out)
 __global__ void k_mpm_unsort(int32_t n, const uint32_t* __restrict__ id, const float2* __restrict__ x0,
                              const float2* __restrict__ v0, const float4* __restrict__ C0,
                              const float4* __restrict__ F0, const float* __restrict__ J0, float2* __restrict__ x1,
@@ -630,25 +630,42 @@ __global__ void k_mpm_unsort(int32_t n, const uint32_t* __restrict__ id, const f
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) { return; }
     const uint32_t d = id[i];
-    x1[d]            = x0[i];
-    v1[d]            = v0[i];
-    C1[d]            = C0[i];
-    F1[d]            = F0[i];
-    J1[d]            = J0[i];
+    if (x1) { x1[d] = x0[i]; }
+    if (v1) { v1[d] = v0[i]; }
+    if (C1) { C1[d] = C0[i]; }
+    if (F1) { F1[d] = F0[i]; }
+    if (J1) { J1[d] = J0[i]; }
 }
 
-__global__ void k_mpm_init(int32_t n, uint32_t* __restrict__ id, float2* __restrict__ v, float4* __restrict__ C,
-                           float4* __restrict__ F, float* __restrict__ J, int32_t* __restrict__ mat, int set_v,
-                           int set_C, int set_F, int set_J, int set_m, int32_t material)
+// A new state: what the caller gives in device arrays is copied, what it does not give set to its default (v = 0,
+// C = 0, F = I, J = 1, the engine's material), where the arrays in `have` say that neither has been done by a copy
+// before. One launch where a copy per field, a pass for the defaults and the count's launch took 60 us at 4M particles.
+struct MpmInit {
+    const float2 *x, *v;
+    const float4 *C, *F;
+    const float* J;
+    const int32_t* mat;
+    bool have_v, have_C, have_F, have_J, have_mat; // already in place
+};
+__global__ void k_mpm_init(int32_t n, const MpmInit in, uint32_t* __restrict__ id, float2* __restrict__ x,
+                           float2* __restrict__ v, float4* __restrict__ C, float4* __restrict__ F,
+                           float* __restrict__ J, int32_t* __restrict__ mat, int32_t* __restrict__ sid,
+                           int32_t material, int32_t* __restrict__ count)
 {
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        count[0] = n;
+        count[1] = n;
+    }
     if (i >= n) { return; }
     id[i] = (uint32_t)i;
-    if (set_v) { v[i] = make_float2(0.f, 0.f); }
-    if (set_C) { C[i] = make_float4(0.f, 0.f, 0.f, 0.f); }
-    if (set_F) { F[i] = make_float4(1.f, 0.f, 0.f, 1.f); }
-    if (set_J) { J[i] = 1.f; }
-    if (set_m) { mat[i] = material; }
+    if (in.x) { x[i] = in.x[i]; }
+    if (!in.have_v) { v[i] = in.v ? in.v[i] : make_float2(0.f, 0.f); }
+    if (!in.have_C) { C[i] = in.C ? in.C[i] : make_float4(0.f, 0.f, 0.f, 0.f); }
+    if (!in.have_F) { F[i] = in.F ? in.F[i] : make_float4(1.f, 0.f, 0.f, 1.f); }
+    if (!in.have_J) { J[i] = in.J ? in.J[i] : 1.f; }
+    if (!in.have_mat) { mat[i] = in.mat ? in.mat[i] : material; }
+    if (sid) { sid[i] = 0; } // every particle in scene 0 until gpe_mpm_set_scene_ids says otherwise
 }
 
 __global__ void k_mpm_set_count(int32_t* __restrict__ c, int32_t n)
@@ -723,6 +740,7 @@ struct gpe_mpm {
     int64_t cap = 0, n = 0;
     int64_t nn  = 0; // nodes
     void* base  = nullptr;
+    size_t bytes = 0; // of base
     float2* x[2]    = {};
     float2* v[2]    = {};
     float4* C[2]    = {};
@@ -960,6 +978,15 @@ int32_t mpm_run(gpe_mpm* s, int32_t n_steps, bool do_sort, cudaStream_t st)
     return rc;
 }
 
+// Zeroes the three grids (and the padding between them: they lie one after the other in the engine's allocation).
+int32_t clear_grids(gpe_mpm* s, cudaStream_t st)
+{
+    const size_t bytes = reinterpret_cast<uint8_t*>(s->grid[2]) - reinterpret_cast<uint8_t*>(s->grid[0]) +
+                         sizeof(float4) * (size_t)s->nn;
+    GPE_TRY_CUDA(cudaMemsetAsync(s->grid[0], 0, bytes, st));
+    return GPE_OK;
+}
+
 // the engine's buffers and scene table in the kernel constants
 void bind_scenes(gpe_mpm* s)
 {
@@ -1003,6 +1030,7 @@ int32_t mpm_alloc(gpe_mpm* s)
         osc     = c.take<MpmScene>(s->scenes.size());
     }
     GPE_TRY_CUDA(cudaMalloc(&s->base, c.off));
+    s->bytes = c.off;
     GPE_TRY_CUDA(cudaMemset(s->base, 0, c.off));
     uint8_t* b = static_cast<uint8_t*>(s->base);
     for (int q = 0; q < 2; ++q) {
@@ -1155,22 +1183,39 @@ int32_t gpe_mpm_set_state(gpe_mpm* s, const float* pos, const float* vel, const 
     cudaStream_t st = as_stream(stream);
     s->cur          = 0;
     if (n > 0) {
-        GPE_TRY_CUDA(cudaMemcpyAsync(s->x[0], pos, sizeof(float2) * (size_t)n, mk_in(mem), st));
-        if (vel) { GPE_TRY_CUDA(cudaMemcpyAsync(s->v[0], vel, sizeof(float2) * (size_t)n, mk_in(mem), st)); }
-        if (C) { GPE_TRY_CUDA(cudaMemcpyAsync(s->C[0], C, sizeof(float4) * (size_t)n, mk_in(mem), st)); }
-        if (F) { GPE_TRY_CUDA(cudaMemcpyAsync(s->F[0], F, sizeof(float4) * (size_t)n, mk_in(mem), st)); }
-        if (J) { GPE_TRY_CUDA(cudaMemcpyAsync(s->J[0], J, sizeof(float) * (size_t)n, mk_in(mem), st)); }
-        if (material) {
-            GPE_TRY_CUDA(cudaMemcpyAsync(s->mat[0], material, sizeof(int32_t) * (size_t)n, mk_in(mem), st));
+        const bool direct = mem == GPE_MEM_DEVICE && gpe::kernel_can_use(pos, 8) && gpe::kernel_can_use(vel, 8) &&
+                            gpe::kernel_can_use(C, 16) && gpe::kernel_can_use(F, 16) && gpe::kernel_can_use(J, 4) &&
+                            gpe::kernel_can_use(material, 4);
+        MpmInit in{};
+        if (direct) {
+            in.x   = reinterpret_cast<const float2*>(pos);
+            in.v   = reinterpret_cast<const float2*>(vel);
+            in.C   = reinterpret_cast<const float4*>(C);
+            in.F   = reinterpret_cast<const float4*>(F);
+            in.J   = J;
+            in.mat = material;
+        } else {
+            in.have_v   = vel != nullptr;
+            in.have_C   = C != nullptr;
+            in.have_F   = F != nullptr;
+            in.have_J   = J != nullptr;
+            in.have_mat = material != nullptr;
+            GPE_TRY_CUDA(cudaMemcpyAsync(s->x[0], pos, sizeof(float2) * (size_t)n, mk_in(mem), st));
+            if (vel) { GPE_TRY_CUDA(cudaMemcpyAsync(s->v[0], vel, sizeof(float2) * (size_t)n, mk_in(mem), st)); }
+            if (C) { GPE_TRY_CUDA(cudaMemcpyAsync(s->C[0], C, sizeof(float4) * (size_t)n, mk_in(mem), st)); }
+            if (F) { GPE_TRY_CUDA(cudaMemcpyAsync(s->F[0], F, sizeof(float4) * (size_t)n, mk_in(mem), st)); }
+            if (J) { GPE_TRY_CUDA(cudaMemcpyAsync(s->J[0], J, sizeof(float) * (size_t)n, mk_in(mem), st)); }
+            if (material) {
+                GPE_TRY_CUDA(cudaMemcpyAsync(s->mat[0], material, sizeof(int32_t) * (size_t)n, mk_in(mem), st));
+            }
         }
-        k_mpm_init<<<mblocks(n), T_MPM, 0, st>>>((int32_t)n, s->id[0], s->v[0], s->C[0], s->F[0], s->J[0], s->mat[0],
-                                                  !vel, !C, !F, !J, !material, s->prm.material);
+        k_mpm_init<<<mblocks(n), T_MPM, 0, st>>>((int32_t)n, in, s->id[0], s->x[0], s->v[0], s->C[0], s->F[0], s->J[0],
+                                                  s->mat[0], s->sid[0], s->prm.material, s->d_count);
         GPE_CHECK_LAUNCH("k_mpm_init");
-        // several scenes: every particle in scene 0 until gpe_mpm_set_scene_ids says otherwise
-        if (s->sid[0]) { GPE_TRY_CUDA(cudaMemsetAsync(s->sid[0], 0, sizeof(int32_t) * (size_t)n, st)); }
+    } else {
+        k_mpm_set_count<<<1, 1, 0, st>>>(s->d_count, 0);
+        GPE_CHECK_LAUNCH("k_mpm_set_count");
     }
-    k_mpm_set_count<<<1, 1, 0, st>>>(s->d_count, (int32_t)n);
-    GPE_CHECK_LAUNCH("k_mpm_set_count");
     if (s->n != n && !s->dynamic) { s->drop_graphs(); }
     s->n                = n;
     s->k.n              = (int32_t)n;
@@ -1196,16 +1241,31 @@ int32_t gpe_mpm_get_state(gpe_mpm* s, float* pos, float* vel, float* C, float* F
     }
     if (!s->have_state) { return GPE_ERR_NOT_READY; }
     if (n > 0) {
-        // particles are returned at their original indices
+        // particles are returned at their original indices: straight into device arrays, else through the other
+        // storage set
         const int c = s->cur, o = c ^ 1;
+        // (an output inside the engine's own arrays, as gpe_mpm_buffers gives them, is not written while it is read)
+        auto outside = [&](const void* p) {
+            return reinterpret_cast<uintptr_t>(p) - reinterpret_cast<uintptr_t>(s->base) >= s->bytes;
+        };
+        const bool direct = mem == GPE_MEM_DEVICE && gpe::kernel_can_use(pos, 8) && gpe::kernel_can_use(vel, 8) &&
+                            gpe::kernel_can_use(C, 16) && gpe::kernel_can_use(F, 16) && gpe::kernel_can_use(J, 4) &&
+                            outside(pos) && outside(vel) && outside(C) && outside(F) && outside(J);
+        float2* xo = direct ? reinterpret_cast<float2*>(pos) : (pos ? s->x[o] : nullptr);
+        float2* vo = direct ? reinterpret_cast<float2*>(vel) : (vel ? s->v[o] : nullptr);
+        float4* Co = direct ? reinterpret_cast<float4*>(C) : (C ? s->C[o] : nullptr);
+        float4* Fo = direct ? reinterpret_cast<float4*>(F) : (F ? s->F[o] : nullptr);
+        float* Jo  = direct ? J : (J ? s->J[o] : nullptr);
         k_mpm_unsort<<<mblocks(n), T_MPM, 0, st>>>((int32_t)n, s->id[c], s->x[c], s->v[c], s->C[c], s->F[c], s->J[c],
-                                                   s->x[o], s->v[o], s->C[o], s->F[o], s->J[o]);
+                                                   xo, vo, Co, Fo, Jo);
         GPE_CHECK_LAUNCH("k_mpm_unsort");
-        if (pos) { GPE_TRY_CUDA(cudaMemcpyAsync(pos, s->x[o], sizeof(float2) * (size_t)n, mk_out(mem), st)); }
-        if (vel) { GPE_TRY_CUDA(cudaMemcpyAsync(vel, s->v[o], sizeof(float2) * (size_t)n, mk_out(mem), st)); }
-        if (C) { GPE_TRY_CUDA(cudaMemcpyAsync(C, s->C[o], sizeof(float4) * (size_t)n, mk_out(mem), st)); }
-        if (F) { GPE_TRY_CUDA(cudaMemcpyAsync(F, s->F[o], sizeof(float4) * (size_t)n, mk_out(mem), st)); }
-        if (J) { GPE_TRY_CUDA(cudaMemcpyAsync(J, s->J[o], sizeof(float) * (size_t)n, mk_out(mem), st)); }
+        if (!direct) {
+            if (pos) { GPE_TRY_CUDA(cudaMemcpyAsync(pos, xo, sizeof(float2) * (size_t)n, mk_out(mem), st)); }
+            if (vel) { GPE_TRY_CUDA(cudaMemcpyAsync(vel, vo, sizeof(float2) * (size_t)n, mk_out(mem), st)); }
+            if (C) { GPE_TRY_CUDA(cudaMemcpyAsync(C, Co, sizeof(float4) * (size_t)n, mk_out(mem), st)); }
+            if (F) { GPE_TRY_CUDA(cudaMemcpyAsync(F, Fo, sizeof(float4) * (size_t)n, mk_out(mem), st)); }
+            if (J) { GPE_TRY_CUDA(cudaMemcpyAsync(J, Jo, sizeof(float) * (size_t)n, mk_out(mem), st)); }
+        }
     }
     if (mem == GPE_MEM_HOST) { GPE_TRY_CUDA(cudaStreamSynchronize(st)); }
     return GPE_OK;
@@ -1268,7 +1328,8 @@ int32_t gpe_mpm_step(gpe_mpm* s, int32_t n_steps, void* stream)
     if (n_steps == 0) { return GPE_OK; }
     cudaStream_t st = as_stream(stream);
     if (s->grids_dirty) {
-        for (int q = 0; q < 3; ++q) { GPE_TRY_CUDA(cudaMemsetAsync(s->grid[q], 0, sizeof(float4) * (size_t)s->nn, st)); }
+        const int32_t rcg = clear_grids(s, st);
+        if (rcg) { return rcg; }
         s->grids_dirty = false;
     }
     const bool do_sort = s->prm.sort_interval > 0 && s->steps_since_sort >= s->prm.sort_interval;
@@ -1461,7 +1522,8 @@ int32_t gpe_mpm_enqueue(gpe_mpm* s, int32_t n_steps, void* stream)
     cudaStream_t st = as_stream(stream);
     if (n_steps == 0) { return GPE_OK; }
     // the recorded sequence starts from cleared grids and grid 0, whatever the previous sequence left
-    for (int q = 0; q < 3; ++q) { GPE_TRY_CUDA(cudaMemsetAsync(s->grid[q], 0, sizeof(float4) * (size_t)s->nn, st)); }
+    const int32_t rcg = clear_grids(s, st);
+    if (rcg) { return rcg; }
     s->ga          = 2; // mpm_run scatters the first step into grid (ga + 1) % 3 == 0
     s->grids_dirty = false;
     const int32_t rc = mpm_run(s, n_steps, false, st);

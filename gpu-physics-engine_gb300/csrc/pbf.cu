@@ -1644,6 +1644,39 @@ __global__ void k_check_domains(const int32_t* __restrict__ dom, int32_t n, int3
 
 __global__ void k_set_count(int32_t* __restrict__ c, int32_t n) { *c = n; }
 
+// A new state from device arrays in one launch: positions, velocities (zero without vel), scenes (with dom_in), ids,
+// the count, no previous multipliers, and the histogram cleared where one was left (cells > 0). Seven copies, memsets
+// and small kernels cost 10 us of a 16,384-particle step's 71 us; at 1M particles 25 us, this kernel 11.
+__global__ void __launch_bounds__(T_PART)
+    k_set_state(int32_t n, const float2* __restrict__ pos, const float2* __restrict__ vel,
+                const int32_t* __restrict__ dom_in, float2* __restrict__ x, float2* __restrict__ v,
+                int32_t* __restrict__ dom, uint32_t* __restrict__ ids, float* __restrict__ acc, int64_t cap,
+                uint32_t* __restrict__ hist, int64_t cells, int32_t* __restrict__ count)
+{
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    if (i0 == 0) { *count = n; }
+    for (int64_t i = i0; i < n; i += step) {
+        x[i]   = pos[i];
+        v[i]   = vel ? vel[i] : make_float2(0.f, 0.f);
+        ids[i] = (uint32_t)i;
+        if (dom_in) { dom[i] = dom_in[i]; }
+    }
+    // (both arrays start on 256-byte boundaries and their allocations end on one)
+    for (int64_t i = i0; 4 * i < cap; i += step) { reinterpret_cast<float4*>(acc)[i] = make_float4(0.f, 0.f, 0.f, 0.f); }
+    for (int64_t i = i0; 4 * i < cells; i += step) { reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u); }
+}
+
+// the state into device arrays in one launch (either may be null)
+__global__ void __launch_bounds__(T_PART)
+    k_get_state(int32_t n, const float2* __restrict__ x, const float2* __restrict__ v, float2* __restrict__ pos,
+                float2* __restrict__ vel)
+{
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) { return; }
+    if (pos) { pos[i] = x[i]; }
+    if (vel) { vel[i] = v[i]; }
+}
+
 // ----- hose emitter (emitterKernel, PBF.cu:968-1032): appends at the device count -------------------------
 __global__ void k_pbf_emit(const PbfK k, const HoseK h, float2* __restrict__ x, float2* __restrict__ v,
                            int32_t* __restrict__ count, int32_t cap, uint32_t* __restrict__ ids,
@@ -1948,12 +1981,12 @@ struct gpe_pbf {
     uint16_t* feat    = nullptr;  // network operand tiles (GPE_WARM_MLP), allocated on demand
     float skin        = 0.075f;   // candidate-list skin in units of h (tuning; 0: full scans only)
     uint4* nhdr       = nullptr;  // candidate lists of the current step: headers
-    uint4* nlist      = nullptr;  // ... and chunks, an allocation of their own (null: none, full scans only)
+    uint4* nlist      = nullptr;  // ... and chunks (null: no room for them, full scans only)
     bool wide         = false;    // ... of 32-bit slots
     uint8_t* mflag    = nullptr;  // per cell: a particle of its 3 x 3 cells moved too far for the lists
     bool lists_valid  = false;    // the lists were made in this step
     bool hist_ready   = false;    // the last step's XSPH left the next step's cell keys and histogram
-    bool count_dirty  = false;    // ... and was dropped: the histogram array must be cleared before a sort
+    int64_t dirty_cells = 0;      // ... and was dropped: so many of the histogram's cells must be cleared before a sort
 
     // within a step (after PREDICT_SORT): XS = the current (x, d) records, XO = the other buffer; -1 between steps
     int XS = -1, XO = -1;
@@ -2135,15 +2168,15 @@ void drop_hist(gpe_pbf* s)
 {
     if (s->hist_ready) {
         s->hist_ready  = false;
-        s->count_dirty = true;
+        s->dirty_cells = std::max<int64_t>(s->dirty_cells, s->ncells);
     }
 }
 
 int32_t clear_hist(gpe_pbf* s, cudaStream_t st)
 {
-    if (s->count_dirty) {
-        GPE_TRY_CUDA(cudaMemsetAsync(s->count, 0, sizeof(uint32_t) * (size_t)s->cells_cap, st));
-        s->count_dirty = false;
+    if (s->dirty_cells > 0) {
+        GPE_TRY_CUDA(cudaMemsetAsync(s->count, 0, sizeof(uint32_t) * (size_t)s->dirty_cells, st));
+        s->dirty_cells = 0;
     }
     return GPE_OK;
 }
@@ -2628,7 +2661,19 @@ int32_t alloc_buffers(gpe_pbf* s)
     const size_t o_gs    = c.take<GridSync>(1);
     const size_t o_nm    = c.take<uint4>(N);
     const size_t o_mf    = c.take<uint8_t>(M);
-    GPE_TRY_CUDA(cudaMalloc(&s->base, c.off));
+    // Candidate lists, behind the rest: 96 bytes a particle, 192 with 32-bit slots, of which a step touches what its
+    // lists fill (32 on a lattice of spacing h / 2). Slots of 16 bits reach 2^15 away: the next cell row of a scene
+    // 4096 cells wide at up to 8 particles a cell; wider scenes take 32-bit slots. Without room for the lists the
+    // passes scan in full.
+    float widest = 0.f;
+    for (const gpe_domain& d : s->doms) { widest = std::max(widest, d.extent[0]); }
+    s->wide                 = widest > 4096.f * s->prm.h;
+    const size_t list_bytes = sizeof(uint4) * (LIST_MAX / (s->wide ? 4 : 8)) * std::max<size_t>(N, 1);
+    const bool lists        = cudaMalloc(&s->base, c.off + list_bytes) == cudaSuccess;
+    if (!lists) {
+        cudaGetLastError();
+        GPE_TRY_CUDA(cudaMalloc(&s->base, c.off));
+    }
     GPE_TRY_CUDA(cudaMemset(s->base, 0, c.off));
     uint8_t* b = static_cast<uint8_t*>(s->base);
     s->d_doms  = reinterpret_cast<DomDev*>(b + o_doms);
@@ -2657,16 +2702,7 @@ int32_t alloc_buffers(gpe_pbf* s)
     s->gsync   = reinterpret_cast<GridSync*>(b + o_gs);
     s->nhdr   = reinterpret_cast<uint4*>(b + o_nm);
     s->mflag   = b + o_mf;
-    // Candidate lists: 96 bytes a particle, 192 with 32-bit slots, of which a step touches what its lists fill (32 on
-    // a lattice of spacing h / 2). Slots of 16 bits reach 2^15 away: the next cell row of a scene 4096 cells wide
-    // at up to 8 particles a cell; wider scenes take 32-bit slots. Without room for them the passes scan in full.
-    float widest = 0.f;
-    for (const gpe_domain& d : s->doms) { widest = std::max(widest, d.extent[0]); }
-    s->wide = widest > 4096.f * s->prm.h;
-    if (cudaMalloc(&s->nlist, sizeof(uint4) * (LIST_MAX / (s->wide ? 4 : 8)) * std::max<size_t>(N, 1)) != cudaSuccess) {
-        cudaGetLastError();
-        s->nlist = nullptr;
-    }
+    s->nlist   = lists ? reinterpret_cast<uint4*>(b + c.off) : nullptr;
     bind_k(s);
     GPE_TRY_CUDA(cudaMemcpy(s->d_doms, s->domdev.data(), sizeof(DomDev) * (size_t)s->nd, cudaMemcpyHostToDevice));
     return GPE_OK;
@@ -2731,7 +2767,6 @@ int32_t gpe_pbf_create(const gpe_pbf_params* params, const gpe_domain* domains, 
     rc = alloc_buffers(s);
     if (rc) {
         if (s->base) { cudaFree(s->base); }
-        if (s->nlist) { cudaFree(s->nlist); }
         delete s;
         return rc;
     }
@@ -2744,7 +2779,6 @@ int32_t gpe_pbf_destroy(gpe_pbf* s)
     if (!s) { return GPE_ERR_BAD_ARG; }
     s->drop_graphs();
     if (s->base) { cudaFree(s->base); }
-    if (s->nlist) { cudaFree(s->nlist); }
     if (s->feat) { cudaFree(s->feat); }
     delete s;
     return GPE_OK;
@@ -2808,36 +2842,49 @@ int32_t gpe_pbf_set_state(gpe_pbf* s, const float* pos, const float* vel, const 
     drop_hist(s);
     s->XS = s->XO   = -1;
     s->id_cur     = 0;
-    if (n > 0) {
+    const int32_t* dom_in = s->nd > 1 ? domain_id : nullptr;
+    const bool direct     = n > 0 && mem == GPE_MEM_DEVICE && gpe::kernel_can_use(pos, 8) &&
+                        gpe::kernel_can_use(vel, 8) && gpe::kernel_can_use(dom_in, 4);
+    if (!direct && n > 0 && dom_in) {
+        GPE_TRY_CUDA(cudaMemcpyAsync(s->dom, dom_in, sizeof(int32_t) * (size_t)n, kind_in(mem), st));
+    }
+    if (n > 0 && dom_in && mem == GPE_MEM_DEVICE) {
+        k_check_domains<<<blocks_for(n), T_PART, 0, st>>>(direct ? dom_in : s->dom, (int32_t)n, s->nd, s->status);
+        GPE_CHECK_LAUNCH("k_check_domains");
+        uint32_t stt = 0;
+        GPE_TRY_CUDA(cudaMemcpyAsync(&stt, s->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        GPE_TRY_CUDA(cudaStreamSynchronize(st));
+        if (stt & GPE_STATUS_CAPACITY) {
+            GPE_TRY_CUDA(cudaMemsetAsync(s->status, 0, sizeof(uint32_t), st));
+            gpe::set_error(GPE_ERR_BAD_ARG,
+                           "gpe_pbf_set_state: domain_id must be in [0, n_domains) and non-decreasing");
+            return GPE_ERR_BAD_ARG;
+        }
+    }
+    if (direct) {
+        const int64_t cells = s->dirty_cells;
+        const int64_t work  = std::max<int64_t>({n, s->cap / 4, cells / 4});
+        k_set_state<<<(unsigned)std::min<int64_t>((work + T_PART - 1) / T_PART, (int64_t)gpe::sm_count() * 32), T_PART,
+                      0, st>>>((int32_t)n, reinterpret_cast<const float2*>(pos), reinterpret_cast<const float2*>(vel),
+                               dom_in, s->pos, s->vel, s->dom, s->ids[0], s->acc, s->cap, s->count, cells, s->d_count);
+        GPE_CHECK_LAUNCH("k_set_state");
+        s->dirty_cells = 0;
+    } else if (n > 0) {
         GPE_TRY_CUDA(cudaMemcpyAsync(s->pos, pos, sizeof(float2) * (size_t)n, kind_in(mem), st));
         if (vel) {
             GPE_TRY_CUDA(cudaMemcpyAsync(s->vel, vel, sizeof(float2) * (size_t)n, kind_in(mem), st));
         } else {
             GPE_TRY_CUDA(cudaMemsetAsync(s->vel, 0, sizeof(float2) * (size_t)n, st));
         }
-        if (s->nd > 1) {
-            GPE_TRY_CUDA(cudaMemcpyAsync(s->dom, domain_id, sizeof(int32_t) * (size_t)n, kind_in(mem), st));
-            if (mem == GPE_MEM_DEVICE) {
-                k_check_domains<<<blocks_for(n), T_PART, 0, st>>>(s->dom, (int32_t)n, s->nd, s->status);
-                GPE_CHECK_LAUNCH("k_check_domains");
-                uint32_t stt = 0;
-                GPE_TRY_CUDA(cudaMemcpyAsync(&stt, s->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-                GPE_TRY_CUDA(cudaStreamSynchronize(st));
-                if (stt & GPE_STATUS_CAPACITY) {
-                    GPE_TRY_CUDA(cudaMemsetAsync(s->status, 0, sizeof(uint32_t), st));
-                    gpe::set_error(GPE_ERR_BAD_ARG,
-                                   "gpe_pbf_set_state: domain_id must be in [0, n_domains) and non-decreasing");
-                    return GPE_ERR_BAD_ARG;
-                }
-            }
-        }
         k_iota<<<blocks_for(n), T_PART, 0, st>>>(s->ids[0], (int32_t)n);
         GPE_CHECK_LAUNCH("k_iota");
     }
-    k_set_count<<<1, 1, 0, st>>>(s->d_count, (int32_t)n);
-    GPE_CHECK_LAUNCH("k_set_count");
-    // a new particle set has no previous multipliers
-    GPE_TRY_CUDA(cudaMemsetAsync(s->acc, 0, sizeof(float) * (size_t)s->cap, st));
+    if (!direct) {
+        k_set_count<<<1, 1, 0, st>>>(s->d_count, (int32_t)n);
+        GPE_CHECK_LAUNCH("k_set_count");
+        // a new particle set has no previous multipliers
+        GPE_TRY_CUDA(cudaMemsetAsync(s->acc, 0, sizeof(float) * (size_t)s->cap, st));
+    }
     if (s->n != n && !s->dynamic) { s->drop_graphs(); }
     s->n          = n;
     s->have_state = true;
@@ -2860,8 +2907,14 @@ int32_t gpe_pbf_get_state(gpe_pbf* s, float* pos, float* vel, int32_t* domain_id
     }
     if (!s->have_state) { return GPE_ERR_NOT_READY; }
     if (n > 0) {
-        if (pos) { GPE_TRY_CUDA(cudaMemcpyAsync(pos, s->pos, sizeof(float2) * (size_t)n, kind_out(mem), st)); }
-        if (vel) { GPE_TRY_CUDA(cudaMemcpyAsync(vel, s->vel, sizeof(float2) * (size_t)n, kind_out(mem), st)); }
+        if (mem == GPE_MEM_DEVICE && pos && vel && gpe::kernel_can_use(pos, 8) && gpe::kernel_can_use(vel, 8)) {
+            k_get_state<<<blocks_for(n), T_PART, 0, st>>>((int32_t)n, s->pos, s->vel, reinterpret_cast<float2*>(pos),
+                                                          reinterpret_cast<float2*>(vel));
+            GPE_CHECK_LAUNCH("k_get_state");
+        } else {
+            if (pos) { GPE_TRY_CUDA(cudaMemcpyAsync(pos, s->pos, sizeof(float2) * (size_t)n, kind_out(mem), st)); }
+            if (vel) { GPE_TRY_CUDA(cudaMemcpyAsync(vel, s->vel, sizeof(float2) * (size_t)n, kind_out(mem), st)); }
+        }
         if (domain_id) {
             if (s->nd > 1) {
                 GPE_TRY_CUDA(cudaMemcpyAsync(domain_id, s->dom, sizeof(int32_t) * (size_t)n, kind_out(mem), st));
@@ -2920,7 +2973,7 @@ int32_t gpe_pbf_step(gpe_pbf* s, int32_t n_steps, void* stream)
     // the step sequence is captured once per (steps, whether the first sort's histogram is already there,
     // starting buffer roles) and replayed as one graph; every step but none in between leaves the next
     // step's keys and histogram (stage_xsph)
-    const auto key = std::make_tuple(n_steps, (s->hist_ready ? 1 : 0) + (s->count_dirty ? 2 : 0), s->id_cur);
+    const auto key = std::make_tuple(n_steps, (s->hist_ready ? 1 : 0) + (s->dirty_cells > 0 ? 2 : 0), s->id_cur);
     auto it        = s->graphs.find(key);
     if (it == s->graphs.end()) {
         cudaStream_t cap_st = st;
@@ -2930,7 +2983,8 @@ int32_t gpe_pbf_step(gpe_pbf* s, int32_t n_steps, void* stream)
             own = true;
         }
         const int id0    = s->id_cur;
-        const bool hist0 = s->hist_ready, dirty0 = s->count_dirty;
+        const bool hist0     = s->hist_ready;
+        const int64_t dirty0 = s->dirty_cells;
         GPE_TRY_CUDA(cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
         s->launches = 0;
         int32_t rc  = GPE_OK;
@@ -2942,7 +2996,7 @@ int32_t gpe_pbf_step(gpe_pbf* s, int32_t n_steps, void* stream)
         pg.hist_end   = s->hist_ready;
         s->id_cur     = id0;
         s->hist_ready = hist0;
-        s->count_dirty = dirty0;
+        s->dirty_cells = dirty0;
         if (rc == GPE_OK && ce != cudaSuccess) {
             gpe::set_cuda_error(ce, "cudaStreamEndCapture");
             rc = GPE_ERR_CUDA;
@@ -2963,7 +3017,7 @@ int32_t gpe_pbf_step(gpe_pbf* s, int32_t n_steps, void* stream)
     GPE_TRY_CUDA(cudaGraphLaunch(it->second.exec, st));
     s->id_cur      = it->second.id_end;
     s->hist_ready  = it->second.hist_end;
-    s->count_dirty = false; // the graph's first sort cleared it
+    s->dirty_cells = 0; // the graph's first sort cleared it
     s->have_sort  = true;
     return GPE_OK;
 }
@@ -3359,7 +3413,7 @@ extern "C" int32_t gpe_pbf_enqueue(gpe_pbf* s, int32_t n_steps, void* stream)
     // in the array): it clears the histogram array, starts from the full sort and leaves no histogram behind
     // (its last step's XSPH computes none)
     drop_hist(s);
-    s->count_dirty = true;
+    s->dirty_cells = std::max<int64_t>(s->dirty_cells, s->ncells);
     int32_t rc    = GPE_OK;
     const int id0 = s->id_cur;
     for (int32_t k = 0; k < n_steps && rc == GPE_OK; ++k) { rc = run_step(s, st, k + 1 < n_steps); }
