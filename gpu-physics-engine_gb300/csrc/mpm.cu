@@ -2,19 +2,20 @@
 //
 // The reference runs, per substep, resetGrid -> P2GKernel -> gridKernel -> G2PKernel (MPM.cu:353-371) with
 // 27 scalar global atomics per particle (MPM.cu:124-126) and a separate streaming pass over the grid.
-// Here one step is three launches:
-//   k_p2g            P2G, two consecutive particles per thread: lanes that share a stencil base node
-//                    (particles are kept sorted by base node) sum their contributions per node with a
-//                    segmented shuffle reduction, and the run's first lane adds each of its 9 node sums to
-//                    the grid with one vector global atomic (red.global.add.v4.f32, resolved in L2).
+// Here the steps of a call are two launches each (and one more, P2G, before the first, whose G2P is the last's):
 //   k_grid_vel       the grid update (v = p/m + g dt, walls, MPM.cu:150-175) once per node into an array of
 //                    node velocities (8 bytes a node), zeroing the grid read two steps earlier in the same
 //                    pass (three grids rotate).
-//   k_g2p            G2P: each particle gathers its 9 node velocities from that array (L1/L2 hits: sorted
-//                    neighbours share nodes).
+//   k_g2p2g          G2P of the step and P2G of the next, two consecutive particles per thread: each gathers its 9 node
+//                    velocities from that array (L1/L2 hits: sorted neighbours share nodes), is updated, and the warp
+//                    scatters its 64 particles to the next grid (scatter_pair), lanes that share a stencil base node
+//                    summing their contributions first. Its bound is instruction issue (72%, 4 blocks of 256 an SM at
+//                    64 registers): 4M mixed particles 125 us a step where k_p2g and k_g2p took 103 and 64.
+//   k_p2g, k_g2p     the halves of the first and the last step.
 // (Measured alternatives, each slower: a G2P that staged its block's node box in shared memory and updated
-// each node there, 0.198 against 0.186 ms per step at 4M particles; a G2P fused with the next step's P2G,
-// 0.159 against 0.153 ms, its 64 registers holding both passes' state.)
+// each node there, 0.198 against 0.186 ms per step at 4M particles; the fused kernel with both particles side by side
+// and velocity and affine matrix written as in k_g2p, 0.159 against 0.153 ms for the separate kernels; at 5 and 6 blocks
+// an SM it spills, 135 and 144 us against 131.)
 // Stage kernels (k_clear, k_p2g, k_grid, k_g2p on an updated grid) reproduce the reference's four kernels
 // one to one for stage-level parity tests.
 #include <cuda_runtime.h>
@@ -360,35 +361,171 @@ __device__ __forceinline__ void g2p_finish(const MpmK& k, const MpmScene& sc, in
     }
 }
 
-// The node term of one particle (stencil s, velocity v, affine matrix Q) for node (i, j) of its stencil,
-// added to (c, cm): w (m v + Q dp) and w m (particleToGrid, MPM.cu:116-126); momentum as packed FP32 pairs
-__device__ __forceinline__ void p2g_term(const MpmK& k, const Stencil& s, float2 v, float4 Q, int i, int j,
-                                         float2& c, float& cm)
+// What a particle scatters to its 9 nodes: w_ij (m v + Q dp_ij) and w_ij m (particleToGrid, MPM.cu:116-126), dp_ij =
+// (i - fx, j - fy) dx from the particle's base node, `node` in the node array (0xffffffff: no particle) whose rows are
+// nx nodes long. Qx, Qy are the columns of Q; the 2D terms are packed FP32 pairs.
+struct Scatter {
+    float2 mv, Qx, Qy;
+    float fx, fy;
+    uint32_t node;
+    int32_t nx;
+};
+
+__device__ __forceinline__ Scatter scatter_of(const MpmK& k, const MpmScene& sc, const Stencil& s, float2 v, float4 Q)
 {
-    const float w   = s.wx[i] * s.wy[j];
-    const float dpx = ((float)i - s.fx) * k.dx;
-    const float dpy = ((float)j - s.fy) * k.dx;
-    const float2 a  = fma2(make_float2(Q.y, Q.w), make_float2(dpy, dpy),
-                           mul2(make_float2(Q.x, Q.z), make_float2(dpx, dpx)));
-    c               = add2(c, mul2(make_float2(w, w), fma2(v, make_float2(k.mass, k.mass), a)));
-    cm += w * k.mass;
+    return Scatter{make_float2(k.mass * v.x, k.mass * v.y), make_float2(Q.x, Q.z), make_float2(Q.y, Q.w), s.fx, s.fy,
+                   sc.goff + (uint32_t)s.by * (uint32_t)sc.nx + (uint32_t)s.bx, sc.nx};
 }
 
-// particle i's scene, stencil, velocity and affine matrix for P2G
-template <int MODE, bool MS>
-__device__ __forceinline__ void p2g_load(const MpmK& k, const float2* __restrict__ x, const float2* __restrict__ v,
-                                         const float4* __restrict__ C, const float4* __restrict__ F,
-                                         const float* __restrict__ J, const int32_t* __restrict__ mat,
-                                         const int32_t* __restrict__ sid, int32_t i, MpmScene& sc, Stencil& s,
-                                         float2& vv, float4& Q, uint32_t* status)
+// the quadratic B-spline weight of node i of a particle f nodes past its base node, MPM.cu:92-110
+__device__ __forceinline__ float weight(float f, int i)
 {
-    sc              = scene_of<MS>(k, sid, i);
-    const int m     = mat_of(k, MODE, mat, i);
-    const float4 Fp = (m == MODE_FLUID) ? make_float4(1.f, 0.f, 0.f, 1.f) : F[i];
-    const float Jp  = keeps_j(m) ? J[i] : 1.f;
-    Q               = affine(k, m, C[i], Fp, Jp);
-    vv              = v[i];
-    s               = stencil(k, sc, x[i], status);
+    return i == 0 ? 0.5f * (1.5f - f) * (1.5f - f)
+                  : (i == 1 ? 0.75f - (f - 1.0f) * (f - 1.0f) : 0.5f * (f - 0.5f) * (f - 0.5f));
+}
+
+// One particle's terms of the three nodes of its stencil's column i: (m v + Qx dpx) is the column's, so a node costs two
+// multiplies and three fused multiply-adds.
+struct ColumnTerms {
+    float2 mv, Qy;
+    float wx, fy;
+    __device__ __forceinline__ ColumnTerms(const MpmK& k, const Scatter& p, int i) : Qy(p.Qy), fy(p.fy)
+    {
+        const float dpx = ((float)i - p.fx) * k.dx;
+        mv              = fma2(p.Qx, make_float2(dpx, dpx), p.mv);
+        wx              = weight(p.fx, i);
+    }
+    // adds node j's momentum to c and its mass to cm; wy is the row's weight
+    __device__ __forceinline__ void add(const MpmK& k, int j, float wy, float2& c, float& cm) const
+    {
+        const float w   = wx * wy;
+        const float dpy = ((float)j - fy) * k.dx;
+        c               = fma2(make_float2(w, w), fma2(Qy, make_float2(dpy, dpy), mv), c);
+        cm              = fmaf(w, k.mass, cm);
+    }
+};
+
+// The scatter of a thread's two particles a, b (consecutive in storage), by whole warps. Particles are kept sorted by
+// stencil base node (or at least stored in some spatial order), so consecutive lanes mostly share their base node and
+// with it all 9 target nodes. The lanes whose second particle has the same base node form a run. A first particle joins
+// its thread's run, or else the run of the lane before, whose last particle it then is; the few that fit neither add
+// their 9 terms to the grid by themselves. Per node the lanes of a run sum their contributions with a segmented shuffle
+// reduction (as many rounds as the warp's longest run needs), and the run's first lane adds the sums to the grid with
+// vector global atomics (red.global.add.v4.f32, resolved in L2). Runs on neighbouring base nodes of a row, which
+// overlap in two of their three columns, first hand those columns on to the next run (CHAIN_RUNS and more runs a warp),
+// so that all but the last of them have one column left to add: the atomics are what bounds the scatter of particles
+// that are not sorted.
+// One particle per thread measured slower: 0.185 against 0.153 ms per 4M-particle step, its shuffle rounds covering
+// half as many particles; staging node sums in a shared-memory tile of the block's nodes (float atomics on shared
+// memory, a block barrier, a flush) slower again. status[2] counts the warps that need the fifth round (a run of more
+// than 16 lanes).
+constexpr int CHAIN_RUNS = 12; // (2, 6, 12 and never: 4.67, 4.66, 4.64, 4.67 ms for 32 steps of 4M sorted particles; 276, 274,
+                               // 274, 310 us for 20 steps of 262,147 in lattice order)
+__device__ __forceinline__ void scatter_pair(const MpmK& k, const Scatter& a, const Scatter& b,
+                                             float4* __restrict__ grid, uint32_t* status)
+{
+    constexpr uint32_t ALL = 0xffffffffu;
+    const bool ok0 = a.node != ALL, ok1 = b.node != ALL;
+    const uint32_t lane    = threadIdx.x & 31u;
+    const uint32_t prev    = __shfl_up_sync(ALL, b.node, 1);
+    const bool join        = ok1 && a.node == b.node;
+    const bool give        = ok0 && !join && lane != 0u && prev == a.node;
+    const bool solo        = ok0 && !join && !give;
+    const bool head        = lane == 0u || prev != b.node;
+    const uint32_t heads   = __ballot_sync(ALL, head);
+    const uint32_t later   = lane == 31u ? 0u : (heads & (ALL << (lane + 1u)));
+    const uint32_t run_end = later ? (uint32_t)(__ffs(later) - 1) : 32u; // first lane of the next run
+    const uint32_t longest = __reduce_max_sync(ALL, head ? run_end - lane : 0u);
+    if (longest > 16u && lane == 0u) { atomicAdd(status + 2, 1u); }
+    float2 c[9]; // column i, row j at 3 i + j
+    float cm[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const ColumnTerms ta(k, a, i), tb(k, b, i);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int q = 3 * i + j;
+            float2 t    = make_float2(0.f, 0.f);
+            float tm    = 0.f;
+            ta.add(k, j, weight(a.fy, j), t, tm);
+            c[q]  = join ? t : make_float2(0.f, 0.f);
+            cm[q] = join ? tm : 0.f;
+            if (ok1) { tb.add(k, j, weight(b.fy, j), c[q], cm[q]); }
+            const float ox = __shfl_down_sync(ALL, give ? t.x : 0.f, 1);
+            const float oy = __shfl_down_sync(ALL, give ? t.y : 0.f, 1);
+            const float om = __shfl_down_sync(ALL, give ? tm : 0.f, 1);
+            if (lane != 31u) {
+                c[q] = add2(c[q], make_float2(ox, oy));
+                cm[q] += om;
+            }
+        }
+    }
+    // (a loop: one copy of the nine nodes' shuffles keeps the kernel in the instruction cache)
+#pragma unroll 1
+    for (uint32_t d = 1u; d < longest; d <<= 1) {
+        const bool take = lane + d < run_end;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            const float ox = __shfl_down_sync(ALL, c[q].x, d);
+            const float oy = __shfl_down_sync(ALL, c[q].y, d);
+            const float om = __shfl_down_sync(ALL, cm[q], d);
+            if (take) {
+                c[q] = add2(c[q], make_float2(ox, oy));
+                cm[q] += om;
+            }
+        }
+    }
+    bool rest = head && ok1; // this lane adds its run's second and third column too
+    if (__popc(heads) >= CHAIN_RUNS) {
+        const uint32_t before = heads & ((1u << lane) - 1u);
+        const int hp          = before ? 31 - __clz(before) : (int)lane; // the run before
+        const uint32_t pnode  = __shfl_sync(ALL, b.node, hp);
+        const bool next_to    = rest && before != 0u && pnode + 1u == b.node; // (base nodes end three short of a row)
+        const bool followed   = __shfl_sync(ALL, next_to ? 1 : 0, (int)(run_end & 31u)) != 0 && run_end < 32u;
+        // column 2 of the run before is this run's column 1, the sum of that its column 0
+#pragma unroll
+        for (int i = 1; i >= 0; --i) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const int q    = 3 * i + j;
+                const float ox = __shfl_sync(ALL, c[q + 3].x, hp);
+                const float oy = __shfl_sync(ALL, c[q + 3].y, hp);
+                const float om = __shfl_sync(ALL, cm[q + 3], hp);
+                if (next_to) {
+                    c[q] = add2(c[q], make_float2(ox, oy));
+                    cm[q] += om;
+                }
+            }
+        }
+        rest = rest && !followed;
+    }
+    if (head && ok1) {
+        float4* const base = grid + (size_t)b.node;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            atomicAdd(base + (size_t)q * (size_t)b.nx, make_float4(c[q].x, c[q].y, cm[q], 0.f));
+        }
+        if (rest) {
+#pragma unroll
+            for (int q = 3; q < 9; ++q) {
+                atomicAdd(base + (size_t)(q % 3) * (size_t)b.nx + q / 3, make_float4(c[q].x, c[q].y, cm[q], 0.f));
+            }
+        }
+    }
+    if (solo) {
+        float4* const base = grid + (size_t)a.node;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const ColumnTerms ta(k, a, i);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                float2 t = make_float2(0.f, 0.f);
+                float tm = 0.f;
+                ta.add(k, j, weight(a.fy, j), t, tm);
+                atomicAdd(base + (size_t)j * (size_t)a.nx + i, make_float4(t.x, t.y, tm, 0.f));
+            }
+        }
+    }
 }
 
 // ----- kernels -------------------------------------------------------------------------------------------
@@ -401,89 +538,30 @@ __global__ void k_clear(float4* __restrict__ grid, int64_t nn)
     }
 }
 
-// P2G, two consecutive particles per thread (particles 2t and 2t + 1). Particles are kept sorted by stencil
-// base node, so consecutive lanes mostly share their base node and with it all 9 target nodes. When a
-// thread's two particles share one, their terms are summed in registers; then, for each node, the lanes of a
-// run (consecutive lanes with the same base node, 64 particles a warp) sum their contributions with a
-// segmented shuffle reduction (2 to 5 rounds, as the warp's longest run needs), and the run's first lane adds
-// the node sum to the grid with one vector global atomic (red.global.add.v4.f32, resolved in L2). A first
-// particle whose base node differs from its partner's (a run boundary inside the thread) adds its 9 terms
-// with atomics of its own. One particle per thread measured slower: 0.185 against 0.153 ms per 4M-particle
-// step, its shuffle rounds covering half as many particles; staging node sums in a shared-memory tile of the
-// block's nodes (float atomics on shared memory, a block barrier, a flush) slower again.
-// status[2] counts the warps that need the 5-round reduction (a run of more than 16 lanes).
+// P2G of particles 2t and 2t + 1 (see scatter_pair)
 template <int MODE, bool MS>
-__global__ void __launch_bounds__(T_MPM)
+__global__ void __launch_bounds__(T_MPM, 4)
     k_p2g(const MpmK k, const float2* __restrict__ x, const float2* __restrict__ v, const float4* __restrict__ C,
           const float4* __restrict__ F, const float* __restrict__ J, const int32_t* __restrict__ mat,
           const int32_t* __restrict__ sid, float4* __restrict__ grid, uint32_t* status)
 {
-    const int32_t t  = blockIdx.x * blockDim.x + threadIdx.x;
+    const int32_t i0 = 2 * (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     const int32_t n  = count_of(k);
-    const int32_t i0 = 2 * t, i1 = 2 * t + 1;
-    const bool ok0 = i0 < n, ok1 = i1 < n;
-    MpmScene sc0 = k.s0, sc1 = k.s0;
-    Stencil s0{}, s1{};
-    float2 v0 = make_float2(0.f, 0.f), v1 = v0;
-    float4 Q0 = make_float4(0.f, 0.f, 0.f, 0.f), Q1 = Q0;
-    if (ok0) { p2g_load<MODE, MS>(k, x, v, C, F, J, mat, sid, i0, sc0, s0, v0, Q0, status); }
-    if (ok1) { p2g_load<MODE, MS>(k, x, v, C, F, J, mat, sid, i1, sc1, s1, v1, Q1, status); }
-    const uint32_t key0 = ok0 ? sc0.goff + (uint32_t)s0.by * (uint32_t)sc0.nx + (uint32_t)s0.bx : 0xffffffffu;
-    const uint32_t key1 = ok1 ? sc1.goff + (uint32_t)s1.by * (uint32_t)sc1.nx + (uint32_t)s1.bx : 0xffffffffu;
-    const bool join = ok1 && key0 == key1; // the first particle joins the thread's run
-    const bool solo = ok0 && !join;        // the first particle goes to the grid on its own
-    // runs of lanes with the same base node (that of the second particle)
-    const uint32_t lane    = threadIdx.x & 31u;
-    const uint32_t prev    = __shfl_up_sync(0xffffffffu, key1, 1);
-    const bool head        = lane == 0u || prev != key1;
-    const uint32_t heads   = __ballot_sync(0xffffffffu, head);
-    const uint32_t later   = lane == 31u ? 0u : (heads & (0xffffffffu << (lane + 1u)));
-    const uint32_t run_end = later ? (uint32_t)(__ffs(later) - 1) : 32u; // first lane of the next run
-    const uint32_t longest = __reduce_max_sync(0xffffffffu, head ? run_end - lane : 0u);
-    float4* const base1    = grid + (size_t)sc1.goff + (size_t)s1.by * (size_t)sc1.nx + (size_t)s1.bx;
-    auto scatter = [&](auto rounds) {
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const int i = q % 3, j = q / 3;
-            float2 c = make_float2(0.f, 0.f);
-            float cm = 0.f;
-            if (join) { p2g_term(k, s0, v0, Q0, i, j, c, cm); }
-            if (ok1) { p2g_term(k, s1, v1, Q1, i, j, c, cm); }
-#pragma unroll
-            for (uint32_t d = 1u; d < (1u << decltype(rounds)::value); d <<= 1) {
-                const float ox = __shfl_down_sync(0xffffffffu, c.x, d);
-                const float oy = __shfl_down_sync(0xffffffffu, c.y, d);
-                const float om = __shfl_down_sync(0xffffffffu, cm, d);
-                if (lane + d < run_end) {
-                    c = add2(c, make_float2(ox, oy));
-                    cm += om;
-                }
-            }
-            if (head && ok1) { atomicAdd(base1 + (size_t)j * (size_t)sc1.nx + i, make_float4(c.x, c.y, cm, 0.f)); }
+    auto load = [&](int32_t i) {
+        Scatter p{};
+        p.node = 0xffffffffu;
+        if (i < n) {
+            const MpmScene sc = scene_of<MS>(k, sid, i);
+            const int m       = mat_of(k, MODE, mat, i);
+            const float4 Fp   = (m == MODE_FLUID) ? make_float4(1.f, 0.f, 0.f, 1.f) : F[i];
+            const float Jp    = keeps_j(m) ? J[i] : 1.f;
+            const float4 Q    = affine(k, m, C[i], Fp, Jp);
+            p                 = scatter_of(k, sc, stencil(k, sc, x[i], status), v[i], Q);
         }
+        return p;
     };
-    // warp-uniform branches on the longest run
-    if (longest <= 4u) {
-        scatter(std::integral_constant<int, 2>{});
-    } else if (longest <= 8u) {
-        scatter(std::integral_constant<int, 3>{});
-    } else if (longest <= 16u) {
-        scatter(std::integral_constant<int, 4>{});
-    } else {
-        if (lane == 0u) { atomicAdd(status + 2, 1u); }
-        scatter(std::integral_constant<int, 5>{});
-    }
-    if (solo) {
-        float4* const base0 = grid + (size_t)sc0.goff + (size_t)s0.by * (size_t)sc0.nx + (size_t)s0.bx;
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const int i = q % 3, j = q / 3;
-            float2 c = make_float2(0.f, 0.f);
-            float cm = 0.f;
-            p2g_term(k, s0, v0, Q0, i, j, c, cm);
-            atomicAdd(base0 + (size_t)j * (size_t)sc0.nx + i, make_float4(c.x, c.y, cm, 0.f));
-        }
-    }
+    const Scatter a = load(i0), b = load(i0 + 1);
+    scatter_pair(k, a, b, grid, status);
 }
 
 // gridKernel, MPM.cu:131-177 (in place)
@@ -548,6 +626,50 @@ __global__ void __launch_bounds__(T_MPM, 6)
     C[i] = ps.C;
     if (keeps_f(m, track_f)) { F[i] = ps.F; }
     if (keeps_j(m)) { J[i] = ps.J; }
+}
+
+// G2P of one step and P2G of the next in one launch, for the steps of a call but its last: velocity and affine matrix
+// pass from one to the other in registers and never reach memory (60 bytes a particle instead of 140), and the
+// gather's latency overlaps the scatter's arithmetic. The two particles of a thread go through G2P one after the other
+// (not unrolled: side by side they take 64 registers and half the warps).
+template <int MODE, bool MS>
+__global__ void __launch_bounds__(T_MPM, 4)
+    k_g2p2g(const MpmK k, const float2* __restrict__ vel, float2* __restrict__ x, float4* __restrict__ F,
+            float* __restrict__ J, const int32_t* __restrict__ mat, const int32_t* __restrict__ sid,
+            float4* __restrict__ grid, uint32_t* status)
+{
+    const int32_t i0   = 2 * (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
+    const int32_t n    = count_of(k);
+    const bool track_f = (k.flags & GPE_MPM_FLAG_FLUID_F) != 0;
+    Scatter a{}, b{};
+    b.node = 0xffffffffu;
+#pragma unroll 1
+    for (int p = 0; p < 2; ++p) {
+        a               = b;
+        b.node          = 0xffffffffu;
+        const int32_t i = i0 + p;
+        if (i < n) {
+            const int m       = mat_of(k, MODE, mat, i);
+            const MpmScene sc = scene_of<MS>(k, sid, i);
+            PState ps;
+            ps.x             = x[i];
+            ps.F             = keeps_f(m, track_f) ? F[i] : make_float4(1.f, 0.f, 0.f, 1.f);
+            ps.J             = keeps_j(m) ? J[i] : 1.f;
+            const Stencil s  = stencil(k, sc, ps.x, status);
+            const float2* nv = vel + (size_t)sc.goff;
+            g2p_finish(k, sc, m, track_f, s,
+                       [&](int32_t nxi, int32_t nyj) {
+                           return __ldg(&nv[(size_t)nyj * (size_t)sc.nx + (size_t)nxi]);
+                       },
+                       ps, status);
+            x[i] = ps.x;
+            if (keeps_f(m, track_f)) { F[i] = ps.F; }
+            if (keeps_j(m)) { J[i] = ps.J; }
+            const float4 Q = affine(k, m, ps.C, (m == MODE_FLUID) ? make_float4(1.f, 0.f, 0.f, 1.f) : ps.F, ps.J);
+            b              = scatter_of(k, sc, stencil(k, sc, ps.x, status), ps.v, Q);
+        }
+    }
+    scatter_pair(k, a, b, grid, status);
 }
 
 // ----- spatial sort of the particles (keeps P2G runs long and G2P gathers local) ---------------------------
@@ -916,6 +1038,36 @@ int32_t launch_g2p(gpe_mpm* s, const float2* vel, cudaStream_t st)
     }
 }
 
+template <int MODE>
+int32_t launch_g2p2g_t(gpe_mpm* s, float4* grid, cudaStream_t st)
+{
+    const int c      = s->cur;
+    const unsigned g = mblocks((lsz(s) + 1) / 2);
+    if (s->scenes.size() > 1) {
+        k_g2p2g<MODE, true><<<g, T_MPM, 0, st>>>(s->k, s->vel_n, s->x[c], s->F[c], s->J[c], s->mat[c], s->sid[c], grid,
+                                                s->status);
+    } else {
+        k_g2p2g<MODE, false><<<g, T_MPM, 0, st>>>(s->k, s->vel_n, s->x[c], s->F[c], s->J[c], s->mat[c], nullptr, grid,
+                                                 s->status);
+    }
+    GPE_CHECK_LAUNCH("k_g2p2g");
+    return GPE_OK;
+}
+
+// G2P from the node velocities s->vel_n and the next step's P2G into grid
+int32_t launch_g2p2g(gpe_mpm* s, float4* grid, cudaStream_t st)
+{
+    s->launches += 1;
+    switch (mode_of(s)) {
+        case MODE_FLUID: return launch_g2p2g_t<MODE_FLUID>(s, grid, st);
+        case MODE_COROT: return launch_g2p2g_t<MODE_COROT>(s, grid, st);
+        case MODE_SNOW: return launch_g2p2g_t<MODE_SNOW>(s, grid, st);
+        case MODE_NEOHOOKEAN: return launch_g2p2g_t<MODE_NEOHOOKEAN>(s, grid, st);
+        case MODE_SAND: return launch_g2p2g_t<MODE_SAND>(s, grid, st);
+        default: return launch_g2p2g_t<MODE_MIXED>(s, grid, st);
+    }
+}
+
 // node velocities of grid into s->vel_n, zeroing grid `zero` (or nothing) in the same pass
 int32_t launch_grid_vel(gpe_mpm* s, const float4* grid, float4* zero, cudaStream_t st)
 {
@@ -962,8 +1114,7 @@ int32_t mpm_run(gpe_mpm* s, int32_t n_steps, bool do_sort, cudaStream_t st)
             // node velocities of this step (zeroing the grid read two steps ago), its G2P, and the P2G of the
             // next step into the zero grid b
             rc = launch_grid_vel(s, s->grid[a], s->grid[z], st);
-            if (rc == GPE_OK) { rc = launch_g2p<1>(s, s->vel_n, st); }
-            if (rc == GPE_OK) { rc = launch_p2g(s, s->grid[b], st); }
+            if (rc == GPE_OK) { rc = launch_g2p2g(s, s->grid[b], st); }
         } else {
             k_clear<<<grid_blocks(s->nn), T_MPM, 0, st>>>(s->grid[z], s->nn);
             GPE_CHECK_LAUNCH("k_clear");
