@@ -1713,9 +1713,9 @@ __global__ void k_pbf_emit(const PbfK k, const HoseK h, float2* __restrict__ x, 
 
 // ----- publish to a chunk-major view (PBFOutputKernel, PBF.cu:861-896) ------------------------------------
 // The target is `vv`, or the struct at `vp` in device memory when vp is set (read when the kernel runs).
-__global__ void k_view_zero(const gpe_view* __restrict__ vp)
+__global__ void k_view_zero(const gpe_view vv, const gpe_view* __restrict__ vp)
 {
-    const gpe_view view = *vp;
+    const gpe_view view = vp ? *vp : vv;
     const int32_t nc    = view.chunks_x * view.chunks_y;
     for (int32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
         view.counts[c] = 0;
@@ -1748,13 +1748,20 @@ __global__ void __launch_bounds__(T_PART)
     __syncthreads();
     const float inv = 1.f / view.chunk_dim;
     int32_t c[PUB_PER_THREAD], slot[PUB_PER_THREAD], rank[PUB_PER_THREAD];
-    float2 p[PUB_PER_THREAD];
+    // (positions and velocities are loaded together, ahead of everything that waits for them: 10.8 us for 1M particles
+    // with the velocities loaded where they are written, 9.0 so)
+    float2 p[PUB_PER_THREAD], w[PUB_PER_THREAD];
+#pragma unroll
+    for (int32_t j = 0; j < PUB_PER_THREAD; ++j) {
+        const int32_t i = i0 + j * T_PART;
+        p[j]            = i < n ? x[i] : make_float2(0.f, 0.f);
+        w[j]            = i < n ? v[i] : make_float2(0.f, 0.f);
+    }
 #pragma unroll
     for (int32_t j = 0; j < PUB_PER_THREAD; ++j) {
         const int32_t i = i0 + j * T_PART;
         c[j]            = -1;
         if (i < n) {
-            p[j]             = x[i];
             const int32_t cx = min(max((int32_t)floorf((p[j].x - k.d0.ox) * inv), 0), view.chunks_x - 1);
             const int32_t cy = min(max((int32_t)floorf((p[j].y - k.d0.oy) * inv), 0), view.chunks_y - 1);
             c[j]             = cx + cy * view.chunks_x;
@@ -1804,7 +1811,7 @@ __global__ void __launch_bounds__(T_PART)
         if (sl >= view.chunk_capacity) { continue; }
         const size_t o                         = (size_t)c[j] * (size_t)view.chunk_capacity + (size_t)sl;
         reinterpret_cast<float2*>(view.pos)[o] = p[j];
-        reinterpret_cast<float2*>(view.vel)[o] = v[i0 + j * T_PART];
+        reinterpret_cast<float2*>(view.vel)[o] = w[j];
     }
 }
 
@@ -3350,12 +3357,12 @@ extern "C" int32_t gpe_pbf_publish(gpe_pbf* s, const gpe_view* view, int32_t vie
     gpe_view vv{};
     if (view_mem == GPE_MEM_HOST) {
         vv = *view;
-        GPE_TRY_CUDA(cudaMemsetAsync(vv.counts, 0, sizeof(int32_t) * (size_t)vv.chunks_x * vv.chunks_y, st));
     } else {
         vp = view;
-        k_view_zero<<<(unsigned)sm_count(), T_PART, 0, st>>>(vp);
-        GPE_CHECK_LAUNCH("k_view_zero");
     }
+    const int64_t chunks = vp ? INT32_MAX : (int64_t)vv.chunks_x * vv.chunks_y;
+    k_view_zero<<<(unsigned)std::min<int64_t>((chunks + T_PART - 1) / T_PART, sm_count()), T_PART, 0, st>>>(vv, vp);
+    GPE_CHECK_LAUNCH("k_view_zero");
     if (lsize(s) > 0) {
         k_pbf_publish<<<(unsigned)((lsize(s) + PUB_PER_BLOCK - 1) / PUB_PER_BLOCK), T_PART, 0, st>>>(
             s->k, vv, vp, s->pos, s->vel, s->status);
