@@ -833,7 +833,7 @@ struct DeltaPass {
         t.r             = offset(me.px, me.pd, ql.q);
         const float r2  = fmaf(t.r.x, t.r.x, t.r.y * t.r.y);
         t.hit           = (r2 <= k.h2) && (r2 > 1e-12f) && valid;
-        const float inv = rsqrt_normal(t.hit ? r2 : 1.f);
+        const float inv = rsqrt_normal(r2); // (what is not hit is dropped below)
         float l         = fmaf(ql.a, k.mass, me.a);
         if (SCORR) {
             const float qq    = k.h2 - r2;
@@ -1231,7 +1231,7 @@ struct VorticityPass {
         t.r              = offset(me.px, me.pd, qw.q);
         const float r2   = fmaf(t.r.x, t.r.x, t.r.y * t.r.y);
         t.hit            = (r2 <= k.h2) && (r2 > 1e-12f) && valid;
-        const float inv  = rsqrt_normal(t.hit ? r2 : 1.f);
+        const float inv  = rsqrt_normal(r2);
         const float diff = fmaf(-r2, inv, k.h);
         t.w              = t.hit ? (fabsf(qw.a) - me.a) * (diff * diff * inv) : 0.f; // grad_i W = -cs (...)
         return t;

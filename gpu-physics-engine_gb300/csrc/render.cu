@@ -107,9 +107,10 @@ constexpr int32_t SH_TW = 32 * SH_PX, SH_TH = SH_ROWS * SH_THREADS / 32;
 // row's gradient value, :224-242) at min(k, 15).
 // VEC: rows of counts and of the image start on 16-byte boundaries and the width is a multiple of 4, so a row's counts
 // are three 16-byte loads and four pixels one store. Bound by memory: 32 MB at 2048 x 2048. A 32 x 64 tile of counts in
-// shared memory, one column of 8 pixels a thread (60 shared loads and 8 four-byte stores): 13.8 us; this 7.
+// shared memory, one column of 8 pixels a thread (60 shared loads and 8 four-byte stores): 13.8 us; this 9.2 (10.3 without the bound of 8
+// blocks an SM, whose 1,024 blocks then take two waves).
 template <bool VEC>
-__global__ void __launch_bounds__(SH_THREADS)
+__global__ void __launch_bounds__(SH_THREADS, 8)
     k_shade(uint8_t* __restrict__ rgba, int64_t pitch, const int32_t* __restrict__ centres, int32_t width,
             int32_t height, int32_t line_every)
 {
