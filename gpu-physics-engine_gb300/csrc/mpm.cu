@@ -10,12 +10,12 @@
 //                    velocities from that array (L1/L2 hits: sorted neighbours share nodes), is updated, and the warp
 //                    scatters its 64 particles to the next grid (scatter_pair), lanes that share a stencil base node
 //                    summing their contributions first. Its bound is instruction issue (72%, 4 blocks of 256 an SM at
-//                    64 registers): 4M mixed particles 125 us a step where k_p2g and k_g2p took 103 and 64.
+//                    64 registers): 4M mixed particles 116 us a step where k_p2g and k_g2p took 103 and 64.
 //   k_p2g, k_g2p     the halves of the first and the last step.
 // (Measured alternatives, each slower: a G2P that staged its block's node box in shared memory and updated
 // each node there, 0.198 against 0.186 ms per step at 4M particles; the fused kernel with both particles side by side
 // and velocity and affine matrix written as in k_g2p, 0.159 against 0.153 ms for the separate kernels; at 5 and 6 blocks
-// an SM it spills, 135 and 144 us against 131.)
+// an SM it spills, 126 us and more.)
 // Stage kernels (k_clear, k_p2g, k_grid, k_g2p on an updated grid) reproduce the reference's four kernels
 // one to one for stage-level parity tests.
 #include <cuda_runtime.h>
@@ -84,13 +84,13 @@ __device__ __forceinline__ MpmScene scene_of(const MpmK& k, const int32_t* __res
 }
 
 // the scene that owns node idx (the last whose first node is not past idx)
-__device__ __forceinline__ MpmScene scene_of_node(const MpmK& k, int64_t idx)
+__device__ __forceinline__ MpmScene scene_of_node(const MpmK& k, uint32_t idx)
 {
     if (k.n_scenes <= 1) { return k.s0; }
     int32_t lo = 0, hi = k.n_scenes - 1;
     while (lo < hi) {
         const int32_t mid = (lo + hi + 1) >> 1;
-        if ((int64_t)k.scenes[mid].goff <= idx) {
+        if (k.scenes[mid].goff <= idx) {
             lo = mid;
         } else {
             hi = mid - 1;
@@ -380,29 +380,36 @@ __device__ __forceinline__ Scatter scatter_of(const MpmK& k, const MpmScene& sc,
 // the quadratic B-spline weight of node i of a particle f nodes past its base node, MPM.cu:92-110
 __device__ __forceinline__ float weight(float f, int i)
 {
-    return i == 0 ? 0.5f * (1.5f - f) * (1.5f - f)
-                  : (i == 1 ? 0.75f - (f - 1.0f) * (f - 1.0f) : 0.5f * (f - 0.5f) * (f - 0.5f));
+    const float d = f - (1.5f - 0.5f * (float)i);
+    const float q = d * d;
+    return i == 1 ? 0.75f - q : 0.5f * q;
 }
 
-// One particle's terms of the three nodes of its stencil's column i: (m v + Qx dpx) is the column's, so a node costs two
-// multiplies and three fused multiply-adds.
-struct ColumnTerms {
-    float2 mv, Qy;
-    float wx, fy;
-    __device__ __forceinline__ ColumnTerms(const MpmK& k, const Scatter& p, int i) : Qy(p.Qy), fy(p.fy)
+// what the three columns of a particle's stencil share over the rows: weights and m v + Qx dpx
+struct Columns {
+    float wx[3];
+    float2 mv[3];
+    __device__ __forceinline__ Columns(const MpmK& k, const Scatter& p)
     {
-        const float dpx = ((float)i - p.fx) * k.dx;
-        mv              = fma2(p.Qx, make_float2(dpx, dpx), p.mv);
-        wx              = weight(p.fx, i);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float dpx = ((float)i - p.fx) * k.dx;
+            wx[i]           = weight(p.fx, i);
+            mv[i]           = fma2(p.Qx, make_float2(dpx, dpx), p.mv);
+        }
     }
-    // adds node j's momentum to c and its mass to cm; wy is the row's weight
-    __device__ __forceinline__ void add(const MpmK& k, int j, float wy, float2& c, float& cm) const
+};
+// and the nodes of one row: weight, and m v + Q dp per node
+struct RowTerms {
+    float wy;
+    float2 dy;
+    __device__ __forceinline__ RowTerms(const MpmK& k, const Scatter& p, int j)
     {
-        const float w   = wx * wy;
-        const float dpy = ((float)j - fy) * k.dx;
-        c               = fma2(make_float2(w, w), fma2(Qy, make_float2(dpy, dpy), mv), c);
-        cm              = fmaf(w, k.mass, cm);
+        const float dpy = ((float)j - p.fy) * k.dx;
+        wy              = weight(p.fy, j);
+        dy              = mul2(p.Qy, make_float2(dpy, dpy));
     }
+    __device__ __forceinline__ float2 velocity(const Columns& c, int i) const { return add2(c.mv[i], dy); }
 };
 
 // The scatter of a thread's two particles a, b (consecutive in storage), by whole warps. Particles are kept sorted by
@@ -419,8 +426,8 @@ struct ColumnTerms {
 // half as many particles; staging node sums in a shared-memory tile of the block's nodes (float atomics on shared
 // memory, a block barrier, a flush) slower again. status[2] counts the warps that need the fifth round (a run of more
 // than 16 lanes).
-constexpr int CHAIN_RUNS = 12; // (2, 6, 12 and never: 4.67, 4.66, 4.64, 4.67 ms for 32 steps of 4M sorted particles; 276, 274,
-                               // 274, 310 us for 20 steps of 262,147 in lattice order)
+constexpr int CHAIN_RUNS = 12; // (2, 6, 12 and never: 4.67, 4.66, 4.64, 4.67 ms for 32 steps of 4M sorted particles; 276,
+                               // 274, 274, 310 us for 20 steps of 262,147 in lattice order)
 __device__ __forceinline__ void scatter_pair(const MpmK& k, const Scatter& a, const Scatter& b,
                                              float4* __restrict__ grid, uint32_t* status)
 {
@@ -437,94 +444,79 @@ __device__ __forceinline__ void scatter_pair(const MpmK& k, const Scatter& a, co
     const uint32_t run_end = later ? (uint32_t)(__ffs(later) - 1) : 32u; // first lane of the next run
     const uint32_t longest = __reduce_max_sync(ALL, head ? run_end - lane : 0u);
     if (longest > 16u && lane == 0u) { atomicAdd(status + 2, 1u); }
-    float2 c[9]; // column i, row j at 3 i + j
-    float cm[9];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const ColumnTerms ta(k, a, i), tb(k, b, i);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const int q = 3 * i + j;
-            float2 t    = make_float2(0.f, 0.f);
-            float tm    = 0.f;
-            ta.add(k, j, weight(a.fy, j), t, tm);
-            c[q]  = join ? t : make_float2(0.f, 0.f);
-            cm[q] = join ? tm : 0.f;
-            if (ok1) { tb.add(k, j, weight(b.fy, j), c[q], cm[q]); }
-            const float ox = __shfl_down_sync(ALL, give ? t.x : 0.f, 1);
-            const float oy = __shfl_down_sync(ALL, give ? t.y : 0.f, 1);
-            const float om = __shfl_down_sync(ALL, give ? tm : 0.f, 1);
-            if (lane != 31u) {
-                c[q] = add2(c[q], make_float2(ox, oy));
-                cm[q] += om;
-            }
-        }
+    // the run before and after, for handing columns on
+    const bool chain      = __popc(heads) >= CHAIN_RUNS; // (of the whole warp)
+    const uint32_t before = heads & ((1u << lane) - 1u);
+    const int hp          = before ? 31 - __clz(before) : (int)lane; // the run before
+    bool next_to = false, rest = head && ok1;
+    if (chain) {
+        const uint32_t pnode = __shfl_sync(ALL, b.node, hp);
+        next_to              = rest && before != 0u && pnode + 1u == b.node; // (base nodes end three short of a row)
+        const bool followed  = __shfl_sync(ALL, next_to ? 1 : 0, (int)(run_end & 31u)) != 0 && run_end < 32u;
+        rest                 = rest && !followed; // this lane adds its run's second and third column too
     }
-    // (a loop: one copy of the nine nodes' shuffles keeps the kernel in the instruction cache)
+    const Columns ca(k, a), cb(k, b);
+    float4* row_a = grid + (size_t)(solo ? a.node : 0u);
+    float4* row_b = grid + (size_t)(ok1 ? b.node : 0u);
+    // row by row (a loop: one copy of the code keeps the kernel in the instruction cache, and only one row's sums are
+    // live; all nine nodes' at once: 125 against 115 us for k_g2p2g at 4M mixed particles)
 #pragma unroll 1
-    for (uint32_t d = 1u; d < longest; d <<= 1) {
-        const bool take = lane + d < run_end;
+    for (int j = 0; j < 3; ++j) {
+        const RowTerms ta(k, a, j), tb(k, b, j);
+        float2 c[3];
+        float cm[3]; // sums of weights
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const float ox = __shfl_down_sync(ALL, c[q].x, d);
-            const float oy = __shfl_down_sync(ALL, c[q].y, d);
-            const float om = __shfl_down_sync(ALL, cm[q], d);
-            if (take) {
-                c[q] = add2(c[q], make_float2(ox, oy));
-                cm[q] += om;
+        for (int i = 0; i < 3; ++i) {
+            const float wa = ca.wx[i] * ta.wy, wb = ok1 ? cb.wx[i] * tb.wy : 0.f;
+            const float2 va = ta.velocity(ca, i);
+            const float wj = join ? wa : 0.f, wg = give ? wa : 0.f;
+            c[i]           = fma2(make_float2(wb, wb), tb.velocity(cb, i), mul2(make_float2(wj, wj), va));
+            cm[i]          = wj + wb;
+            const float ox = __shfl_down_sync(ALL, wg * va.x, 1);
+            const float oy = __shfl_down_sync(ALL, wg * va.y, 1);
+            const float om = __shfl_down_sync(ALL, wg, 1);
+            if (lane != 31u) {
+                c[i] = add2(c[i], make_float2(ox, oy));
+                cm[i] += om;
             }
+            if (solo) { atomicAdd(row_a + i, make_float4(wa * va.x, wa * va.y, wa * k.mass, 0.f)); }
         }
-    }
-    bool rest = head && ok1; // this lane adds its run's second and third column too
-    if (__popc(heads) >= CHAIN_RUNS) {
-        const uint32_t before = heads & ((1u << lane) - 1u);
-        const int hp          = before ? 31 - __clz(before) : (int)lane; // the run before
-        const uint32_t pnode  = __shfl_sync(ALL, b.node, hp);
-        const bool next_to    = rest && before != 0u && pnode + 1u == b.node; // (base nodes end three short of a row)
-        const bool followed   = __shfl_sync(ALL, next_to ? 1 : 0, (int)(run_end & 31u)) != 0 && run_end < 32u;
-        // column 2 of the run before is this run's column 1, the sum of that its column 0
+#pragma unroll 1
+        for (uint32_t d = 1u; d < longest; d <<= 1) {
+            const bool take = lane + d < run_end;
 #pragma unroll
-        for (int i = 1; i >= 0; --i) {
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const int q    = 3 * i + j;
-                const float ox = __shfl_sync(ALL, c[q + 3].x, hp);
-                const float oy = __shfl_sync(ALL, c[q + 3].y, hp);
-                const float om = __shfl_sync(ALL, cm[q + 3], hp);
-                if (next_to) {
-                    c[q] = add2(c[q], make_float2(ox, oy));
-                    cm[q] += om;
+            for (int i = 0; i < 3; ++i) {
+                const float ox = __shfl_down_sync(ALL, c[i].x, d);
+                const float oy = __shfl_down_sync(ALL, c[i].y, d);
+                const float om = __shfl_down_sync(ALL, cm[i], d);
+                if (take) {
+                    c[i] = add2(c[i], make_float2(ox, oy));
+                    cm[i] += om;
                 }
             }
         }
-        rest = rest && !followed;
-    }
-    if (head && ok1) {
-        float4* const base = grid + (size_t)b.node;
+        if (chain) {
+            // column 2 of the run before is this run's column 1, the sum of that its column 0
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            atomicAdd(base + (size_t)q * (size_t)b.nx, make_float4(c[q].x, c[q].y, cm[q], 0.f));
-        }
-        if (rest) {
-#pragma unroll
-            for (int q = 3; q < 9; ++q) {
-                atomicAdd(base + (size_t)(q % 3) * (size_t)b.nx + q / 3, make_float4(c[q].x, c[q].y, cm[q], 0.f));
+            for (int i = 1; i >= 0; --i) {
+                const float ox = __shfl_sync(ALL, c[i + 1].x, hp);
+                const float oy = __shfl_sync(ALL, c[i + 1].y, hp);
+                const float om = __shfl_sync(ALL, cm[i + 1], hp);
+                if (next_to) {
+                    c[i] = add2(c[i], make_float2(ox, oy));
+                    cm[i] += om;
+                }
             }
         }
-    }
-    if (solo) {
-        float4* const base = grid + (size_t)a.node;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const ColumnTerms ta(k, a, i);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                float2 t = make_float2(0.f, 0.f);
-                float tm = 0.f;
-                ta.add(k, j, weight(a.fy, j), t, tm);
-                atomicAdd(base + (size_t)j * (size_t)a.nx + i, make_float4(t.x, t.y, tm, 0.f));
+        if (head && ok1) {
+            atomicAdd(row_b, make_float4(c[0].x, c[0].y, cm[0] * k.mass, 0.f));
+            if (rest) {
+                atomicAdd(row_b + 1, make_float4(c[1].x, c[1].y, cm[1] * k.mass, 0.f));
+                atomicAdd(row_b + 2, make_float4(c[2].x, c[2].y, cm[2] * k.mass, 0.f));
             }
         }
+        row_a += a.nx;
+        row_b += b.nx;
     }
 }
 
@@ -567,13 +559,13 @@ __global__ void __launch_bounds__(T_MPM, 4)
 // gridKernel, MPM.cu:131-177 (in place)
 __global__ void k_grid(const MpmK k, float4* __restrict__ grid)
 {
-    const int64_t nn     = k.nn;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < nn; idx += stride) {
-        float4 g        = grid[idx];
+    const uint32_t nn     = (uint32_t)k.nn; // at most 2^30
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nn; idx += stride) {
+        float4 g             = grid[idx];
         const MpmScene sc    = scene_of_node(k, idx);
-        const int64_t local  = idx - (int64_t)sc.goff;
-        const float2 vv      = node_velocity(k, sc, g, (int32_t)(local % sc.nx), (int32_t)(local / sc.nx));
+        const uint32_t local = idx - sc.goff, row = local / (uint32_t)sc.nx;
+        const float2 vv      = node_velocity(k, sc, g, (int32_t)(local - row * (uint32_t)sc.nx), (int32_t)row);
         g.x             = vv.x;
         g.y             = vv.y;
         grid[idx]       = g;
@@ -582,16 +574,18 @@ __global__ void k_grid(const MpmK k, float4* __restrict__ grid)
 
 // The grid update once per node (gridKernel, MPM.cu:131-177) into node velocities, and the zeroing of the
 // grid read two steps earlier (zero may be null).
+// Node indices are 32-bit (the engine holds at most 2^30): with 64-bit remainders and quotients the pass took 8.5 us
+// for 1024^2 nodes.
 template <bool MS>
 __global__ void k_grid_vel(const MpmK k, const float4* __restrict__ grid, float2* __restrict__ vel,
-                           float4* __restrict__ zero, int64_t nn)
+                           float4* __restrict__ zero, uint32_t nn)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < nn; idx += stride) {
-        const float4 g      = grid[idx];
-        const MpmScene sc   = MS ? scene_of_node(k, idx) : k.s0;
-        const int64_t local = idx - (int64_t)sc.goff;
-        vel[idx]            = node_velocity(k, sc, g, (int32_t)(local % sc.nx), (int32_t)(local / sc.nx));
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nn; idx += stride) {
+        const float4 g       = grid[idx];
+        const MpmScene sc    = MS ? scene_of_node(k, idx) : k.s0;
+        const uint32_t local = idx - sc.goff, row = local / (uint32_t)sc.nx;
+        vel[idx]             = node_velocity(k, sc, g, (int32_t)(local - row * (uint32_t)sc.nx), (int32_t)row);
         if (zero) { zero[idx] = make_float4(0.f, 0.f, 0.f, 0.f); }
     }
 }
@@ -1072,9 +1066,9 @@ int32_t launch_g2p2g(gpe_mpm* s, float4* grid, cudaStream_t st)
 int32_t launch_grid_vel(gpe_mpm* s, const float4* grid, float4* zero, cudaStream_t st)
 {
     if (s->scenes.size() > 1) {
-        k_grid_vel<true><<<grid_blocks(s->nn), T_MPM, 0, st>>>(s->k, grid, s->vel_n, zero, s->nn);
+        k_grid_vel<true><<<grid_blocks(s->nn), T_MPM, 0, st>>>(s->k, grid, s->vel_n, zero, (uint32_t)s->nn);
     } else {
-        k_grid_vel<false><<<grid_blocks(s->nn), T_MPM, 0, st>>>(s->k, grid, s->vel_n, zero, s->nn);
+        k_grid_vel<false><<<grid_blocks(s->nn), T_MPM, 0, st>>>(s->k, grid, s->vel_n, zero, (uint32_t)s->nn);
     }
     GPE_CHECK_LAUNCH("k_grid_vel");
     s->launches += 1;
