@@ -59,6 +59,16 @@ bool kernel_can_use(const void* p, size_t align)
     return a.device == dev && (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged);
 }
 
+Place behind(cudaStream_t st)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return {st, false};
+    }
+    return {st, c == cudaStreamCaptureStatusNone};
+}
+
 int32_t sm_count()
 {
     int dev = 0, n = 0;

@@ -647,7 +647,7 @@ int32_t shuffle_order(gpe_mlp* m, uint32_t n, uint64_t rs, cudaStream_t st)
     const unsigned g = (n + 255u) / 256u;
     k_shuffle_draw<<<g, 256, 0, st>>>(rs, n, m->sh_target, m->sh_rank, m->sh_count);
     GPE_CHECK_LAUNCH("k_shuffle_draw");
-    const int32_t rc = launch_exclusive_scan(m->sh_count, n, m->sh_bsum, m->sh_start, st);
+    const int32_t rc = launch_exclusive_scan(m->sh_count, n, m->sh_bsum, m->sh_start, {st, false});
     if (rc) { return rc; }
     k_shuffle_place<<<g, 256, 0, st>>>(n, m->sh_target, m->sh_rank, m->sh_start, m->sh_swaps);
     GPE_CHECK_LAUNCH("k_shuffle_place");

@@ -537,6 +537,7 @@ __global__ void __launch_bounds__(T_MPM, 4)
           const float4* __restrict__ F, const float* __restrict__ J, const int32_t* __restrict__ mat,
           const int32_t* __restrict__ sid, float4* __restrict__ grid, uint32_t* status)
 {
+    follow();
     const int32_t i0 = 2 * (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     const int32_t n  = count_of(k);
     auto load = [&](int32_t i) {
@@ -580,6 +581,7 @@ template <bool MS>
 __global__ void k_grid_vel(const MpmK k, const float4* __restrict__ grid, float2* __restrict__ vel,
                            float4* __restrict__ zero, uint32_t nn)
 {
+    follow();
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nn; idx += stride) {
         const float4 g       = grid[idx];
@@ -599,6 +601,7 @@ __global__ void __launch_bounds__(T_MPM, 6)
           float4* __restrict__ C, float4* __restrict__ F, float* __restrict__ J, const int32_t* __restrict__ mat,
           const int32_t* __restrict__ sid, uint32_t* status)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count_of(k)) { return; }
     const int m        = mat_of(k, MODE, mat, i);
@@ -632,6 +635,7 @@ __global__ void __launch_bounds__(T_MPM, 4)
             float* __restrict__ J, const int32_t* __restrict__ mat, const int32_t* __restrict__ sid,
             float4* __restrict__ grid, uint32_t* status)
 {
+    follow();
     const int32_t i0   = 2 * (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     const int32_t n    = count_of(k);
     const bool track_f = (k.flags & GPE_MPM_FLAG_FLUID_F) != 0;
@@ -671,6 +675,7 @@ __global__ void __launch_bounds__(T_MPM)
     k_mpm_key(const MpmK k, const float2* __restrict__ x, const int32_t* __restrict__ sid, uint2* __restrict__ keyrank,
               uint32_t* __restrict__ count, uint32_t* status)
 {
+    follow();
     const int32_t i    = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid   = i < count_of(k);
     const int32_t lane = threadIdx.x & 31;
@@ -703,6 +708,7 @@ __global__ void __launch_bounds__(T_MPM)
                 int32_t* __restrict__ m1, uint32_t* __restrict__ id1, const int32_t* __restrict__ sid0,
                 int32_t* __restrict__ sid1)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int32_t n = __ldg(n_dev);
     if (i >= n) { return; }
@@ -880,6 +886,7 @@ struct gpe_mpm {
     int ga  = 0;        // grid holding the current step's nodes; ga+1, ga+2 (mod 3) are zero between steps
     bool grids_dirty = false;
     bool have_state  = false;
+    Sequence seq;                // the launches of the graph that gpe_mpm_step captures
     int64_t steps_since_sort = 0;
     int32_t launches = 0;
     std::map<std::tuple<int, int, int, int>, MpmGraph> graphs;
@@ -975,15 +982,11 @@ unsigned grid_blocks(int64_t nn)
 template <int MODE>
 int32_t launch_p2g_t(gpe_mpm* s, float4* grid, cudaStream_t st)
 {
-    const int c = s->cur;
-    if (s->scenes.size() > 1) {
-        k_p2g<MODE, true><<<mblocks((lsz(s) + 1) / 2), T_MPM, 0, st>>>(s->k, s->x[c], s->v[c], s->C[c], s->F[c], s->J[c],
-                                                            s->mat[c], s->sid[c], grid, s->status);
-    } else {
-        k_p2g<MODE, false><<<mblocks((lsz(s) + 1) / 2), T_MPM, 0, st>>>(s->k, s->x[c], s->v[c], s->C[c], s->F[c], s->J[c],
-                                                             s->mat[c], nullptr, grid, s->status);
-    }
-    GPE_CHECK_LAUNCH("k_p2g");
+    const int c   = s->cur;
+    const bool ms = s->scenes.size() > 1;
+    GPE_TRY_CUDA(launch(s->seq.at(st), mblocks((lsz(s) + 1) / 2), T_MPM, ms ? k_p2g<MODE, true> : k_p2g<MODE, false>,
+                        s->k, s->x[c], s->v[c], s->C[c], s->F[c], s->J[c], s->mat[c], ms ? s->sid[c] : nullptr, grid,
+                        s->status));
     return GPE_OK;
 }
 
@@ -1005,15 +1008,11 @@ int32_t launch_p2g(gpe_mpm* s, float4* grid, cudaStream_t st)
 template <int MODE, int VS>
 int32_t launch_g2p_t(gpe_mpm* s, const float2* vel, cudaStream_t st)
 {
-    const int c = s->cur;
-    if (s->scenes.size() > 1) {
-        k_g2p<MODE, VS, true><<<mblocks(lsz(s)), T_MPM, 0, st>>>(s->k, vel, s->x[c], s->v[c], s->C[c], s->F[c],
-                                                                s->J[c], s->mat[c], s->sid[c], s->status);
-    } else {
-        k_g2p<MODE, VS, false><<<mblocks(lsz(s)), T_MPM, 0, st>>>(s->k, vel, s->x[c], s->v[c], s->C[c], s->F[c],
-                                                                 s->J[c], s->mat[c], nullptr, s->status);
-    }
-    GPE_CHECK_LAUNCH("k_g2p");
+    const int c   = s->cur;
+    const bool ms = s->scenes.size() > 1;
+    GPE_TRY_CUDA(launch(s->seq.at(st), mblocks(lsz(s)), T_MPM, ms ? k_g2p<MODE, VS, true> : k_g2p<MODE, VS, false>, s->k,
+                        vel, s->x[c], s->v[c], s->C[c], s->F[c], s->J[c], s->mat[c], ms ? s->sid[c] : nullptr,
+                        s->status));
     return GPE_OK;
 }
 
@@ -1035,16 +1034,11 @@ int32_t launch_g2p(gpe_mpm* s, const float2* vel, cudaStream_t st)
 template <int MODE>
 int32_t launch_g2p2g_t(gpe_mpm* s, float4* grid, cudaStream_t st)
 {
-    const int c      = s->cur;
-    const unsigned g = mblocks((lsz(s) + 1) / 2);
-    if (s->scenes.size() > 1) {
-        k_g2p2g<MODE, true><<<g, T_MPM, 0, st>>>(s->k, s->vel_n, s->x[c], s->F[c], s->J[c], s->mat[c], s->sid[c], grid,
-                                                s->status);
-    } else {
-        k_g2p2g<MODE, false><<<g, T_MPM, 0, st>>>(s->k, s->vel_n, s->x[c], s->F[c], s->J[c], s->mat[c], nullptr, grid,
-                                                 s->status);
-    }
-    GPE_CHECK_LAUNCH("k_g2p2g");
+    const int c   = s->cur;
+    const bool ms = s->scenes.size() > 1;
+    GPE_TRY_CUDA(launch(s->seq.at(st), mblocks((lsz(s) + 1) / 2), T_MPM, ms ? k_g2p2g<MODE, true> : k_g2p2g<MODE, false>,
+                        s->k, s->vel_n, s->x[c], s->F[c], s->J[c], s->mat[c], ms ? s->sid[c] : nullptr, grid,
+                        s->status));
     return GPE_OK;
 }
 
@@ -1065,12 +1059,9 @@ int32_t launch_g2p2g(gpe_mpm* s, float4* grid, cudaStream_t st)
 // node velocities of grid into s->vel_n, zeroing grid `zero` (or nothing) in the same pass
 int32_t launch_grid_vel(gpe_mpm* s, const float4* grid, float4* zero, cudaStream_t st)
 {
-    if (s->scenes.size() > 1) {
-        k_grid_vel<true><<<grid_blocks(s->nn), T_MPM, 0, st>>>(s->k, grid, s->vel_n, zero, (uint32_t)s->nn);
-    } else {
-        k_grid_vel<false><<<grid_blocks(s->nn), T_MPM, 0, st>>>(s->k, grid, s->vel_n, zero, (uint32_t)s->nn);
-    }
-    GPE_CHECK_LAUNCH("k_grid_vel");
+    GPE_TRY_CUDA(launch(s->seq.at(st), grid_blocks(s->nn), T_MPM,
+                        s->scenes.size() > 1 ? k_grid_vel<true> : k_grid_vel<false>, s->k, grid, s->vel_n, zero,
+                        (uint32_t)s->nn));
     s->launches += 1;
     return GPE_OK;
 }
@@ -1079,15 +1070,13 @@ int32_t mpm_sort(gpe_mpm* s, cudaStream_t st)
 {
     if (lsz(s) <= 1) { return GPE_OK; }
     const int c = s->cur, o = c ^ 1;
-    k_mpm_key<<<mblocks(lsz(s)), T_MPM, 0, st>>>(s->k, s->x[c], s->sid[c], s->keyrank, s->count, s->status);
-    GPE_CHECK_LAUNCH("k_mpm_key");
-    int32_t rc = launch_exclusive_scan(s->count, (uint32_t)s->nn, s->bsum, s->start, st);
+    GPE_TRY_CUDA(launch(s->seq.at(st), mblocks(lsz(s)), T_MPM, k_mpm_key, s->k, s->x[c], s->sid[c], s->keyrank, s->count,
+                        s->status));
+    int32_t rc = launch_exclusive_scan(s->count, (uint32_t)s->nn, s->bsum, s->start, s->seq.at(st));
     if (rc) { return rc; }
-    k_mpm_place<<<mblocks(lsz(s)), T_MPM, 0, st>>>(s->d_count, (uint32_t)s->nn, s->keyrank, s->start, s->x[c],
-                                                  s->v[c], s->C[c], s->F[c], s->J[c], s->mat[c], s->id[c], s->x[o],
-                                                  s->v[o], s->C[o], s->F[o], s->J[o], s->mat[o], s->id[o],
-                                                  s->sid[c], s->sid[o]);
-    GPE_CHECK_LAUNCH("k_mpm_place");
+    GPE_TRY_CUDA(launch(s->seq.at(st), mblocks(lsz(s)), T_MPM, k_mpm_place, s->d_count, (uint32_t)s->nn, s->keyrank,
+                        s->start, s->x[c], s->v[c], s->C[c], s->F[c], s->J[c], s->mat[c], s->id[c], s->x[o], s->v[o],
+                        s->C[o], s->F[o], s->J[o], s->mat[o], s->id[o], s->sid[c], s->sid[o]));
     s->cur ^= 1;
     s->launches += 2 + scan_launches((uint32_t)s->nn); // key, scan, placement
     return GPE_OK;
@@ -1490,7 +1479,9 @@ int32_t gpe_mpm_step(gpe_mpm* s, int32_t n_steps, void* stream)
         const int ga0 = s->ga, cur0 = s->cur;
         GPE_TRY_CUDA(cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
         s->launches = 0;
+        s->seq.begin();
         int32_t rc  = mpm_run(s, n_steps, do_sort, cap_st);
+        s->seq.end();
         cudaGraph_t graph    = nullptr;
         const cudaError_t ce = cudaStreamEndCapture(cap_st, &graph);
         MpmGraph g;

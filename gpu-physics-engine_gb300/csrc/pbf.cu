@@ -612,6 +612,7 @@ __global__ void __launch_bounds__(T_PART)
                    const float2* __restrict__ x, const float2* __restrict__ v, uint2* __restrict__ keyrank,
                    uint32_t* __restrict__ count)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     predict_hist_one<MULTI>(k, doms, dom, x, v, keyrank, count, i, i < count_of(k));
 }
@@ -672,6 +673,7 @@ __global__ void __launch_bounds__(T_PART)
             const uint32_t* __restrict__ id_in, uint32_t* __restrict__ id_out, const float* __restrict__ acc_in,
             float* __restrict__ prev_out, float* __restrict__ lam_out)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count_of(k)) { return; }
     place_one(k, keyrank, start, bucket, x_in, v_in, xd_out, x_out, xs_out, perm, key_out, id_in, id_out, acc_in,
@@ -803,6 +805,7 @@ __global__ void __launch_bounds__(T_MAX, LIST == LIST_OFF ? 1 : (SELFG || LIST =
              const uint32_t* __restrict__ start, const float4* __restrict__ xd, float* __restrict__ lam,
              const uint32_t* __restrict__ pair_id, float* __restrict__ acc)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count_of(k)) {
         lambda_one<MULTI, SELFG, ACC, false, LIST>(k, doms, dom, start, xd, lam, pair_id, acc, i);
@@ -887,6 +890,7 @@ __global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : (LIST == LIST_FE
               const uint32_t* __restrict__ start, const float4* __restrict__ xd, const float* __restrict__ lam,
               float4* __restrict__ xd_out, float* __restrict__ acc)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count_of(k)) {
         delta_p_one<MULTI, SCORR, ACCINIT, false, LIST>(k, doms, dom, start, xd, lam, xd_out, acc, i);
@@ -988,6 +992,7 @@ __global__ void __launch_bounds__(T_PART)
                   const uint32_t* __restrict__ start, const float4* __restrict__ xd, const float* __restrict__ prev,
                   const uint32_t* __restrict__ pair_id, const MlpDev* __restrict__ mlp, uint16_t* __restrict__ feat)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count_of(k)) { return; }
     const DomDev d       = load_dom<MULTI>(k, doms, dom, i);
@@ -1014,6 +1019,7 @@ __global__ void __launch_bounds__(MLP_TILE)
                 const MlpDev* __restrict__ mlp, uint32_t* __restrict__ status)
 {
     __shared__ MlpFwdSmem S;
+    follow();
     const int32_t n      = count_of(k);
     const int32_t ntiles = (n + MLP_TILE - 1) / MLP_TILE;
     if ((int32_t)blockIdx.x >= ntiles) { return; } // uniform over the CTA, before any barrier
@@ -1062,6 +1068,7 @@ __global__ void __launch_bounds__(T_PART)
                      const float* __restrict__ prev, float* __restrict__ lam, const uint32_t* __restrict__ pair_id,
                      const CollectK col)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count_of(k)) { return; }
     const DomDev d       = load_dom<MULTI>(k, doms, dom, i);
@@ -1195,6 +1202,7 @@ __global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : (LIST == LIST_FE
            const uint32_t* __restrict__ start, const float4* __restrict__ xd, float2* __restrict__ x_out,
            float2* __restrict__ v_out, float* __restrict__ omega, uint32_t* __restrict__ status)
 {
+    follow();
     const int32_t i  = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < count_of(k);
     if (!k.hist_cnt) { // uniform
@@ -1275,6 +1283,7 @@ __global__ void __launch_bounds__(T_MAX, LIST == LIST_USE ? 3 : (LIST == LIST_FE
                 const uint32_t* __restrict__ start, const float4* __restrict__ xd,
                 const float* __restrict__ omega, float2* __restrict__ v)
 {
+    follow();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count_of(k)) { vorticity_one<MULTI, false, LIST>(k, doms, dom, start, xd, omega, v, i); }
 }
@@ -1736,6 +1745,7 @@ __global__ void __launch_bounds__(T_PART)
     k_pbf_publish(const PbfK k, const gpe_view vv, const gpe_view* __restrict__ vp, const float2* __restrict__ x,
                   const float2* __restrict__ v, uint32_t* __restrict__ status)
 {
+    follow();
     __shared__ int32_t key[PUB_SLOTS], cnt[PUB_SLOTS], base[PUB_SLOTS];
     const gpe_view view = vp ? *vp : vv;
     const int32_t n     = count_of(k);
@@ -1992,6 +2002,7 @@ struct gpe_pbf {
     bool wide         = false;    // ... of 32-bit slots
     uint8_t* mflag    = nullptr;  // per cell: a particle of its 3 x 3 cells moved too far for the lists
     bool lists_valid  = false;    // the lists were made in this step
+    Sequence seq;                 // the launches of the graph that gpe_pbf_step captures
     bool hist_ready   = false;    // the last step's XSPH left the next step's cell keys and histogram
     int64_t dirty_cells = 0;      // ... and was dropped: so many of the histogram's cells must be cleared before a sort
 
@@ -2184,6 +2195,7 @@ int32_t clear_hist(gpe_pbf* s, cudaStream_t st)
     if (s->dirty_cells > 0) {
         GPE_TRY_CUDA(cudaMemsetAsync(s->count, 0, sizeof(uint32_t) * (size_t)s->dirty_cells, st));
         s->dirty_cells = 0;
+        s->seq.cut();
     }
     return GPE_OK;
 }
@@ -2201,29 +2213,22 @@ int32_t stage_predict_sort(gpe_pbf* s, cudaStream_t st)
     const int32_t rch = clear_hist(s, st);
     if (rch) { return rch; }
     if (n > 0 && !fused) {
-        if (multi(s)) {
-            k_predict_hist<true><<<blocks_for(n), T_PART, 0, st>>>(s->k, s->d_doms, s->dom, s->pos, s->vel,
-                                                                   s->keyrank, s->count);
-        } else {
-            k_predict_hist<false><<<blocks_for(n), T_PART, 0, st>>>(s->k, s->d_doms, s->dom, s->pos, s->vel,
-                                                                    s->keyrank, s->count);
-        }
-        GPE_CHECK_LAUNCH("k_predict_hist");
+        GPE_TRY_CUDA(launch(s->seq.at(st), blocks_for(n), T_PART, multi(s) ? k_predict_hist<true> : k_predict_hist<false>,
+                            s->k, s->d_doms, s->dom, s->pos, s->vel, s->keyrank, s->count));
     }
     // the scan also clears the candidate lists' cell marks for this step
-    int32_t rc = launch_exclusive_scan(s->count, s->ncells, s->bsum, s->start, st, lists_on(s) ? s->mflag : nullptr);
+    int32_t rc = launch_exclusive_scan(s->count, s->ncells, s->bsum, s->start, s->seq.at(st),
+                                       lists_on(s) ? s->mflag : nullptr);
     if (rc) { return rc; }
-    rc = launch_scatter(s->keyrank, n, s->start, s->bucket, (uint32_t)s->ncells, st, s->d_count);
+    rc = launch_scatter(s->keyrank, n, s->start, s->bucket, (uint32_t)s->ncells, s->seq.at(st), s->d_count);
     if (rc) { return rc; }
     if (n > 0) {
         const bool ids = (s->prm.flags & (GPE_PBF_TRACK_IDS | GPE_PBF_PAIR_IDS)) != 0;
-        k_place<<<blocks_for(n), T_PART, 0, st>>>(s->k, s->keyrank, s->start, s->bucket, s->pos, s->vel,
-                                                  s->xd[s->XS], nullptr, nullptr, s->perm, s->keys,
-                                                  ids ? s->ids[s->id_cur] : nullptr,
-                                                  ids ? s->ids[s->id_cur ^ 1] : nullptr,
-                                                  accumulating(s) ? s->acc : nullptr, s->prev,
-                                                  (s->warm == GPE_WARM_PREV && !s->collecting) ? s->lam : nullptr);
-        GPE_CHECK_LAUNCH("k_place");
+        GPE_TRY_CUDA(launch(s->seq.at(st), blocks_for(n), T_PART, k_place, s->k, s->keyrank, s->start, s->bucket, s->pos,
+                            s->vel, s->xd[s->XS], nullptr, nullptr, s->perm, s->keys,
+                            ids ? s->ids[s->id_cur] : nullptr, ids ? s->ids[s->id_cur ^ 1] : nullptr,
+                            accumulating(s) ? s->acc : nullptr, s->prev,
+                            (s->warm == GPE_WARM_PREV && !s->collecting) ? s->lam : nullptr));
         if (ids) { s->id_cur ^= 1; }
     }
     s->have_sort = true;
@@ -2232,27 +2237,22 @@ int32_t stage_predict_sort(gpe_pbf* s, cudaStream_t st)
 }
 
 // Template dispatch tables: [multi scene][flag][accumulation mode]
-using LamFn = cudaError_t (*)(unsigned, unsigned, cudaStream_t, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
+using LamFn = cudaError_t (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
                        const float4*, float*, const uint32_t*, float*, int);
 template <bool M, bool S, int A>
-cudaError_t lam_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
+cudaError_t lam_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
                 const uint32_t* start, const float4* xs, float* lam, const uint32_t* pid, float* acc, int list)
 {
     if constexpr (A == ACC_PROJ) { // the projected-increment ablation keeps full scans
-        k_lambda<M, S, A, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_lambda<M, S, A, LIST_OFF>, k, doms, dom, start, xs, lam, pid, acc);
     } else if (list == LIST_BUILD) {
-        k_lambda<M, S, A, LIST_BUILD><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_lambda<M, S, A, LIST_BUILD>, k, doms, dom, start, xs, lam, pid, acc);
     } else if (list == LIST_USE) {
-        k_lambda<M, S, A, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_lambda<M, S, A, LIST_USE>, k, doms, dom, start, xs, lam, pid, acc);
     } else if (list == LIST_FEW) {
-        k_lambda<M, S, A, LIST_FEW><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_lambda<M, S, A, LIST_FEW>, k, doms, dom, start, xs, lam, pid, acc);
     } else {
-        k_lambda<M, S, A, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, pid, acc);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_lambda<M, S, A, LIST_OFF>, k, doms, dom, start, xs, lam, pid, acc);
     }
 }
 #define GPE_LAM3(M, S) {lam_launch<M, S, ACC_NONE>, lam_launch<M, S, ACC_SUM>, lam_launch<M, S, ACC_PROJ>}
@@ -2260,21 +2260,18 @@ const LamFn kLam[2][2][3] = {{GPE_LAM3(false, false), GPE_LAM3(false, true)},
                              {GPE_LAM3(true, false), GPE_LAM3(true, true)}};
 #undef GPE_LAM3
 
-using DpFn = cudaError_t (*)(unsigned, unsigned, cudaStream_t, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
+using DpFn = cudaError_t (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
                       const float4*, const float*, float4*, float*, int);
 template <bool M, bool S, bool A>
-cudaError_t dp_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
+cudaError_t dp_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
                const uint32_t* start, const float4* xs, const float* lam, float4* out, float* acc, int list)
 {
     if (list == LIST_USE) {
-        k_delta_p<M, S, A, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_delta_p<M, S, A, LIST_USE>, k, doms, dom, start, xs, lam, out, acc);
     } else if (list == LIST_FEW) {
-        k_delta_p<M, S, A, LIST_FEW><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_delta_p<M, S, A, LIST_FEW>, k, doms, dom, start, xs, lam, out, acc);
     } else {
-        k_delta_p<M, S, A, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xs, lam, out, acc);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_delta_p<M, S, A, LIST_OFF>, k, doms, dom, start, xs, lam, out, acc);
     }
 }
 const DpFn kDp[2][2][2] = {{{dp_launch<false, false, false>, dp_launch<false, false, true>},
@@ -2282,50 +2279,47 @@ const DpFn kDp[2][2][2] = {{{dp_launch<false, false, false>, dp_launch<false, fa
                            {{dp_launch<true, false, false>, dp_launch<true, false, true>},
                             {dp_launch<true, true, false>, dp_launch<true, true, true>}}};
 
-using FeatFn = void (*)(unsigned, unsigned, cudaStream_t, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
+using FeatFn = void (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
                         const float4*, const float*, const uint32_t*, const MlpDev*, uint16_t*, int);
 template <bool M, bool S>
-void feat_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
+void feat_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
                  const uint32_t* start, const float4* xd, const float* prev, const uint32_t* pid, const MlpDev* mlp,
                  uint16_t* feat, int list)
 {
     if (list == LIST_BUILD) {
-        k_lambda_feat<M, S, LIST_BUILD><<<g, blk, 0, st>>>(k, doms, dom, start, xd, prev, pid, mlp, feat);
+        launch(at, g, blk, k_lambda_feat<M, S, LIST_BUILD>, k, doms, dom, start, xd, prev, pid, mlp, feat);
     } else {
-        k_lambda_feat<M, S, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xd, prev, pid, mlp, feat);
+        launch(at, g, blk, k_lambda_feat<M, S, LIST_OFF>, k, doms, dom, start, xd, prev, pid, mlp, feat);
     }
 }
 const FeatFn kFeat[2][2] = {{feat_launch<false, false>, feat_launch<false, true>},
                             {feat_launch<true, false>, feat_launch<true, true>}};
 
-using ColFn = void (*)(unsigned, unsigned, cudaStream_t, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
+using ColFn = void (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
                        const float4*, const float*, float*, const uint32_t*, const CollectK&);
 template <bool M, bool S>
-void col_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
+void col_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
                 const uint32_t* start, const float4* xd, const float* prev, float* lam, const uint32_t* pid,
                 const CollectK& col)
 {
-    k_lambda_collect<M, S><<<g, blk, 0, st>>>(k, doms, dom, start, xd, prev, lam, pid, col);
+    launch(at, g, blk, k_lambda_collect<M, S>, k, doms, dom, start, xd, prev, lam, pid, col);
 }
 const ColFn kCol[2][2] = {{col_launch<false, false>, col_launch<false, true>},
                           {col_launch<true, false>, col_launch<true, true>}};
 
-using XsFn = cudaError_t (*)(unsigned, unsigned, cudaStream_t, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
+using XsFn = cudaError_t (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
                       const float4*, float2*, float2*, float*, uint32_t*, int);
 template <bool M, bool V>
-cudaError_t xs_launch(unsigned g, unsigned blk, cudaStream_t st, const PbfK& k, const DomDev* doms, const int32_t* dom,
+cudaError_t xs_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
                const uint32_t* start, const float4* xd, float2* x_out, float2* v, float* om, uint32_t* status,
                int list)
 {
     if (list == LIST_USE) {
-        k_xsph<M, V, LIST_USE><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_xsph<M, V, LIST_USE>, k, doms, dom, start, xd, x_out, v, om, status);
     } else if (list == LIST_FEW) {
-        k_xsph<M, V, LIST_FEW><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_xsph<M, V, LIST_FEW>, k, doms, dom, start, xd, x_out, v, om, status);
     } else {
-        k_xsph<M, V, LIST_OFF><<<g, blk, 0, st>>>(k, doms, dom, start, xd, x_out, v, om, status);
-        return cudaGetLastError();
+        return launch(at, g, blk, k_xsph<M, V, LIST_OFF>, k, doms, dom, start, xd, x_out, v, om, status);
     }
 }
 const XsFn kXs[2][2] = {{xs_launch<false, false>, xs_launch<false, true>},
@@ -2351,7 +2345,7 @@ int32_t stage_lambda(gpe_pbf* s, cudaStream_t st, int acc)
         // make scans full, never skip a candidate)
         list = s->lists_valid ? list_mode(s) : LIST_BUILD;
     }
-    GPE_TRY_CUDA(kLam[multi(s) ? 1 : 0][sg][acc](nblk(s), (unsigned)s->block, st, s->k, s->d_doms, s->dom, s->start,
+    GPE_TRY_CUDA(kLam[multi(s) ? 1 : 0][sg][acc](nblk(s), (unsigned)s->block, s->seq.at(st), s->k, s->d_doms, s->dom, s->start,
                                                  s->xd[s->XS], s->lam, pid, s->acc, list));
     if (list == LIST_BUILD) {
         s->lists_valid = true;
@@ -2374,7 +2368,7 @@ int32_t stage_lambda_warm(gpe_pbf* s, cudaStream_t st)
         const gpe::MlpDev* md = gpe::mlp_device(s->mlp);
         // the feature pass scans every neighbour on the sorted positions: it makes the step's lists
         const int list = lists_on(s) ? LIST_BUILD : LIST_OFF;
-        kFeat[mi][sg](nblk(s), (unsigned)s->block, st, s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev, pid,
+        kFeat[mi][sg](nblk(s), (unsigned)s->block, s->seq.at(st), s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev, pid,
                       md, s->feat, list);
         GPE_CHECK_LAUNCH("k_lambda_feat");
         if (list == LIST_BUILD) {
@@ -2382,11 +2376,10 @@ int32_t stage_lambda_warm(gpe_pbf* s, cudaStream_t st)
         }
         const int64_t tiles = (lsize(s) + MLP_TILE - 1) / MLP_TILE;
         const unsigned g    = (unsigned)std::min<int64_t>(tiles, s->lam_grid);
-        k_mlp_apply<<<g, MLP_TILE, 0, st>>>(s->k, s->feat, s->prev, s->lam, md, s->status);
-        GPE_CHECK_LAUNCH("k_mlp_apply");
+        GPE_TRY_CUDA(launch(s->seq.at(st), g, MLP_TILE, k_mlp_apply, s->k, s->feat, s->prev, s->lam, md, s->status));
         s->launches += 1;
     } else {
-        kCol[mi][sg](nblk(s), (unsigned)s->block, st, s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev,
+        kCol[mi][sg](nblk(s), (unsigned)s->block, s->seq.at(st), s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev,
                      s->lam, pid, s->col);
         GPE_CHECK_LAUNCH("k_lambda_collect");
     }
@@ -2399,7 +2392,7 @@ int32_t stage_delta_p(gpe_pbf* s, cudaStream_t st, bool accinit)
     if (lsize(s) > 0) {
         const int sc = s->prm.scorr_k != 0.f ? 1 : 0;
         const int list = s->lists_valid ? list_mode(s) : LIST_OFF;
-        GPE_TRY_CUDA(kDp[multi(s) ? 1 : 0][sc][accinit ? 1 : 0](nblk(s), (unsigned)s->block, st, s->k, s->d_doms,
+        GPE_TRY_CUDA(kDp[multi(s) ? 1 : 0][sc][accinit ? 1 : 0](nblk(s), (unsigned)s->block, s->seq.at(st), s->k, s->d_doms,
                                                                 s->dom, s->start, s->xd[s->XS], s->lam,
                                                                 s->xd[s->XO], s->acc, list));
         s->launches += 1;
@@ -2420,7 +2413,7 @@ int32_t stage_xsph(gpe_pbf* s, cudaStream_t st, bool next_hist = false)
         kk.hist_kr  = s->keyrank;
         kk.hist_cnt = s->count; // zeroed by this step's scan
     }
-    GPE_TRY_CUDA(kXs[multi(s) ? 1 : 0][vort](nblk(s), (unsigned)s->block, st, kk, s->d_doms, s->dom, s->start,
+    GPE_TRY_CUDA(kXs[multi(s) ? 1 : 0][vort](nblk(s), (unsigned)s->block, s->seq.at(st), kk, s->d_doms, s->dom, s->start,
                                              s->xd[s->XS], s->pos, s->vel, s->omega, s->status,
                                              s->lists_valid ? list_mode(s) : LIST_OFF));
     s->launches += 1;
@@ -2437,8 +2430,8 @@ int32_t stage_vorticity(gpe_pbf* s, cudaStream_t st)
                                                   : (list == LIST_USE ? k_vorticity<true, LIST_USE> : k_vorticity<true, LIST_FEW>))
                               : (list == LIST_OFF ? k_vorticity<false, LIST_OFF>
                                                   : (list == LIST_USE ? k_vorticity<false, LIST_USE> : k_vorticity<false, LIST_FEW>));
-    fn<<<nblk(s), (unsigned)s->block, 0, st>>>(s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->omega, s->vel);
-    GPE_CHECK_LAUNCH("k_vorticity");
+    GPE_TRY_CUDA(launch(s->seq.at(st), nblk(s), (unsigned)s->block, fn, s->k, s->d_doms, s->dom, s->start, s->xd[s->XS],
+                        s->omega, s->vel));
     s->launches += 1;
     return GPE_OK;
 }
@@ -2581,7 +2574,7 @@ int32_t stage_step_persistent(gpe_pbf* s, cudaStream_t st)
         s->launches += 1;
     } else {
         // no particle: the cell starts are all zero (as the separate scan leaves them)
-        int32_t rc = launch_exclusive_scan(s->count, s->ncells, s->bsum, s->start, st);
+        int32_t rc = launch_exclusive_scan(s->count, s->ncells, s->bsum, s->start, {st, false});
         if (rc) { return rc; }
         s->launches += scan_launches(s->ncells);
     }
@@ -2995,7 +2988,9 @@ int32_t gpe_pbf_step(gpe_pbf* s, int32_t n_steps, void* stream)
         GPE_TRY_CUDA(cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
         s->launches = 0;
         int32_t rc  = GPE_OK;
+        s->seq.begin();
         for (int32_t k = 0; k < n_steps && rc == GPE_OK; ++k) { rc = run_step(s, cap_st, true); }
+        s->seq.end();
         cudaGraph_t graph = nullptr;
         const cudaError_t ce = cudaStreamEndCapture(cap_st, &graph);
         PbfGraph pg;
@@ -3364,9 +3359,8 @@ extern "C" int32_t gpe_pbf_publish(gpe_pbf* s, const gpe_view* view, int32_t vie
     k_view_zero<<<(unsigned)std::min<int64_t>((chunks + T_PART - 1) / T_PART, sm_count()), T_PART, 0, st>>>(vv, vp);
     GPE_CHECK_LAUNCH("k_view_zero");
     if (lsize(s) > 0) {
-        k_pbf_publish<<<(unsigned)((lsize(s) + PUB_PER_BLOCK - 1) / PUB_PER_BLOCK), T_PART, 0, st>>>(
-            s->k, vv, vp, s->pos, s->vel, s->status);
-        GPE_CHECK_LAUNCH("k_pbf_publish");
+        GPE_TRY_CUDA(launch(behind(st), (unsigned)((lsize(s) + PUB_PER_BLOCK - 1) / PUB_PER_BLOCK), T_PART, k_pbf_publish,
+                            s->k, vv, vp, s->pos, s->vel, s->status));
     }
     return GPE_OK;
 }
@@ -3877,10 +3871,10 @@ extern "C" int32_t gpe_pbf_predict_sort_noalloc(const gpe_pbf_params* params, co
                                                                 count);
         GPE_CHECK_LAUNCH("k_predict_hist (noalloc)");
     }
-    rc = launch_exclusive_scan(count, (uint32_t)cells, bsum, cell_start, st);
+    rc = launch_exclusive_scan(count, (uint32_t)cells, bsum, cell_start, {st, false});
     if (rc) { return rc; }
     if (n > 0) {
-        rc = launch_scatter(keyrank, n, cell_start, bucket, (uint32_t)cells, st);
+        rc = launch_scatter(keyrank, n, cell_start, bucket, (uint32_t)cells, {st, false});
         if (rc) { return rc; }
         k_place<<<blocks_for(n), T_PART, 0, st>>>(k, keyrank, cell_start, bucket,
                                                   reinterpret_cast<const float2*>(pos),

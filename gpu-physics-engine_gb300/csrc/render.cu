@@ -64,6 +64,7 @@ __device__ __forceinline__ void build_blend_row(int32_t row)
 __global__ void k_splat_point(const gpe_view* __restrict__ vp, gpe_view vv, int32_t* __restrict__ centres,
                               int32_t width, int32_t height, float scale)
 {
+    follow();
     if (blockIdx.x == 0 && blockIdx.y == 0) {
         for (int32_t row = threadIdx.x; row < BLEND_ROWS; row += blockDim.x) { build_blend_row(row); }
     }
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(SH_THREADS, 8)
     k_shade(uint8_t* __restrict__ rgba, int64_t pitch, const int32_t* __restrict__ centres, int32_t width,
             int32_t height, int32_t line_every)
 {
+    follow();
     const uint32_t across = ((uint32_t)width + SH_TW - 1u) / SH_TW; // blocks a row of tiles
     const int64_t x64     = (int64_t)(blockIdx.x % across) * SH_TW + (threadIdx.x & 31u) * SH_PX;
     const int64_t y64     = (int64_t)(blockIdx.x / across) * SH_TH + (threadIdx.x >> 5) * SH_ROWS;
@@ -214,15 +216,13 @@ extern "C" int32_t gpe_render_frame(const gpe_raster* r, const gpe_view* view, i
     {
         // about 32 blocks of 256 per SM: one particle a thread for a million particles
         const int32_t cols = max(1, (int32_t)std::min<int64_t>((32 * sm_count() + rows - 1) / rows, 65535));
-        k_splat_point<<<dim3((unsigned)cols, (unsigned)rows), 256, 0, st>>>(vp, vv, r->coverage, r->width, r->height,
-                                                                           r->scale);
-        GPE_CHECK_LAUNCH("k_splat_point");
+        GPE_TRY_CUDA(launch(behind(st), dim3((unsigned)cols, (unsigned)rows), 256, k_splat_point, vp, vv, r->coverage,
+                            r->width, r->height, r->scale));
     }
     const bool vec = r->width % 4 == 0 && reinterpret_cast<uintptr_t>(r->coverage) % 16 == 0 &&
                      reinterpret_cast<uintptr_t>(r->rgba) % 16 == 0 && r->pitch % 16 == 0;
     const unsigned grid = (unsigned)(((int64_t)r->width + SH_TW - 1) / SH_TW * (((int64_t)r->height + SH_TH - 1) / SH_TH));
-    (vec ? k_shade<true> : k_shade<false>)<<<grid, SH_THREADS, 0, st>>>(r->rgba, r->pitch, r->coverage, r->width,
-                                                                       r->height, line_every);
-    GPE_CHECK_LAUNCH("k_shade");
+    GPE_TRY_CUDA(launch(behind(st), grid, SH_THREADS, vec ? k_shade<true> : k_shade<false>, r->rgba, r->pitch,
+                        r->coverage, r->width, r->height, line_every));
     return GPE_OK;
 }

@@ -54,6 +54,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(SCAN_T) k_scan_reduce(const uint32_t* __restrict__ count, uint32_t M,
                                                         uint32_t* __restrict__ bsum)
 {
+    follow();
     const uint32_t base = blockIdx.x * SCAN_TILE;
     uint32_t s          = 0;
     if constexpr (VEC) {
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_reduce(const uint32_t* __restri
 // one block: in-place exclusive scan of the block sums
 __global__ void __launch_bounds__(SCAN_T) k_scan_bsum(uint32_t* __restrict__ bsum, uint32_t nb)
 {
+    follow();
     uint32_t carry = 0;
     for (uint32_t base = 0; base < nb; base += SCAN_T) {
         const uint32_t idx = base + threadIdx.x;
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_down(uint32_t* __restrict__ cou
                                                       uint32_t* __restrict__ start, uint8_t* __restrict__ zero8)
 {
     __shared__ __align__(16) uint32_t s_tile[SCAN_TILE];
+    follow();
     const uint32_t base = blockIdx.x * SCAN_TILE;
     uint32_t prefix;
     if (SUMS) {
@@ -192,6 +195,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_down(uint32_t* __restrict__ cou
 __global__ void k_scatter(const uint2* __restrict__ keyrank, int64_t n_host, const int32_t* __restrict__ n_dev,
                           const uint32_t* __restrict__ start, uint32_t* __restrict__ bucket, uint32_t ncells)
 {
+    follow();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t n = n_dev ? (int64_t)__ldg(n_dev) : n_host;
     if (i >= n) { return; }
@@ -205,36 +209,30 @@ __global__ void k_scatter(const uint2* __restrict__ keyrank, int64_t n_host, con
 
 size_t scan_blocks(uint32_t n_keys) { return (n_keys + SCAN_TILE - 1) / SCAN_TILE; }
 
-int32_t launch_exclusive_scan(uint32_t* count, uint32_t n_keys, uint32_t* bsum, uint32_t* start,
-                              cudaStream_t st, uint8_t* zero_bytes)
+int32_t launch_exclusive_scan(uint32_t* count, uint32_t n_keys, uint32_t* bsum, uint32_t* start, Place at,
+                              uint8_t* zero_bytes)
 {
     const uint32_t nb = (uint32_t)scan_blocks(n_keys);
     if (nb == 0) { return GPE_ERR_BAD_ARG; }
     const bool vec = n_keys % 4 == 0 && reinterpret_cast<uintptr_t>(count) % 16 == 0 &&
                      reinterpret_cast<uintptr_t>(start) % 16 == 0 && reinterpret_cast<uintptr_t>(zero_bytes) % 4 == 0;
-    (vec ? k_scan_reduce<true> : k_scan_reduce<false>)<<<nb, SCAN_T, 0, st>>>(count, n_keys, bsum);
-    GPE_CHECK_LAUNCH("k_scan_reduce");
+    GPE_TRY_CUDA(launch(at, nb, SCAN_T, vec ? k_scan_reduce<true> : k_scan_reduce<false>, count, n_keys, bsum));
     const bool sums = nb <= FUSED_MAX_TILES;
-    if (!sums) {
-        k_scan_bsum<<<1, SCAN_T, 0, st>>>(bsum, nb);
-        GPE_CHECK_LAUNCH("k_scan_bsum");
-    }
+    if (!sums) { GPE_TRY_CUDA(launch(at, 1, SCAN_T, k_scan_bsum, bsum, nb)); }
     auto down = sums ? (vec ? k_scan_down<true, true> : k_scan_down<true, false>)
                      : (vec ? k_scan_down<false, true> : k_scan_down<false, false>);
-    down<<<nb, SCAN_T, 0, st>>>(count, n_keys, bsum, start, zero_bytes);
-    GPE_CHECK_LAUNCH("k_scan_down");
+    GPE_TRY_CUDA(launch(at, nb, SCAN_T, down, count, n_keys, bsum, start, zero_bytes));
     return GPE_OK;
 }
 
 int32_t scan_launches(uint32_t n_keys) { return scan_blocks(n_keys) <= FUSED_MAX_TILES ? 2 : 3; }
 
 int32_t launch_scatter(const uint2* keyrank, int64_t n, const uint32_t* start, uint32_t* bucket, uint32_t ncells,
-                       cudaStream_t st, const int32_t* n_dev)
+                       Place at, const int32_t* n_dev)
 {
     if (n <= 0) { return GPE_OK; }
     const int T = 256;
-    k_scatter<<<(unsigned)((n + T - 1) / T), T, 0, st>>>(keyrank, n, n_dev, start, bucket, ncells);
-    GPE_CHECK_LAUNCH("k_scatter");
+    GPE_TRY_CUDA(launch(at, (unsigned)((n + T - 1) / T), T, k_scatter, keyrank, n, n_dev, start, bucket, ncells));
     return GPE_OK;
 }
 
