@@ -120,7 +120,7 @@ size_t scan_blocks(uint32_t n_keys);
 // needs scan_blocks(n_keys) entries.
 int32_t launch_exclusive_scan(uint32_t* count, uint32_t n_keys, uint32_t* bsum, uint32_t* start,
                               Place at, uint8_t* zero_bytes = nullptr);
-// kernel launches of launch_exclusive_scan for n_keys buckets (2, or 3 beyond 2048 tiles)
+// kernel launches of launch_exclusive_scan for n_keys buckets (2, or 3 beyond 4096 tiles)
 int32_t scan_launches(uint32_t n_keys);
 // bucket[start[key] + rank] = i for every (key, rank) pair. n sizes the launch; with n_dev the kernel takes
 // the live count from the device (which must not exceed n).

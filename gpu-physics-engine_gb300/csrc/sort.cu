@@ -6,7 +6,7 @@
 // (PBF.cu:806-833). Chunks here are not bounded by shared memory (a scene holds up to millions of
 // particles and cells), so the histogram and the scan run device-wide: the histogram is fused into the
 // predict kernel (pbf.cu), the scan below is a reduce / down-sweep over tiles of 2048 cells (with a
-// scan-of-block-sums launch in between for more than 2048 tiles), and the stable placement is finished by
+// scan-of-block-sums launch in between for more than 4096 tiles), and the stable placement is finished by
 // pbf.cu's gather kernel.
 #include "gpe_internal.h"
 
@@ -49,29 +49,57 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total)
     return before + inc - v;
 }
 
-// VEC: M is a multiple of 4 and count is 16-byte aligned (four cells per load)
-template <bool VEC>
+// How a thread moves its four cells: one by one (arrays of a caller that are not 16-byte aligned), 16 bytes at a time with
+// a last group that may not be whole, or 16 bytes at a time throughout (the cell count is a multiple of four: without
+// the ragged group's code a step of 16,384 atoms is 0.16 us shorter).
+enum { CELLS_SINGLE, CELLS_RAGGED, CELLS_WHOLE };
+
+template <int VEC>
+__device__ __forceinline__ bool whole4(uint32_t idx, uint32_t M)
+{
+    return VEC == CELLS_WHOLE ? idx < M : (VEC == CELLS_RAGGED && idx < M && M - idx >= 4u);
+}
+
+// four cells from idx on; zero past M
+template <int VEC>
+__device__ __forceinline__ uint4 load4(const uint32_t* __restrict__ a, uint32_t idx, uint32_t M)
+{
+    uint4 c = make_uint4(0u, 0u, 0u, 0u);
+    if (whole4<VEC>(idx, M)) {
+        c = *reinterpret_cast<const uint4*>(a + idx);
+    } else if (VEC != CELLS_WHOLE) {
+        if (idx < M) { c.x = a[idx]; }
+        if (idx + 1u < M) { c.y = a[idx + 1u]; }
+        if (idx + 2u < M) { c.z = a[idx + 2u]; }
+        if (idx + 3u < M) { c.w = a[idx + 3u]; }
+    }
+    return c;
+}
+
+template <int VEC>
+__device__ __forceinline__ void store4(uint32_t* __restrict__ a, uint32_t idx, uint32_t M, const uint4 c)
+{
+    if (whole4<VEC>(idx, M)) {
+        *reinterpret_cast<uint4*>(a + idx) = c;
+    } else if (VEC != CELLS_WHOLE) {
+        if (idx < M) { a[idx] = c.x; }
+        if (idx + 1u < M) { a[idx + 1u] = c.y; }
+        if (idx + 2u < M) { a[idx + 2u] = c.z; }
+        if (idx + 3u < M) { a[idx + 3u] = c.w; }
+    }
+}
+
+template <int VEC>
 __global__ void __launch_bounds__(SCAN_T) k_scan_reduce(const uint32_t* __restrict__ count, uint32_t M,
                                                         uint32_t* __restrict__ bsum)
 {
     follow();
     const uint32_t base = blockIdx.x * SCAN_TILE;
     uint32_t s          = 0;
-    if constexpr (VEC) {
 #pragma unroll
-        for (int t = 0; t < SCAN_I / 4; ++t) {
-            const uint32_t idx = base + 4u * (t * SCAN_T + threadIdx.x);
-            if (idx < M) {
-                const uint4 c = *reinterpret_cast<const uint4*>(count + idx);
-                s += (c.x + c.y) + (c.z + c.w);
-            }
-        }
-    } else {
-#pragma unroll
-        for (int t = 0; t < SCAN_I; ++t) {
-            const uint32_t idx = base + t * SCAN_T + threadIdx.x;
-            if (idx < M) { s += count[idx]; }
-        }
+    for (int t = 0; t < SCAN_I / 4; ++t) {
+        const uint4 c = load4<VEC>(count, base + 4u * (t * SCAN_T + threadIdx.x), M);
+        s += (c.x + c.y) + (c.z + c.w);
     }
     uint32_t total;
     block_excl_scan(s, &total);
@@ -93,15 +121,15 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_bsum(uint32_t* __restrict__ bsu
     }
 }
 
-// SUMS: bsum holds the tiles' totals (not scanned) and each block adds up those before it itself, which
-// saves the single-block scan launch while the tiles are few (FUSED_MAX_TILES); else bsum is already the
-// exclusive scan of the totals.
-constexpr uint32_t FUSED_MAX_TILES = 2048;
+// SUMS: bsum holds the tiles' totals (not scanned) and each block adds up those before it itself, which saves the
+// single-block scan launch while the tiles are few (FUSED_MAX_TILES: 16 sums a thread at most); else bsum is already the
+// exclusive scan of the totals. At 2,081 tiles (256 scenes
+// of 129 x 129 cells) the separate launch cost 6.3 us and the sums cost less than can be told.
+constexpr uint32_t FUSED_MAX_TILES = 4096;
 
-// VEC: M is a multiple of 4 and the arrays are 16-byte aligned (zero8: 4-byte), so each thread moves four
-// cells per access; the per-thread runs of SCAN_I cells are then read from shared memory as 16-byte words
-// (2-way bank conflicts instead of 8-way).
-template <bool SUMS, bool VEC>
+// Bound by the memory traffic: four cells per access (256 scenes of 129 x 129 cells 24 us one by one, 10 so); the
+// per-thread runs of SCAN_I cells are read from shared memory as 16-byte words (2-way bank conflicts instead of 8-way).
+template <bool SUMS, int VEC>
 __global__ void __launch_bounds__(SCAN_T) k_scan_down(uint32_t* __restrict__ count, uint32_t M,
                                                       const uint32_t* __restrict__ bsum,
                                                       uint32_t* __restrict__ start, uint8_t* __restrict__ zero8)
@@ -109,6 +137,10 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_down(uint32_t* __restrict__ cou
     __shared__ __align__(16) uint32_t s_tile[SCAN_TILE];
     follow();
     const uint32_t base = blockIdx.x * SCAN_TILE;
+    // coalesced loads, in flight while the tiles before are added up
+    uint4 cell[SCAN_I / 4];
+#pragma unroll
+    for (int t = 0; t < SCAN_I / 4; ++t) { cell[t] = load4<VEC>(count, base + 4u * (t * SCAN_T + threadIdx.x), M); }
     uint32_t prefix;
     if (SUMS) {
         uint32_t part = 0;
@@ -117,33 +149,20 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_down(uint32_t* __restrict__ cou
     } else {
         prefix = bsum[blockIdx.x];
     }
-    // coalesced load, and zero the histogram for the next sort
-    if constexpr (VEC) {
+    // zero the histogram for the next sort
 #pragma unroll
-        for (int t = 0; t < SCAN_I / 4; ++t) {
-            const uint32_t li  = 4u * (t * SCAN_T + threadIdx.x);
-            const uint32_t idx = base + li;
-            uint4 c            = make_uint4(0u, 0u, 0u, 0u);
-            if (idx < M) {
-                c                                        = *reinterpret_cast<const uint4*>(count + idx);
-                *reinterpret_cast<uint4*>(count + idx)   = make_uint4(0u, 0u, 0u, 0u);
-                if (zero8) { *reinterpret_cast<uint32_t*>(zero8 + idx) = 0u; }
+    for (int t = 0; t < SCAN_I / 4; ++t) {
+        const uint32_t li  = 4u * (t * SCAN_T + threadIdx.x);
+        const uint32_t idx = base + li;
+        store4<VEC>(count, idx, M, make_uint4(0u, 0u, 0u, 0u));
+        if (zero8) {
+            if (whole4<VEC>(idx, M)) {
+                *reinterpret_cast<uint32_t*>(zero8 + idx) = 0u;
+            } else if (VEC != CELLS_WHOLE) {
+                for (uint32_t e = idx; e < idx + 4u && e < M; ++e) { zero8[e] = 0u; }
             }
-            *reinterpret_cast<uint4*>(s_tile + li) = c;
         }
-    } else {
-#pragma unroll
-        for (int t = 0; t < SCAN_I; ++t) {
-            const uint32_t li  = t * SCAN_T + threadIdx.x;
-            const uint32_t idx = base + li;
-            uint32_t c         = 0;
-            if (idx < M) {
-                c          = count[idx];
-                count[idx] = 0u;
-                if (zero8) { zero8[idx] = 0u; }
-            }
-            s_tile[li] = c;
-        }
+        *reinterpret_cast<uint4*>(s_tile + li) = cell[t];
     }
     __syncthreads();
     // each thread owns SCAN_I consecutive cells
@@ -172,20 +191,10 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_down(uint32_t* __restrict__ cou
             make_uint4(off + v[4 * q], off + v[4 * q + 1], off + v[4 * q + 2], off + v[4 * q + 3]);
     }
     __syncthreads();
-    if constexpr (VEC) {
 #pragma unroll
-        for (int t = 0; t < SCAN_I / 4; ++t) {
-            const uint32_t li  = 4u * (t * SCAN_T + threadIdx.x);
-            const uint32_t idx = base + li;
-            if (idx < M) { *reinterpret_cast<uint4*>(start + idx) = *reinterpret_cast<const uint4*>(s_tile + li); }
-        }
-    } else {
-#pragma unroll
-        for (int t = 0; t < SCAN_I; ++t) {
-            const uint32_t li  = t * SCAN_T + threadIdx.x;
-            const uint32_t idx = base + li;
-            if (idx < M) { start[idx] = s_tile[li]; }
-        }
+    for (int t = 0; t < SCAN_I / 4; ++t) {
+        const uint32_t li = 4u * (t * SCAN_T + threadIdx.x);
+        store4<VEC>(start, base + li, M, *reinterpret_cast<const uint4*>(s_tile + li));
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) { start[M] = prefix + total; }
 }
@@ -214,13 +223,21 @@ int32_t launch_exclusive_scan(uint32_t* count, uint32_t n_keys, uint32_t* bsum, 
 {
     const uint32_t nb = (uint32_t)scan_blocks(n_keys);
     if (nb == 0) { return GPE_ERR_BAD_ARG; }
-    const bool vec = n_keys % 4 == 0 && reinterpret_cast<uintptr_t>(count) % 16 == 0 &&
-                     reinterpret_cast<uintptr_t>(start) % 16 == 0 && reinterpret_cast<uintptr_t>(zero_bytes) % 4 == 0;
-    GPE_TRY_CUDA(launch(at, nb, SCAN_T, vec ? k_scan_reduce<true> : k_scan_reduce<false>, count, n_keys, bsum));
+    const bool aligned = reinterpret_cast<uintptr_t>(count) % 16 == 0 && reinterpret_cast<uintptr_t>(start) % 16 == 0 &&
+                         reinterpret_cast<uintptr_t>(zero_bytes) % 4 == 0;
+    const int vec   = !aligned ? CELLS_SINGLE : (n_keys % 4 == 0 ? CELLS_WHOLE : CELLS_RAGGED);
     const bool sums = nb <= FUSED_MAX_TILES;
+    auto reduce     = k_scan_reduce<CELLS_SINGLE>;
+    auto down       = sums ? k_scan_down<true, CELLS_SINGLE> : k_scan_down<false, CELLS_SINGLE>;
+    if (vec == CELLS_RAGGED) {
+        reduce = k_scan_reduce<CELLS_RAGGED>;
+        down   = sums ? k_scan_down<true, CELLS_RAGGED> : k_scan_down<false, CELLS_RAGGED>;
+    } else if (vec == CELLS_WHOLE) {
+        reduce = k_scan_reduce<CELLS_WHOLE>;
+        down   = sums ? k_scan_down<true, CELLS_WHOLE> : k_scan_down<false, CELLS_WHOLE>;
+    }
+    GPE_TRY_CUDA(launch(at, nb, SCAN_T, reduce, count, n_keys, bsum));
     if (!sums) { GPE_TRY_CUDA(launch(at, 1, SCAN_T, k_scan_bsum, bsum, nb)); }
-    auto down = sums ? (vec ? k_scan_down<true, true> : k_scan_down<true, false>)
-                     : (vec ? k_scan_down<false, true> : k_scan_down<false, false>);
     GPE_TRY_CUDA(launch(at, nb, SCAN_T, down, count, n_keys, bsum, start, zero_bytes));
     return GPE_OK;
 }
