@@ -116,12 +116,13 @@ bool kernel_can_use(const void* p, size_t align);
 // ----- counting sort of 32-bit keys (shared by PBF and the MPM spatial sort) -----
 // Workspace sizes for a sort of up to n_max items into n_keys buckets.
 size_t scan_blocks(uint32_t n_keys);
+constexpr int SCAN_TILE = 2048; // cells of one tile of the scan
 // count[n_keys] -> start[n_keys+1] exclusive scan; zeroes count (and zero_bytes[n_keys] when given). bsum
-// needs scan_blocks(n_keys) entries.
+// needs scan_blocks(n_keys) entries; with have_sums it holds the tiles' totals on entry.
 int32_t launch_exclusive_scan(uint32_t* count, uint32_t n_keys, uint32_t* bsum, uint32_t* start,
-                              Place at, uint8_t* zero_bytes = nullptr);
-// kernel launches of launch_exclusive_scan for n_keys buckets (2, or 3 beyond 4096 tiles)
-int32_t scan_launches(uint32_t n_keys);
+                              Place at, uint8_t* zero_bytes = nullptr, bool have_sums = false);
+// kernel launches of launch_exclusive_scan for n_keys buckets
+int32_t scan_launches(uint32_t n_keys, bool have_sums = false);
 // bucket[start[key] + rank] = i for every (key, rank) pair. n sizes the launch; with n_dev the kernel takes
 // the live count from the device (which must not exceed n).
 int32_t launch_scatter(const uint2* keyrank, int64_t n, const uint32_t* start, uint32_t* bucket, uint32_t ncells,

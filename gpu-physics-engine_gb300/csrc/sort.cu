@@ -16,7 +16,7 @@ namespace {
 
 constexpr int SCAN_T    = 256;
 constexpr int SCAN_I    = 8;
-constexpr int SCAN_TILE = SCAN_T * SCAN_I;
+static_assert(SCAN_TILE == SCAN_T * SCAN_I, "a thread takes SCAN_I cells");
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
 {
@@ -219,7 +219,7 @@ __global__ void k_scatter(const uint2* __restrict__ keyrank, int64_t n_host, con
 size_t scan_blocks(uint32_t n_keys) { return (n_keys + SCAN_TILE - 1) / SCAN_TILE; }
 
 int32_t launch_exclusive_scan(uint32_t* count, uint32_t n_keys, uint32_t* bsum, uint32_t* start, Place at,
-                              uint8_t* zero_bytes)
+                              uint8_t* zero_bytes, bool have_sums)
 {
     const uint32_t nb = (uint32_t)scan_blocks(n_keys);
     if (nb == 0) { return GPE_ERR_BAD_ARG; }
@@ -236,13 +236,16 @@ int32_t launch_exclusive_scan(uint32_t* count, uint32_t n_keys, uint32_t* bsum, 
         reduce = k_scan_reduce<CELLS_WHOLE>;
         down   = sums ? k_scan_down<true, CELLS_WHOLE> : k_scan_down<false, CELLS_WHOLE>;
     }
-    GPE_TRY_CUDA(launch(at, nb, SCAN_T, reduce, count, n_keys, bsum));
+    if (!have_sums) { GPE_TRY_CUDA(launch(at, nb, SCAN_T, reduce, count, n_keys, bsum)); }
     if (!sums) { GPE_TRY_CUDA(launch(at, 1, SCAN_T, k_scan_bsum, bsum, nb)); }
     GPE_TRY_CUDA(launch(at, nb, SCAN_T, down, count, n_keys, bsum, start, zero_bytes));
     return GPE_OK;
 }
 
-int32_t scan_launches(uint32_t n_keys) { return scan_blocks(n_keys) <= FUSED_MAX_TILES ? 2 : 3; }
+int32_t scan_launches(uint32_t n_keys, bool have_sums)
+{
+    return (have_sums ? 1 : 2) + (scan_blocks(n_keys) <= FUSED_MAX_TILES ? 0 : 1);
+}
 
 int32_t launch_scatter(const uint2* keyrank, int64_t n, const uint32_t* start, uint32_t* bucket, uint32_t ncells,
                        Place at, const int32_t* n_dev)

@@ -16,21 +16,22 @@ def _engine(gpe_mod, option, n=6000):
         p.vort_eps = 0.02
     if option == "ids":
         p.flags |= gpe_mod.PBF_PAIR_IDS | gpe_mod.PBF_SELF_GRAD
-    boxes = [(0.0, 0.0, 1.0, 1.0)]
+    size = 1.0 if n <= 6000 else 4.0
+    boxes = [(0.0, 0.0, size, size)]
     g = np.random.default_rng(n)
-    pos = g.uniform(0.0, 1.0, (n, 2)).astype(np.float32)
+    pos = g.uniform(0.0, size, (n, 2)).astype(np.float32)
     dom = None
     if option == "scenes":
-        boxes = [(0.0, 0.0, 1.0, 1.0), (2.0, 0.0, 1.0, 1.0), (4.0, 0.0, 1.0, 1.0)]
+        boxes = [(2.0 * size * d, 0.0, size, size) for d in range(3)]
         dom = np.sort(np.arange(n) % 3).astype(np.int32)
-        pos[:, 0] += 2.0 * dom
+        pos[:, 0] += np.float32(2.0 * size) * dom
     e = gpe_mod.Pbf(p, boxes, capacity=n)
     e.set_state(pos, g.normal(0, 0.2, (n, 2)).astype(np.float32), domain=dom)
     return e
 
 
 @pytest.mark.parametrize("option", ["plain", "vorticity", "ids", "scenes"])
-@pytest.mark.parametrize("n", [1, 129, 6000])
+@pytest.mark.parametrize("n", [1, 129, 6000, 65536, 65537])  # 65,536: the last whose histogram counts tile sums
 def test_steps_of_one_call_equal_enqueued_steps(gpe_mod, cuda_ok, option, n):
     got = []
     for whole in (True, False):
