@@ -530,7 +530,9 @@ __global__ void k_clear(float4* __restrict__ grid, int64_t nn)
     }
 }
 
-// P2G of particles 2t and 2t + 1 (see scatter_pair)
+// P2G of particles 2t and 2t + 1 (see scatter_pair): both are loaded, then one copy of the constitutive code takes them
+// one after the other. One step of 4M mixed particles, sorted, L2 flushed before: 150 us; with the code twice 158, with
+// each particle loaded in its turn 156. 32 scenes of 5.8M 225, 236 and 240 us. 5 blocks an SM spill: 166.
 template <int MODE, bool MS>
 __global__ void __launch_bounds__(T_MPM, 4)
     k_p2g(const MpmK k, const float2* __restrict__ x, const float2* __restrict__ v, const float4* __restrict__ C,
@@ -540,20 +542,39 @@ __global__ void __launch_bounds__(T_MPM, 4)
     follow();
     const int32_t i0 = 2 * (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     const int32_t n  = count_of(k);
+    struct In {
+        MpmScene sc;
+        int m;
+        float4 F, C;
+        float J;
+        float2 x, v;
+    };
     auto load = [&](int32_t i) {
-        Scatter p{};
-        p.node = 0xffffffffu;
+        In p{};
         if (i < n) {
-            const MpmScene sc = scene_of<MS>(k, sid, i);
-            const int m       = mat_of(k, MODE, mat, i);
-            const float4 Fp   = (m == MODE_FLUID) ? make_float4(1.f, 0.f, 0.f, 1.f) : F[i];
-            const float Jp    = keeps_j(m) ? J[i] : 1.f;
-            const float4 Q    = affine(k, m, C[i], Fp, Jp);
-            p                 = scatter_of(k, sc, stencil(k, sc, x[i], status), v[i], Q);
+            p.sc = scene_of<MS>(k, sid, i);
+            p.m  = mat_of(k, MODE, mat, i);
+            p.F  = (p.m == MODE_FLUID) ? make_float4(1.f, 0.f, 0.f, 1.f) : F[i];
+            p.J  = keeps_j(p.m) ? J[i] : 1.f;
+            p.C  = C[i];
+            p.x  = x[i];
+            p.v  = v[i];
         }
         return p;
     };
-    const Scatter a = load(i0), b = load(i0 + 1);
+    In cur = load(i0), next = load(i0 + 1);
+    Scatter a{}, b{};
+    b.node = 0xffffffffu;
+#pragma unroll 1
+    for (int p = 0; p < 2; ++p) {
+        a      = b;
+        b.node = 0xffffffffu;
+        if (i0 + p < n) {
+            const float4 Q = affine(k, cur.m, cur.C, cur.F, cur.J);
+            b              = scatter_of(k, cur.sc, stencil(k, cur.sc, cur.x, status), cur.v, Q);
+        }
+        cur = next;
+    }
     scatter_pair(k, a, b, grid, status);
 }
 
