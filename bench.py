@@ -50,15 +50,15 @@ ALG_BYTES = {  # algorithmic bytes per particle per launch (FP32 SoA, each field
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the 1M-particle step's neighbour
 # kernels from ncu captures of this workload's first timed step (cold caches: ncu flushes them before each
-# replay). lambda: the mean over a step's four launches, the mask-recording pass (22.1 MB) and three masked
-# passes (39.1 MB each, which also read the 16 MB candidate-mask array and the cell starts that stay in L2
-# in a live step)
-NCU_TRAFFIC = {"lambda": 34.87e6, "delta_p": 43.5e6, "xsph": 39.27e6}
+# replay). lambda: the mean over a step's four launches, the list-recording pass (29.9 MB) and three listed
+# passes (67.7 MB each, which also read the lists' headers and chunks, 48 MB, and the cell starts that stay in
+# L2 in a live step)
+NCU_TRAFFIC = {"lambda": 58.26e6, "delta_p": 72.93e6, "xsph": 69.47e6}
 # warp instructions per launch (smsp__inst_executed.sum) of the same kernels from the same captures; lambda:
-# the mean over a step's four launches (the mask-recording lambda executes 45.8 M, a masked one 20.8 M). The
+# the mean over a step's four launches (the list-recording lambda executes 41.1 M, a listed one 16.1 M). The
 # neighbour kernels are bound by instruction issue, and the issue roofline is these instructions over the
 # live launch time against 4 schedulers x SMs x the sampled SM clock.
-NCU_WARP_INST = {"lambda": 27.05e6, "delta_p": 20.21e6, "xsph": 15.71e6}
+NCU_WARP_INST = {"lambda": 22.37e6, "delta_p": 15.36e6, "xsph": 14.61e6}
 
 # engines whose steps alternate in the end-to-end measurement (measured when every step restarted from the
 # initial state: 1 engine 0.608 ms per step with synchronous copies, 2 engines 0.411, 3 engines 0.386)
@@ -527,7 +527,7 @@ def batched_leg(args, stream, flush_l2):
     """Batched PBF: 256 independent dam-break scenes, particle counts log-uniform in [2048, 65536] (seed 3),
     box aspect U(0.5, 2), C0 physics at dt = 1/480, 4 iterations, all scenes in one engine; timed with the
     default tuning, with the autotuner's choice (cell size, block size, persistent solve) and with the two
-    persistent forms at the chosen cell size, block size and mask skin."""
+    persistent forms at the chosen cell size, block size and list skin."""
     import torch
 
     import gpe
@@ -744,7 +744,7 @@ def run_gpe(args, rank, ws):
     o_vel = torch.empty((n, 2), dtype=torch.float32).pin_memory()
 
     eng.set_state(pos, vel, stream=sh)
-    # the engine's autotuner picks cell size, block size, persistent solve and mask skin for this scene (it
+    # the engine's autotuner picks cell size, block size, persistent solve and list skin for this scene (it
     # restores the state afterwards); untimed. Its trials run consecutive steps without an L2 flush, as a
     # simulation loop does; the timed steps below flush L2 before each step, and under that protocol its
     # choice can trail another candidate by about 1% (skin 0.1 h against 0.075 h at 1M particles).

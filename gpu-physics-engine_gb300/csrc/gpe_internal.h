@@ -82,7 +82,7 @@ Place behind(cudaStream_t st);
 #if defined(__CUDACC__)
 // First statement of every kernel that may be launched so: the rest of it waits until the kernel before it is complete
 // and its writes are visible, so that only the launch overlaps and no pass sees another order. Short passes gain most:
-// one step of 16,384 atoms with its state in and out 51.2 -> 47.1 us, 20 substeps of them 675 -> 616, 20 MLS-MPM steps
+// one step of 16,384 atoms with its state in and out 51.2 -> 47.1 us, 20 substeps of them 675 -> 616, 16 MLS-MPM steps
 // of 65,536 particles 126 -> 115, a published and drawn frame of 1M 40.3 -> 32.9, a step of 1M 307.6 -> 304.4. The
 // kernel before gives no earlier signal than its blocks' ends: with one at its start the waiting blocks took the room of those still to
 // come (1M particles 304 -> 317 us a step, 256 batched scenes 1353 -> 1405).

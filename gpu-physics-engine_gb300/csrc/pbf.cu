@@ -324,7 +324,7 @@ constexpr int TOGETHER_MAX = 4; // lanes for which that is cheaper: about 250 in
 // skin / (2 iterations) on every single pass's move, which a state fresh from outside broke nearly everywhere.
 // One step of 1,048,576 particles from such a state: listed lambda 50 -> 25 us, delta p 41 -> 26 us, XSPH
 // 41 -> 28 us, the step with its state's copies 0.468 -> 0.325 ms; from an evolved state lambda 27 -> 23 us and
-// delta p 27 -> 23 us. 256 batched scenes (5.1M particles) 2.20 -> 1.42 ms.
+// delta p 27 -> 23 us. 256 batched scenes (5.0M particles) 2.20 -> 1.42 ms.
 // LIST_FEW is LIST_USE for launches whose warps are all resident at once at 64 registers a thread (stage launchers,
 // list_mode): there a pass lasts as long as its slowest warp, so its kernels take 64 registers instead of 40 and
 // spare the warp scan_full's chain of loads (scan_together). 16,384 atoms in 20 substeps 0.79 -> 0.70 ms; at 1M
@@ -1654,7 +1654,7 @@ __global__ void __launch_bounds__(T_PART)
     }
 }
 
-// Four entries a thread, a block apart, so that enough loads are in flight (4.3M entries 18.4 -> 7.3 us)
+// Four entries a thread, a block apart, so that enough loads are in flight (5.0M entries 18.4 -> 7.3 us)
 constexpr int CHECK_PER = 4;
 __global__ void __launch_bounds__(T_PART)
     k_check_domains(const int32_t* __restrict__ dom, int32_t n, int32_t nd, uint32_t* status)
@@ -1678,7 +1678,7 @@ __global__ void k_set_count(int32_t* __restrict__ c, int32_t n) { *c = n; }
 // A new state from device arrays in one launch: positions, velocities (zero without vel), scenes (with dom_in), ids,
 // the count, no previous multipliers, and the histogram cleared where one was left (cells > 0). Seven copies, memsets
 // and small kernels cost 10 us of a 16,384-particle step's 71 us and 25 us at 1M particles; this kernel 2.3 and 7.9 us
-// (with one particle a thread 15 at 1M; 4.3M 36 against 51).
+// (with one particle a thread 15 at 1M; 5.0M 36 against 51).
 constexpr int SET_PER = 2; // particles a thread
 __global__ void __launch_bounds__(T_PART)
     k_set_state(int32_t n, const float2* __restrict__ pos, const float2* __restrict__ vel,

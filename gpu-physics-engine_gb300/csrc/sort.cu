@@ -123,11 +123,11 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_bsum(uint32_t* __restrict__ bsu
 
 // SUMS: bsum holds the tiles' totals (not scanned) and each block adds up those before it itself, which saves the
 // single-block scan launch while the tiles are few (FUSED_MAX_TILES: 16 sums a thread at most); else bsum is already the
-// exclusive scan of the totals. At 2,081 tiles (256 scenes
-// of 129 x 129 cells) the separate launch cost 6.3 us and the sums cost less than can be told.
+// exclusive scan of the totals. At some 2,440 tiles (256 scenes
+// of 5.0M cells) the separate launch cost 6.3 us and the sums cost less than can be told.
 constexpr uint32_t FUSED_MAX_TILES = 4096;
 
-// Bound by the memory traffic: four cells per access (256 scenes of 129 x 129 cells 24 us one by one, 10 so); the
+// Bound by the memory traffic: four cells per access (5.0M cells, a count not divisible by four, 24 us one by one, 10 so); the
 // per-thread runs of SCAN_I cells are read from shared memory as 16-byte words (2-way bank conflicts instead of 8-way).
 template <bool SUMS, int VEC>
 __global__ void __launch_bounds__(SCAN_T) k_scan_down(uint32_t* __restrict__ count, uint32_t M,
