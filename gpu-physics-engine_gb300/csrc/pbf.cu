@@ -1251,7 +1251,9 @@ struct VorticityPass {
         const float r2   = fmaf(t.r.x, t.r.x, t.r.y * t.r.y);
         t.hit            = (r2 <= k.h2) && (r2 > 1e-12f) && valid;
         const float inv  = rsqrt_normal(r2);
-        const float diff = fmaf(-r2, inv, k.h);
+        // rounded twice, not fused: where the terms of eta nearly cancel, their last bits decide the direction of a
+        // force of full strength, so this form is part of the result
+        const float diff = __fsub_rn(k.h, __fmul_rn(r2, inv));
         t.w              = t.hit ? (fabsf(qw.a) - me.a) * (diff * diff * inv) : 0.f; // grad_i W = -cs (...)
         return t;
     }
