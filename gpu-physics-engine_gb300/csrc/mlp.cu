@@ -81,7 +81,8 @@ struct __align__(128) MlpTrainSmem {
     float b1[MLP_H], b2[MLP_H], w3[MLP_H], mu[MLP_FP], isd[MLP_FP];
     float y[MLP_TILE];        // outputs
     float tn[MLP_TILE];       // standardised targets
-    float dw3[4][MLP_H];      // by 32 rows
+    float dw3[MLP_H];
+    float dw3q[4][MLP_H];     // a tile's sums over 32 rows each
     float db3, loss, b3, ymu, iysd;
     uint64_t bar;
     uint32_t tmem;
@@ -140,7 +141,9 @@ __device__ __forceinline__ float warp_sum16(float (&v)[16])
 __device__ __forceinline__ void put_param(MlpDev* m, int p, float w);
 
 // All threads of one CTA: every parameter's step. A thread loads all of its parameters' state before it writes any, so
-// that the update costs one memory latency instead of ten.
+// that the update costs one memory latency instead of ten. The fused and unfused forms are explicit: the first steps
+// divide a small gradient by its own size, so a last bit of the moments is worth 1e-4 of some weights after an epoch,
+// and the kernel that this is compiled into must not choose it.
 __device__ __forceinline__ void adamw(const AdamW& ad, float* grad)
 {
     constexpr int PER = (MLP_NW + TRAIN_T - 1) / TRAIN_T;
@@ -160,13 +163,15 @@ __device__ __forceinline__ void adamw(const AdamW& ad, float* grad)
         const int p = q * TRAIN_T + (int)threadIdx.x;
         if (p < MLP_NW) {
             grad[p] = 0.f;
-            mm[q]   = ad.b1 * mm[q] + (1.f - ad.b1) * g[q];
-            vv[q]   = ad.b2 * vv[q] + (1.f - ad.b2) * g[q] * g[q];
+            mm[q]   = fmaf(1.f - ad.b1, g[q], __fmul_rn(ad.b1, mm[q]));
+            vv[q]   = fmaf((1.f - ad.b2) * g[q], g[q], __fmul_rn(ad.b2, vv[q]));
             ad.m[p] = mm[q];
             ad.v[p] = vv[q];
             const bool decay = (p < MLP_OFF_B1) || (p >= MLP_OFF_W2 && p < MLP_OFF_B2) ||
                                (p >= MLP_OFF_W3 && p < MLP_OFF_B3);
-            w[q] -= ad.lr * ((mm[q] / ad.bc1) / (sqrtf(vv[q] / ad.bc2) + ad.eps) + (decay ? ad.wd * w[q] : 0.f));
+            float step = (mm[q] / ad.bc1) / (sqrtf(vv[q] / ad.bc2) + ad.eps);
+            if (decay) { step = __fadd_rn(step, __fmul_rn(ad.wd, w[q])); }
+            w[q] = fmaf(-ad.lr, step, w[q]);
             ad.master[p] = w[q];
             put_param(ad.net, p, w[q]);
         }
@@ -216,7 +221,7 @@ __global__ void __launch_bounds__(TRAIN_T, 1)
             S.b2[t] = m->b2[t];
             S.w3[t] = m->w3[t];
         }
-        if (t < 4 * MLP_H) { (&S.dw3[0][0])[t] = 0.f; }
+        if (t < MLP_H) { S.dw3[t] = 0.f; }
         if (t < MLP_FP) {
             S.mu[t]  = m->mu[t];
             S.isd[t] = m->isd[t];
@@ -336,7 +341,7 @@ __global__ void __launch_bounds__(TRAIN_T, 1)
             *reinterpret_cast<uint4*>(&S.dz[kmajor(r, c0, DZ_N)])      = pack8(d, 0);
             *reinterpret_cast<uint4*>(&S.dz[kmajor(r, c0 + 8u, DZ_N)]) = pack8(d, 1);
             const float sum = warp_sum16(v);
-            if ((t & 1u) == 0u) { S.dw3[quad][c0 + ((t & 31u) >> 1)] += sum; }
+            if ((t & 1u) == 0u) { S.dw3q[quad][c0 + ((t & 31u) >> 1)] = sum; }
         }
         tc::fence_before();
         tc::fence_async_smem();
@@ -349,6 +354,10 @@ __global__ void __launch_bounds__(TRAIN_T, 1)
                         tc::sdesc(tc::saddr(S.w2t) + 256u * k, 128, MLP_H * 16), ID64, k > 0 ? 1u : 0u);
             }
             tc::commit(&S.bar);
+        }
+        if (t >= 64u && t < 64u + MLP_H) { // while the product runs: one sum, 32 rows after 32 rows
+            const uint32_t c = t - 64u;
+            S.dw3[c] = (((S.dw3[c] + S.dw3q[0][c]) + S.dw3q[1][c]) + S.dw3q[2][c]) + S.dw3q[3][c];
         }
         ok = tc::mbar_wait(&S.bar, phase) && ok;
         phase ^= 1u;
@@ -416,7 +425,7 @@ __global__ void __launch_bounds__(TRAIN_T, 1)
     }
     tc::fence_before();
     __syncthreads();
-    if (t < MLP_H) { atomicAdd(&grad[MLP_OFF_W3 + t], (S.dw3[0][t] + S.dw3[1][t]) + (S.dw3[2][t] + S.dw3[3][t])); }
+    if (t < MLP_H) { atomicAdd(&grad[MLP_OFF_W3 + t], S.dw3[t]); }
     if (t == 0) {
         atomicAdd(&grad[MLP_OFF_B3], S.db3);
         atomicAdd(&grad[MLP_NW], S.loss);
