@@ -416,7 +416,8 @@ struct RowTerms {
 // stencil base node (or at least stored in some spatial order), so consecutive lanes mostly share their base node and
 // with it all 9 target nodes. The lanes whose second particle has the same base node form a run. A first particle joins
 // its thread's run, or else the run of the lane before, whose last particle it then is; the few that fit neither add
-// their 9 terms to the grid by themselves. Per node the lanes of a run sum their contributions with a segmented shuffle
+// their 9 terms to the grid by themselves. What a lane does not add is left out by a select or a branch, not by a zero
+// weight: zero times a non-finite velocity would reach particles on other nodes, and in other scenes. Per node the lanes of a run sum their contributions with a segmented shuffle
 // reduction (as many rounds as the warp's longest run needs), and the run's first lane adds the sums to the grid with
 // vector global atomics (red.global.add.v4.f32, resolved in L2). Runs on neighbouring base nodes of a row, which
 // overlap in two of their three columns, first hand those columns on to the next run (CHAIN_RUNS and more runs a warp),
@@ -438,6 +439,8 @@ __device__ __forceinline__ void scatter_pair(const MpmK& k, const Scatter& a, co
     const bool join        = ok1 && a.node == b.node;
     const bool give        = ok0 && !join && lane != 0u && prev == a.node;
     const bool solo        = ok0 && !join && !give;
+    const uint32_t gives   = __ballot_sync(ALL, give);
+    const bool given       = lane != 31u && ((gives >> (lane + 1u)) & 1u) != 0u; // by the lane after
     const bool head        = lane == 0u || prev != b.node;
     const uint32_t heads   = __ballot_sync(ALL, head);
     const uint32_t later   = lane == 31u ? 0u : (heads & (ALL << (lane + 1u)));
@@ -468,18 +471,17 @@ __device__ __forceinline__ void scatter_pair(const MpmK& k, const Scatter& a, co
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             const float wa = ca.wx[i] * ta.wy, wb = ok1 ? cb.wx[i] * tb.wy : 0.f;
-            const float2 va = ta.velocity(ca, i);
-            const float wj = join ? wa : 0.f, wg = give ? wa : 0.f;
-            c[i]           = fma2(make_float2(wb, wb), tb.velocity(cb, i), mul2(make_float2(wj, wj), va));
-            cm[i]          = wj + wb;
-            const float ox = __shfl_down_sync(ALL, wg * va.x, 1);
-            const float oy = __shfl_down_sync(ALL, wg * va.y, 1);
-            const float om = __shfl_down_sync(ALL, wg, 1);
-            if (lane != 31u) {
+            const float2 pa = mul2(make_float2(wa, wa), ta.velocity(ca, i));
+            c[i]            = fma2(make_float2(wb, wb), tb.velocity(cb, i), join ? pa : make_float2(0.f, 0.f));
+            cm[i]           = (join ? wa : 0.f) + wb;
+            const float ox  = __shfl_down_sync(ALL, pa.x, 1);
+            const float oy  = __shfl_down_sync(ALL, pa.y, 1);
+            const float om  = __shfl_down_sync(ALL, wa, 1);
+            if (given) {
                 c[i] = add2(c[i], make_float2(ox, oy));
                 cm[i] += om;
             }
-            if (solo) { atomicAdd(row_a + i, make_float4(wa * va.x, wa * va.y, wa * k.mass, 0.f)); }
+            if (solo) { atomicAdd(row_a + i, make_float4(pa.x, pa.y, wa * k.mass, 0.f)); }
         }
 #pragma unroll 1
         for (uint32_t d = 1u; d < longest; d <<= 1) {
