@@ -59,15 +59,18 @@ bool kernel_can_use(const void* p, size_t align)
     return a.device == dev && (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged);
 }
 
-Place behind(cudaStream_t st)
+// (the legacy default stream gives an error while another stream is being captured: it cannot be used then at all)
+bool capturing(cudaStream_t st)
 {
     cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &c) != cudaSuccess) {
         cudaGetLastError();
-        return {st, false};
+        return true;
     }
-    return {st, c == cudaStreamCaptureStatusNone};
+    return c != cudaStreamCaptureStatusNone;
 }
+
+Place behind(cudaStream_t st) { return {st, !capturing(st)}; }
 
 int32_t sm_count()
 {

@@ -76,6 +76,8 @@ struct Sequence {
     }
 };
 
+// Whether a caller (or the engine itself) is capturing st.
+bool capturing(cudaStream_t st);
 // For a kernel right behind another of the same call on st: full dependencies where a caller is capturing.
 Place behind(cudaStream_t st);
 

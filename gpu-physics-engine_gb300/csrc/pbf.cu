@@ -2053,6 +2053,7 @@ struct gpe_pbf {
     bool lists_valid  = false;    // the lists were made in this step
     Sequence seq;                 // the launches of the graph that gpe_pbf_step captures
     bool hist_ready   = false;    // the last step's XSPH left the next step's cell keys and histogram
+    bool recorded     = false;    // a caller has recorded work of this engine (note_recording)
     int64_t dirty_cells = 0;      // ... and was dropped: so many of the histogram's cells must be cleared before a sort
 
     // within a step (after PREDICT_SORT): XS = the current (x, d) records, XO = the other buffer; -1 between steps
@@ -2243,6 +2244,18 @@ void drop_hist(gpe_pbf* s)
         s->hist_ready  = false;
         s->dirty_cells = std::max<int64_t>(s->dirty_cells, s->ncells);
     }
+}
+
+// A call whose work a caller records runs when the recording is replayed, once, often or never, and the host is not told.
+// So from the first recorded call on, no step leaves a histogram behind for a later call (gpe_pbf_step), and after a
+// recorded call the histogram counts as uncleared: what was recorded to clear it may not run before the next sort.
+// Returns whether the call is being recorded.
+bool note_recording(gpe_pbf* s, cudaStream_t st)
+{
+    if (!gpe::capturing(st)) { return false; }
+    s->recorded    = true;
+    s->dirty_cells = std::max<int64_t>(s->dirty_cells, s->ncells);
+    return true;
 }
 
 int32_t clear_hist(gpe_pbf* s, cudaStream_t st)
@@ -2901,6 +2914,7 @@ int32_t gpe_pbf_set_state(gpe_pbf* s, const float* pos, const float* vel, const 
     }
     cudaStream_t st = as_stream(stream);
     drop_hist(s);
+    const bool recording = note_recording(s, st);
     s->XS = s->XO   = -1;
     s->id_cur     = 0;
     const int32_t* dom_in = s->nd > 1 ? domain_id : nullptr;
@@ -2923,14 +2937,14 @@ int32_t gpe_pbf_set_state(gpe_pbf* s, const float* pos, const float* vel, const 
         }
     }
     if (direct) {
-        const int64_t cells = s->dirty_cells;
+        const int64_t cells = recording ? 0 : s->dirty_cells;
         const int64_t work  = std::max<int64_t>({n, s->cap / 4, cells / 4});
         k_set_state<<<(unsigned)std::min<int64_t>((work + T_PART - 1) / T_PART, (int64_t)gpe::sm_count() * 32), T_PART,
                       0, st>>>((int32_t)n, reinterpret_cast<const float2*>(pos), reinterpret_cast<const float2*>(vel),
                                dom_in, s->pos, s->vel, s->dom, s->ids[0], s->acc, s->cap, s->count, cells, s->tsum,
                                counts_sums(s) ? (int64_t)scan_blocks((uint32_t)cells) : 0, s->d_count);
         GPE_CHECK_LAUNCH("k_set_state");
-        s->dirty_cells = 0;
+        if (!recording) { s->dirty_cells = 0; }
     } else if (n > 0) {
         GPE_TRY_CUDA(cudaMemcpyAsync(s->pos, pos, sizeof(float2) * (size_t)n, kind_in(mem), st));
         if (vel) {
@@ -3027,15 +3041,16 @@ int32_t gpe_pbf_step(gpe_pbf* s, int32_t n_steps, void* stream)
         const int32_t iters = s->prm.iters;
         s->prm.iters        = gpe::mlp_pair_iters(s->mlp);
         s->launches         = 0;
-        const int32_t rc    = run_step(s, st, true);
+        const int32_t rc    = run_step(s, st, !s->recorded || n_steps > 1);
         s->prm.iters        = iters;
         if (rc) { return rc; }
         if (--n_steps == 0) { return GPE_OK; }
     }
     // the step sequence is captured once per (steps, whether the first sort's histogram is already there,
     // starting buffer roles) and replayed as one graph; every step but none in between leaves the next
-    // step's keys and histogram (stage_xsph)
-    const auto key = std::make_tuple(n_steps, (s->hist_ready ? 1 : 0) + (s->dirty_cells > 0 ? 2 : 0), s->id_cur);
+    // step's keys and histogram (stage_xsph), and the last one too unless a caller has recorded work
+    const auto key = std::make_tuple(n_steps, (s->hist_ready ? 1 : 0) + (s->dirty_cells > 0 ? 2 : 0) + (s->recorded ? 4 : 0),
+                                     s->id_cur);
     auto it        = s->graphs.find(key);
     if (it == s->graphs.end()) {
         cudaStream_t cap_st = st;
@@ -3051,7 +3066,7 @@ int32_t gpe_pbf_step(gpe_pbf* s, int32_t n_steps, void* stream)
         s->launches = 0;
         int32_t rc  = GPE_OK;
         s->seq.begin();
-        for (int32_t k = 0; k < n_steps && rc == GPE_OK; ++k) { rc = run_step(s, cap_st, true); }
+        for (int32_t k = 0; k < n_steps && rc == GPE_OK; ++k) { rc = run_step(s, cap_st, !s->recorded || k + 1 < n_steps); }
         s->seq.end();
         cudaGraph_t graph = nullptr;
         const cudaError_t ce = cudaStreamEndCapture(cap_st, &graph);
@@ -3095,9 +3110,13 @@ int32_t gpe_pbf_stage(gpe_pbf* s, int32_t stage, void* stream)
     const bool in_step = s->XS >= 0;
     if (stage != GPE_PBF_STAGE_DENSITY) { drop_hist(s); } // the density pass reads positions and cell starts
     switch (stage) {
-        case GPE_PBF_STAGE_PREDICT_SORT:
+        case GPE_PBF_STAGE_PREDICT_SORT: {
             if (in_step) { break; }
-            return stage_predict_sort(s, st);
+            note_recording(s, st);
+            const int32_t rc = stage_predict_sort(s, st);
+            note_recording(s, st);
+            return rc;
+        }
         case GPE_PBF_STAGE_LAMBDA:
             if (!in_step) { break; }
             return stage_lambda(s, st, acc_mode(s));
@@ -3260,6 +3279,7 @@ int32_t gpe_pbf_get_field(gpe_pbf* s, int32_t field, void* dst, int64_t n_elems,
         if (f.kind == 1) {
             // x* = x + d into the sort's (key, rank) scratch, which is free within a step, then out
             drop_hist(s); // the next step's keys may be waiting there
+            note_recording(s, st);
             float2* tmp = reinterpret_cast<float2*>(s->keyrank);
             k_xd_pred<<<blocks_for((int64_t)n), T_PART, 0, st>>>(static_cast<const float4*>(f.p), tmp, (int32_t)n);
             GPE_CHECK_LAUNCH("k_xd_pred");
@@ -3285,6 +3305,7 @@ int32_t gpe_pbf_set_field(gpe_pbf* s, int32_t field, const void* src, int64_t n_
     }
     s->lists_valid = false; // a written position (or anything else) may move a particle past its lists
     drop_hist(s);
+    note_recording(s, as_stream(stream));
     FieldLoc f{};
     int32_t rc = field_ptr(s, field, &f);
     if (rc) { return rc; }
@@ -3381,6 +3402,7 @@ extern "C" int32_t gpe_pbf_emit(gpe_pbf* s, const gpe_hose* hose, uint64_t seed,
         return GPE_ERR_NOT_READY;
     }
     drop_hist(s); // the new particles are not in the histogram the last step may have left
+    note_recording(s, as_stream(stream));
     HoseK h{};
     const int32_t cnt = make_hose(*hose, s->prm.dt, seed, &h);
     if (requested) { *requested = cnt; }
@@ -3446,6 +3468,7 @@ extern "C" int32_t gpe_pbf_publish_chunks(gpe_pbf* s, const gpe_chunk_state* sta
     cudaStream_t st     = as_stream(stream);
     const size_t chunks = (size_t)c.chunks_x * (size_t)c.chunks_y;
     drop_hist(s); // the chunk sort uses the (key, rank) array, where the next step's keys may be waiting
+    note_recording(s, st);
     GPE_TRY_CUDA(cudaMemsetAsync(c.offsets, 0, sizeof(uint32_t) * chunks * (size_t)(c.chunk_cells * c.chunk_cells), st));
     const int64_t n = lsize(s);
     if (n > 0) {
@@ -3477,9 +3500,11 @@ extern "C" int32_t gpe_pbf_enqueue(gpe_pbf* s, int32_t n_steps, void* stream)
     // (its last step's XSPH computes none)
     drop_hist(s);
     s->dirty_cells = std::max<int64_t>(s->dirty_cells, s->ncells);
+    note_recording(s, st);
     int32_t rc    = GPE_OK;
     const int id0 = s->id_cur;
     for (int32_t k = 0; k < n_steps && rc == GPE_OK; ++k) { rc = run_step(s, st, k + 1 < n_steps); }
+    note_recording(s, st);
     if (rc) { return rc; }
     // return the id buffer role to where it started, so the recorded sequence can be replayed (positions stay
     // in one buffer: every step writes its end positions where it read its start positions)
