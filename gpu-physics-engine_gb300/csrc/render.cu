@@ -210,7 +210,7 @@ extern "C" int32_t gpe_render_frame(const gpe_raster* r, const gpe_view* view, i
     {
         const int64_t n = (int64_t)r->width * r->height;
         const bool vec  = reinterpret_cast<uintptr_t>(r->coverage) % 16 == 0;
-        k_clear_centres<<<(unsigned)((vec ? (n + 3) / 4 : n) + 255) / 256, 256, 0, st>>>(r->coverage, n, vec);
+        k_clear_centres<<<(unsigned)(((vec ? (n + 3) / 4 : n) + 255) / 256), 256, 0, st>>>(r->coverage, n, vec);
         GPE_CHECK_LAUNCH("k_clear_centres");
     }
     {
