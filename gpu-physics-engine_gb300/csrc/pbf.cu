@@ -2350,30 +2350,30 @@ const DpFn kDp[2][2][2] = {{{dp_launch<false, false, false>, dp_launch<false, fa
                            {{dp_launch<true, false, false>, dp_launch<true, false, true>},
                             {dp_launch<true, true, false>, dp_launch<true, true, true>}}};
 
-using FeatFn = void (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
+using FeatFn = cudaError_t (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
                         const float4*, const float*, const uint32_t*, const MlpDev*, uint16_t*, int);
 template <bool M, bool S>
-void feat_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
+cudaError_t feat_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
                  const uint32_t* start, const float4* xd, const float* prev, const uint32_t* pid, const MlpDev* mlp,
                  uint16_t* feat, int list)
 {
     if (list == LIST_BUILD) {
-        launch(at, g, blk, k_lambda_feat<M, S, LIST_BUILD>, k, doms, dom, start, xd, prev, pid, mlp, feat);
+        return launch(at, g, blk, k_lambda_feat<M, S, LIST_BUILD>, k, doms, dom, start, xd, prev, pid, mlp, feat);
     } else {
-        launch(at, g, blk, k_lambda_feat<M, S, LIST_OFF>, k, doms, dom, start, xd, prev, pid, mlp, feat);
+        return launch(at, g, blk, k_lambda_feat<M, S, LIST_OFF>, k, doms, dom, start, xd, prev, pid, mlp, feat);
     }
 }
 const FeatFn kFeat[2][2] = {{feat_launch<false, false>, feat_launch<false, true>},
                             {feat_launch<true, false>, feat_launch<true, true>}};
 
-using ColFn = void (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
+using ColFn = cudaError_t (*)(unsigned, unsigned, Place, const PbfK&, const DomDev*, const int32_t*, const uint32_t*,
                        const float4*, const float*, float*, const uint32_t*, const CollectK&);
 template <bool M, bool S>
-void col_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
+cudaError_t col_launch(unsigned g, unsigned blk, Place at, const PbfK& k, const DomDev* doms, const int32_t* dom,
                 const uint32_t* start, const float4* xd, const float* prev, float* lam, const uint32_t* pid,
                 const CollectK& col)
 {
-    launch(at, g, blk, k_lambda_collect<M, S>, k, doms, dom, start, xd, prev, lam, pid, col);
+    return launch(at, g, blk, k_lambda_collect<M, S>, k, doms, dom, start, xd, prev, lam, pid, col);
 }
 const ColFn kCol[2][2] = {{col_launch<false, false>, col_launch<false, true>},
                           {col_launch<true, false>, col_launch<true, true>}};
@@ -2435,13 +2435,15 @@ int32_t stage_lambda_warm(gpe_pbf* s, cudaStream_t st)
     const int mi        = multi(s) ? 1 : 0;
     const int sg        = (s->prm.flags & GPE_PBF_SELF_GRAD) ? 1 : 0;
     const uint32_t* pid = (s->prm.flags & GPE_PBF_PAIR_IDS) ? s->ids[s->id_cur] : nullptr;
+    // these two kernels are compiled for T_PART threads a block; the tuned block may be larger
+    const unsigned blk  = (unsigned)std::min(s->block, T_PART);
+    const unsigned grid = (unsigned)((lsize(s) + blk - 1) / blk);
     if (s->warm == GPE_WARM_MLP && s->mem_valid && !s->collecting) {
         const gpe::MlpDev* md = gpe::mlp_device(s->mlp);
         // the feature pass scans every neighbour on the sorted positions: it makes the step's lists
         const int list = lists_on(s) ? LIST_BUILD : LIST_OFF;
-        kFeat[mi][sg](nblk(s), (unsigned)s->block, s->seq.at(st), s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev, pid,
-                      md, s->feat, list);
-        GPE_CHECK_LAUNCH("k_lambda_feat");
+        GPE_TRY_CUDA(kFeat[mi][sg](grid, blk, s->seq.at(st), s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev,
+                                   pid, md, s->feat, list));
         if (list == LIST_BUILD) {
             s->lists_valid = true;
         }
@@ -2450,9 +2452,8 @@ int32_t stage_lambda_warm(gpe_pbf* s, cudaStream_t st)
         GPE_TRY_CUDA(launch(s->seq.at(st), g, MLP_TILE, k_mlp_apply, s->k, s->feat, s->prev, s->lam, md, s->status));
         s->launches += 1;
     } else {
-        kCol[mi][sg](nblk(s), (unsigned)s->block, s->seq.at(st), s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev,
-                     s->lam, pid, s->col);
-        GPE_CHECK_LAUNCH("k_lambda_collect");
+        GPE_TRY_CUDA(kCol[mi][sg](grid, blk, s->seq.at(st), s->k, s->d_doms, s->dom, s->start, s->xd[s->XS], s->prev,
+                                  s->lam, pid, s->col));
     }
     s->launches += 1;
     return GPE_OK;
