@@ -194,7 +194,6 @@ __device__ __forceinline__ void for_neighbours(const DomDev& d, const PbfK& k, c
         const uint32_t row = d.coff + (uint32_t)y * (uint32_t)d.ncx;
         const uint32_t b   = __ldg(&start[row + x0]);
         const uint32_t e   = __ldg(&start[row + x1 + 1]);
-#pragma unroll 1
         for (uint32_t j = b; j < e; ++j) { f(j); }
     }
 }
