@@ -62,6 +62,7 @@ struct PbfK {
     uint8_t* mflag;
     int64_t nstride;          // particles a list chunk's array holds (the capacity)
     int32_t wide;             // lists of 32-bit slots
+    uint32_t list_max;        // candidates a list holds
     float skin2;              // (h + skin)^2
     float move2;              // (skin / 2)^2, shrunk for rounding
     // set for the XSPH pass of a step that also computes the next step's predicted cell keys and their
@@ -330,7 +331,7 @@ constexpr int TOGETHER_MAX = 4; // lanes for which that is cheaper: about 250 in
 // particles the same form costs 0.339 against 0.318 ms.
 enum { LIST_OFF = 0, LIST_BUILD = 1, LIST_USE = 2, LIST_FEW = 3 };
 constexpr uint32_t LIST_BAD   = 0x80000000u; // in the header's count: this particle's list is not usable
-constexpr uint32_t LIST_MAX   = 48;          // candidates a list holds (a multiple of 8)
+constexpr uint32_t LIST_MAX   = 48;          // candidates a list holds where there is room (a multiple of 8)
 constexpr uint32_t LIST_REACH = 32767;       // largest distance of a 16-bit slot
 
 // rsqrt of a value that is never subnormal (here: above 1e-12): the hardware's approximation, which rsqrtf
@@ -413,7 +414,7 @@ __device__ __forceinline__ bool scan_record(const DomDev& d, const PbfK& k, cons
         w[r] = wr;
     }
     const uint32_t cnt = (uint32_t)(__popc(w[0]) + __popc(w[1]) + __popc(w[2]));
-    fits               = fits && cnt <= LIST_MAX;
+    fits               = fits && cnt <= k.list_max;
     const uint32_t key = ldn<CG>(&k.keys[i]);
     // a list built around another cell than the sort cell (or none) is not used later
     const bool usable  = fits && key == d.coff + (uint32_t)by * (uint32_t)d.ncx + (uint32_t)bx;
@@ -2047,6 +2048,7 @@ struct gpe_pbf {
     float skin        = 0.075f;   // candidate-list skin in units of h (tuning; 0: full scans only)
     uint4* nhdr       = nullptr;  // candidate lists of the current step: headers
     uint4* nlist      = nullptr;  // ... and chunks (null: no room for them, full scans only)
+    uint32_t list_max = 0;        // ... candidates a particle
     bool wide         = false;    // ... of 32-bit slots
     uint8_t* mflag    = nullptr;  // per cell: a particle of its 3 x 3 cells moved too far for the lists
     bool lists_valid  = false;    // the lists were made in this step
@@ -2142,6 +2144,7 @@ void bind_k(gpe_pbf* s)
     s->k.nlist       = s->nlist;
     s->k.nstride     = s->cap;
     s->k.wide        = s->wide ? 1 : 0;
+    s->k.list_max    = s->list_max;
     s->k.mflag       = s->mflag;
     const float skin = s->skin * s->prm.h;
     s->k.skin2       = (s->prm.h + skin) * (s->prm.h + skin);
@@ -2736,17 +2739,18 @@ int32_t alloc_buffers(gpe_pbf* s)
     const size_t o_mf    = c.take<uint8_t>(M);
     // Candidate lists, behind the rest: 96 bytes a particle, 192 with 32-bit slots, of which a step touches what its
     // lists fill (32 on a lattice of spacing h / 2). Slots of 16 bits reach 2^15 away: the next cell row of a scene
-    // 4096 cells wide at up to 8 particles a cell; wider scenes take 32-bit slots. Without room for the lists the
-    // passes scan in full.
+    // 4096 cells wide at up to 8 particles a cell; wider scenes take 32-bit slots. Where that does not fit the lists
+    // hold 32 candidates, or 16 (12 lie within h on that lattice; a particle with more scans in full), and without
+    // room for those the passes scan in full.
     float widest = 0.f;
     for (const gpe_domain& d : s->doms) { widest = std::max(widest, d.extent[0]); }
     s->wide                 = widest > 4096.f * s->prm.h;
-    const size_t list_bytes = sizeof(uint4) * (LIST_MAX / (s->wide ? 4 : 8)) * std::max<size_t>(N, 1);
-    const bool lists        = cudaMalloc(&s->base, c.off + list_bytes) == cudaSuccess;
-    if (!lists) {
+    const size_t per_slot   = (s->wide ? sizeof(uint32_t) : sizeof(uint16_t)) * std::max<size_t>(N, 1);
+    for (s->list_max = LIST_MAX; s->list_max > 0; s->list_max -= 16) {
+        if (cudaMalloc(&s->base, c.off + per_slot * s->list_max) == cudaSuccess) { break; }
         cudaGetLastError();
-        GPE_TRY_CUDA(cudaMalloc(&s->base, c.off));
     }
+    if (s->list_max == 0) { GPE_TRY_CUDA(cudaMalloc(&s->base, c.off)); }
     GPE_TRY_CUDA(cudaMemset(s->base, 0, c.off));
     uint8_t* b = static_cast<uint8_t*>(s->base);
     s->d_doms  = reinterpret_cast<DomDev*>(b + o_doms);
@@ -2776,7 +2780,7 @@ int32_t alloc_buffers(gpe_pbf* s)
     s->gsync   = reinterpret_cast<GridSync*>(b + o_gs);
     s->nhdr   = reinterpret_cast<uint4*>(b + o_nm);
     s->mflag   = b + o_mf;
-    s->nlist   = lists ? reinterpret_cast<uint4*>(b + c.off) : nullptr;
+    s->nlist   = s->list_max > 0 ? reinterpret_cast<uint4*>(b + c.off) : nullptr;
     bind_k(s);
     GPE_TRY_CUDA(cudaMemcpy(s->d_doms, s->domdev.data(), sizeof(DomDev) * (size_t)s->nd, cudaMemcpyHostToDevice));
     return GPE_OK;
@@ -3582,7 +3586,7 @@ extern "C" int32_t gpe_pbf_get_tuning(const gpe_pbf* s, gpe_pbf_tuning* t)
     t->cell       = s->prm.cell > 0.f ? s->prm.cell : s->prm.h;
     t->block      = s->block;
     t->persistent = s->step_kernel ? 2 : (s->persistent ? 1 : 0);
-    t->skin       = s->skin;
+    t->skin       = s->nlist ? s->skin : 0.f; // (without room for lists every pass scans in full)
     return GPE_OK;
 }
 
@@ -3610,7 +3614,7 @@ extern "C" int32_t gpe_pbf_autotune(gpe_pbf* s, int32_t trial_steps, gpe_pbf_tun
     const TuneKey key{s->nd, (int32_t)std::lround(std::log2((double)std::max<int64_t>(s->n, 1))),
                       (int32_t)std::lround(aspect / (double)s->nd), s->prm.iters,
                       s->prm.flags & (GPE_PBF_SELF_GRAD | GPE_PBF_PAIR_IDS)};
-    {
+    if (s->nlist) { // (an engine without room for lists neither takes nor leaves a choice made with them)
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
@@ -3688,6 +3692,7 @@ extern "C" int32_t gpe_pbf_autotune(gpe_pbf* s, int32_t trial_steps, gpe_pbf_tun
     const int32_t blocks[3] = {128, 256, 512};
     std::vector<std::pair<float, gpe_pbf_tuning>> timed;
     for (int ci = 0; ci < 5 && rc == GPE_OK; ++ci) {
+        if (skins[ci] > 0.f && !s->nlist) { continue; }
         for (int bi = 0; bi < 3 && rc == GPE_OK; ++bi) {
             for (int pi = 0; pi < 3 && rc == GPE_OK; ++pi) {
                 const gpe_pbf_tuning cand{cells[ci], blocks[bi], pi, skins[ci]};
@@ -3727,7 +3732,7 @@ extern "C" int32_t gpe_pbf_autotune(gpe_pbf* s, int32_t trial_steps, gpe_pbf_tun
     cudaFree(save);
     if (rc) { return rc; }
     if (rc2) { return rc2; }
-    if (win_ms >= 0.f) {
+    if (win_ms >= 0.f && s->nlist) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tune_cache[key] = win;
     }

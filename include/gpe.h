@@ -369,7 +369,9 @@ typedef struct gpe_pbf_tuning {
                            3 x 3 cells lie within h + skin * h, and the later passes of the step visit
                            only those while no particle nearby is skin * h / 2 or more from where it was
                            then (else that particle's neighbourhood scans in full). Same result bit for
-                           bit; 0 turns the lists off                                                   */
+                           bit; 0 turns the lists off. The lists take 96 bytes of device memory a particle
+                           of the capacity (192 in scenes wider than 4096 h), or 64 or 32 (128 or 64) where
+                           that does not fit; an engine without room for any reports skin 0          */
 } gpe_pbf_tuning;
 
 int32_t gpe_pbf_get_tuning(const gpe_pbf* pbf, gpe_pbf_tuning* tuning);
