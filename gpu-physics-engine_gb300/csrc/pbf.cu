@@ -2875,6 +2875,7 @@ int32_t gpe_pbf_set_params(gpe_pbf* s, const gpe_pbf_params* params)
         return GPE_ERR_BAD_ARG;
     }
     drop_hist(s);
+    s->lists_valid = false; // (within a step: other radii than the lists were made with)
     s->prm     = *params;
     s->dynamic = (params->flags & GPE_PBF_DYNAMIC_COUNT) != 0;
     build_domains(s);
