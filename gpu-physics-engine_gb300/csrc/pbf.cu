@@ -334,8 +334,8 @@ constexpr uint32_t LIST_BAD   = 0x80000000u; // in the header's count: this part
 constexpr uint32_t LIST_MAX   = 48;          // candidates a list holds where there is room (a multiple of 8)
 constexpr uint32_t LIST_REACH = 32767;       // largest distance of a 16-bit slot
 
-// rsqrt of a value that is never subnormal (here: above 1e-12): the hardware's approximation, which rsqrtf
-// returns for such values too, without rsqrtf's scaling of subnormal arguments
+// 1 / sqrt(v) as the PTX ISA's rsqrt.approx.ftz.f32, which takes subnormal arguments as zero: for arguments above
+// 1e-12, or whose result is dropped
 __device__ __forceinline__ float rsqrt_normal(float v)
 {
     float r;

@@ -233,7 +233,8 @@ typedef struct gpe_chunk_state {
 int32_t gpe_pbf_publish_chunks(gpe_pbf* pbf, const gpe_chunk_state* state, void* stream);
 /* Issues n_steps steps on the stream without an engine-owned graph, so that they can be recorded into the
  * caller's own stream capture (the reference's instantiatePBFGraph builds one graph per tick, PBF.cu:901-961).
- * Buffer roles are returned to their starting state at the end, so a captured sequence can be replayed. */
+ * Buffer roles are returned to their starting state at the end, so a captured sequence can be replayed, and
+ * gpe_pbf_step can run before the first replay and between replays. */
 int32_t gpe_pbf_enqueue(gpe_pbf* pbf, int32_t n_steps, void* stream);
 
 /* ======================================================================================================

@@ -51,7 +51,8 @@ def test_steps_around_recorded_calls(gpe_mod, cuda_ok, kind, what):
         pytest.skip("emitters need a device-resident count")
     (a, pos, vel), (b, _, _) = _engine(gpe_mod, kind, 4000), _engine(gpe_mod, kind, 4000)
     new = [torch.from_numpy(np.ascontiguousarray(q[::-1])).cuda() for q in (pos, vel)]
-    hose = gpe_mod.make_hose((50.0, 150.0), (1.0, -0.3), 8.0, 1.05, 0.02, 20)
+    # (32 particles: a warp's emission has one order, several warps' append in any)
+    hose = gpe_mod.make_hose((50.0, 150.0), (1.0, -0.3), 8.0, 1.05, 0.02, 4)
     stages = [gpe_mod.PBF_STAGE_PREDICT_SORT] + 2 * [gpe_mod.PBF_STAGE_LAMBDA, gpe_mod.PBF_STAGE_DELTA_P] + [
         gpe_mod.PBF_STAGE_XSPH, gpe_mod.PBF_STAGE_FINISH]
 
@@ -61,7 +62,7 @@ def test_steps_around_recorded_calls(gpe_mod, cuda_ok, kind, what):
         if what in ("enqueue", "both"):
             e.enqueue(2, stream=st)
         if what == "emit":
-            e.emit(hose, seed=9, stream=st)
+            assert e.emit(hose, seed=9, stream=st) == 32
         if what == "stages":
             for s in stages:
                 e.stage(s, stream=st)
