@@ -9,7 +9,7 @@
 //   k_g2p2g          G2P of the step and P2G of the next, two consecutive particles per thread: each gathers its 9 node
 //                    velocities from that array (L1/L2 hits: sorted neighbours share nodes), is updated, and the warp
 //                    scatters its 64 particles to the next grid (scatter_pair), lanes that share a stencil base node
-//                    summing their contributions first. Its bound is instruction issue (77%, 4 blocks of 256 an SM at
+//                    summing their contributions first. Its bound is instruction issue (76%, 4 blocks of 256 an SM at
 //                    64 registers): 4M mixed particles 116 us a step where k_p2g and k_g2p took 103 and 64.
 //   k_p2g, k_g2p     the halves of the first and the last step.
 // (Measured alternatives, each slower: a G2P that staged its block's node box in shared memory and updated

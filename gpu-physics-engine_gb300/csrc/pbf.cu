@@ -414,9 +414,9 @@ __device__ __forceinline__ bool scan_record(const DomDev& d, const PbfK& k, cons
         w[r] = wr;
     }
     const uint32_t cnt = (uint32_t)(__popc(w[0]) + __popc(w[1]) + __popc(w[2]));
-    fits               = fits && cnt <= k.list_max;
     const uint32_t key = ldn<CG>(&k.keys[i]);
     // a list built around another cell than the sort cell (or none) is not used later
+    if (cnt > k.list_max) { fits = false; }
     const bool usable  = fits && key == d.coff + (uint32_t)by * (uint32_t)d.ncx + (uint32_t)bx;
     k.nhdr[i] = make_uint4(key, cnt | (usable ? 0u : LIST_BAD), __float_as_uint(me.pd.x), __float_as_uint(me.pd.y));
     if (!fits) { return scan_full(d, start, bx, by, me, ld, pass, acc); }
@@ -2191,14 +2191,16 @@ void build_domains(gpe_pbf* s)
     bind_k(s);
 }
 
-// Launch size: with a device-resident count that emitters can grow inside a captured graph, every launch
-// covers the capacity and the kernels read the live count; otherwise the host count.
 // Whether the histogram's kernels also count the scan's tile totals, which saves the scan a pass of its own. The atomics
-// of all warps go to few addresses, so this is for few particles: 16,384 in one step with the state in and out 47.1 ->
-// 45.1 us, in 20 substeps 610 -> 589; 100k 67.6 either way; 1M 298 -> 310.
+// of all warps go to few addresses, so this is for few particles. 20 substeps without and with it, us: 8,192 atoms 581
+// and 560, 32,768 639 and 617, 65,536 699 and 678, 131,072 885 and 875, 262,144 1437 and 1432; one step with the state in
+// and out: 16,384 47.5 and 45.5, 65,536 51.7 and 51.6, 98,304 57.8 both, 131,072 64.0 and 65.3, 262,144 97.8 and 103.6,
+// 1M 298 and 310. The line is the largest power of two at which neither loses.
 constexpr int64_t SUMS_MAX = 65536;
 bool counts_sums(const gpe_pbf* s) { return s->cap <= SUMS_MAX; }
 
+// Launch size: with a device-resident count that emitters can grow inside a captured graph, every launch
+// covers the capacity and the kernels read the live count; otherwise the host count.
 int64_t lsize(const gpe_pbf* s) { return s->dynamic ? s->cap : s->n; }
 
 // Refreshes the host copy of the particle count from the device (only needed with a dynamic count).

@@ -123,8 +123,9 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_bsum(uint32_t* __restrict__ bsu
 
 // SUMS: bsum holds the tiles' totals (not scanned) and each block adds up those before it itself, which saves the
 // single-block scan launch while the tiles are few (FUSED_MAX_TILES: 16 sums a thread at most); else bsum is already the
-// exclusive scan of the totals. At some 2,440 tiles (256 scenes
-// of 5.0M cells) the separate launch cost 6.3 us and the sums cost less than can be told.
+// exclusive scan of the totals. One step of 262,144 particles with that launch and without it, us: 600 tiles 73.0 and
+// 71.3, 1,024 74.7 and 72.9, 2,048 85.6 and 80.7, 3,000 96.3 and 88.2, 4,000 105 and 94; 6,000 141 and 107, so the line
+// is not where the two meet but where it has been tested.
 constexpr uint32_t FUSED_MAX_TILES = 4096;
 
 // Bound by the memory traffic: four cells per access (5.0M cells, a count not divisible by four, 24 us one by one, 10 so); the
